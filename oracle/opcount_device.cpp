@@ -68,6 +68,25 @@ static inline cdouble fmax(cdouble a, cdouble b) { return cdouble(::fmax(a.v, b.
 static inline cdouble fmin(cdouble a, cdouble b) { return cdouble(::fmin(a.v, b.v)); }
 static inline cdouble copysign(cdouble a, cdouble b) { return cdouble(::copysign(a.v, b.v)); }
 
+// gpr_fastmath.cuh's operations by their meaning (its own instructions are a
+// reciprocal start and a few fused multiply-adds)
+#define GPR_FASTMATH_PROVIDED
+static inline cdouble rcp64(cdouble a) { T.div++; return cdouble(1.0 / a.v); }
+static inline cdouble sqrt64(cdouble a) { T.sqrt_++; return cdouble(::sqrt(a.v)); }
+static inline cdouble pow53(cdouble a) {
+  T.trans++; T.mul += 2;
+  return cdouble(a.v * ::cbrt(a.v) * ::cbrt(a.v));
+}
+static inline float f32_scaled(cdouble a, int sh) { return (float)::ldexp(a.v, -sh); }
+static inline cdouble f64_scaled(float f, int sh) { return cdouble(::ldexp((double)f, sh)); }
+static inline float rcp32(float x) { return 1.0f / x; }
+static inline float sqrt32(float x) { return ::sqrtf(x); }
+static inline int __double2hiint(cdouble a) {
+  long long b;
+  memcpy(&b, &a.v, 8);
+  return (int)(b >> 32);
+}
+
 // the oracle (plain doubles) provides the states
 extern "C" {
 int or_configure(int n, int thermal, int lset, double dg_tol, int dg_it);
@@ -87,6 +106,7 @@ int or_predictor(double *qh, const double *wh, double dt, const double *dX, int 
 #define __host__
 #define __device__
 #define __forceinline__ inline
+#define __noinline__
 #define cuda_runtime_h_stub
 #define double cdouble
 #include "../phd_gb300/csrc/gpr_device.cuh"

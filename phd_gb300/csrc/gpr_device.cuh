@@ -20,6 +20,10 @@
 #define GPR_HD __host__ __device__ __forceinline__
 #define GPR_D __device__ __forceinline__
 
+#ifndef GPR_FASTMATH_PROVIDED  // a host build of this header brings its own
+#include "gpr_fastmath.cuh"
+#endif
+
 namespace gpr {
 
 // the least positive normal double (DBL_MIN)
@@ -37,6 +41,15 @@ struct DevPar {
   double tau1;   // 6 mu^(1/n) / (rho0 b02)      (analytic.cpp:62)
   double iG;     // 1/Gamma for the constant-Gamma EOS; 1/(Gamma0 rho0) for shock MG
   double C0f;    // 1 - beta/Gamma for the constant-Gamma EOS
+  // Per-material products and tests, formed once on the host: in a kernel
+  // each would be an FP64 instruction of every thread (a comparison too runs
+  // on the FP64 pipe).
+  double gm1;    // gamma - 1
+  double b1;     // 1 + beta
+  double b02q;   // b02 / 4
+  double hca2;   // calpha2 / 2
+  double ca2ik;  // calpha2 / kappa
+  int has_beta, has_tref, has_dp;  // beta, Tref, dp not all zero
 };
 
 inline DevPar make_devpar(const gpr_par &p) {
@@ -75,6 +88,15 @@ inline DevPar make_devpar(const gpr_par &p) {
   double G = p.EOS == 0 ? p.gamma - 1.0 : (p.EOS == 4 ? p.gamma : p.Gamma0);
   d.iG = p.EOS == 1 ? 1.0 / (p.Gamma0 * p.rho0) : 1.0 / G;
   d.C0f = 1.0 - p.beta / G;
+  d.gm1 = p.gamma - 1.0;
+  d.b1 = 1.0 + p.beta;
+  d.b02q = 0.25 * p.b02;
+  d.hca2 = 0.5 * p.calpha2;
+  d.ca2ik = p.calpha2 * d.ikappa;
+  // a NaN counts as present, as it does in the comparison x != 0
+  d.has_beta = p.beta != 0.0;
+  d.has_tref = p.Tref != 0.0;
+  d.has_dp = p.dp[0] != 0.0 || p.dp[1] != 0.0 || p.dp[2] != 0.0;
   return d;
 }
 
@@ -96,13 +118,13 @@ GPR_D EosRho eos_rho(double r, double ir, const DevPar &P) {
   EosRho e;
   switch (P.EOS) {
   case 0: {  // stiffened gas
-    e.G = P.gamma - 1.0;
+    e.G = P.gm1;
     e.dG = 0.0;
     e.pr = -P.pINF;
     e.dpr = 0.0;
     e.er = P.pINF * ir;
     e.der = e.pr * ir * ir;
-    e.phi = P.Tref != 0.0 ? pow(r * P.ir0, P.gamma - 1.0) : 0.0;
+    e.phi = P.has_tref ? pow(r * P.ir0, P.gm1) : 0.0;
   } break;
   case 1: {  // shock Mie-Gruneisen
     e.G = P.Gamma0 * P.rho0 * ir;
@@ -120,7 +142,7 @@ GPR_D EosRho eos_rho(double r, double ir, const DevPar &P) {
       e.er = 0.0;
       e.der = 0.0;
     }
-    e.phi = P.Tref != 0.0 ? exp(P.Gamma0 * (1.0 - P.rho0 * ir)) : 0.0;
+    e.phi = P.has_tref ? exp(P.Gamma0 * (1.0 - P.rho0 * ir)) : 0.0;
   } break;
   case 4: {  // Godunov-Romenski
     e.G = P.gamma;
@@ -130,7 +152,7 @@ GPR_D EosRho eos_rho(double r, double ir, const DevPar &P) {
     e.dpr = P.c02 / P.alpha * tmp * ((1.0 + P.alpha) * (tmp - 1.0) + P.alpha * tmp);
     e.er = P.c02 / (2.0 * P.alpha * P.alpha) * (tmp - 1.0) * (tmp - 1.0);
     e.der = e.pr * ir * ir;
-    e.phi = P.Tref != 0.0 ? pow(r * P.ir0, P.gamma) : 0.0;
+    e.phi = P.has_tref ? pow(r * P.ir0, P.gamma) : 0.0;
   } break;
   case 2: {  // JWL
     e.G = P.Gamma0;
@@ -141,7 +163,7 @@ GPR_D EosRho eos_rho(double r, double ir, const DevPar &P) {
     e.dpr = v_ * ir * (P.A * P.R1 * e1 + P.B * P.R2 * e2);
     e.er = P.A / (P.rho0 * P.R1) * e1 + P.B / (P.rho0 * P.R2) * e2;
     e.der = e.pr * ir * ir;
-    e.phi = P.Tref != 0.0 ? pow(r * P.ir0, P.Gamma0) : 0.0;
+    e.phi = P.has_tref ? pow(r * P.ir0, P.Gamma0) : 0.0;
   } break;
   default: {  // Cochran-Chan
     e.G = P.Gamma0;
@@ -153,7 +175,7 @@ GPR_D EosRho eos_rho(double r, double ir, const DevPar &P) {
     e.er = -P.A / (P.rho0 * (1.0 - P.R1)) * (pow(v_, 1.0 - P.R1) - 1.0) +
            P.B / (P.rho0 * (1.0 - P.R2)) * (pow(v_, 1.0 - P.R2) - 1.0);
     e.der = e.pr * ir * ir;
-    e.phi = P.Tref != 0.0 ? pow(r * P.ir0, P.Gamma0) : 0.0;
+    e.phi = P.has_tref ? pow(r * P.ir0, P.Gamma0) : 0.0;
   } break;
   }
   return e;
@@ -169,6 +191,8 @@ template <bool TH> struct Prim {
   double v[3];           // velocity
   double J[3];           // thermal impulse (TH)
   double AdG[9];         // A devG (row-major)
+  double G[6];           // A^T A: 00, 11, 22, 01, 02, 12
+  double S[6];           // devG A^T A (symmetric: the factors commute), same order
   double cs2;            // b02 (rho/rho0)^beta
   double devGsq;         // |dev G|^2
   double p, T;           // pressure, temperature
@@ -176,10 +200,20 @@ template <bool TH> struct Prim {
   EosRho e;
 };
 
+// entry (i, d) of a symmetric 3x3 matrix stored as 00, 11, 22, 01, 02, 12 (i a
+// compile-time constant after unrolling; selects for a run-time d)
+GPR_D double sym3(const double *m, int i, int d) {
+  if (i == 0)
+    return d == 0 ? m[0] : (d == 1 ? m[3] : m[4]);
+  if (i == 1)
+    return d == 0 ? m[3] : (d == 1 ? m[1] : m[5]);
+  return d == 0 ? m[4] : (d == 1 ? m[5] : m[2]);
+}
+
 template <bool TH>
 GPR_D void prim(const double *q, const DevPar &P, Prim<TH> &s) {
   s.r = q[0];
-  s.ir = 1.0 / s.r;
+  s.ir = rcp64(s.r);
   s.v[0] = q[2] * s.ir;
   s.v[1] = q[3] * s.ir;
   s.v[2] = q[4] * s.ir;
@@ -193,6 +227,18 @@ GPR_D void prim(const double *q, const DevPar &P, Prim<TH> &s) {
   double t = (G00 + G11 + G22) * (1.0 / 3.0);
   double D00 = G00 - t, D11 = G11 - t, D22 = G22 - t;
   s.devGsq = D00 * D00 + D11 * D11 + D22 * D22 + 2.0 * (G01 * G01 + G02 * G02 + G12 * G12);
+  s.G[0] = G00;
+  s.G[1] = G11;
+  s.G[2] = G22;
+  s.G[3] = G01;
+  s.G[4] = G02;
+  s.G[5] = G12;
+  s.S[0] = D00 * G00 + G01 * G01 + G02 * G02;
+  s.S[1] = G01 * G01 + D11 * G11 + G12 * G12;
+  s.S[2] = G02 * G02 + G12 * G12 + D22 * G22;
+  s.S[3] = D00 * G01 + G01 * G11 + G02 * G12;
+  s.S[4] = D00 * G02 + G01 * G12 + G02 * G22;
+  s.S[5] = G01 * G02 + D11 * G12 + G12 * G22;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     double a0 = A[3 * i], a1 = A[3 * i + 1], a2 = A[3 * i + 2];
@@ -201,33 +247,39 @@ GPR_D void prim(const double *q, const DevPar &P, Prim<TH> &s) {
     s.AdG[3 * i + 2] = a0 * G02 + a1 * G12 + a2 * D22;
   }
   s.e = eos_rho(s.r, s.ir, P);
-  s.cs2 = P.beta == 0.0 ? P.b02 : P.b02 * pow(s.r * P.ir0, P.beta);
-  // C_0 = (1 - beta/Gamma) cs2 (shear.cpp:23-29); rho Gamma = Gamma0 rho0 for shock MG
-  double C0 = P.beta == 0.0 ? s.cs2
-                            : (P.EOS == 1 ? (1.0 - P.beta / s.e.G) : P.C0f) * s.cs2;
+  s.cs2 = P.b02;
+  // C_0 / 4 with C_0 = (1 - beta/Gamma) cs2 (shear.cpp:23-29); rho Gamma =
+  // Gamma0 rho0 for shock MG
+  double C0q = P.b02q;
+  if (P.has_beta) {
+    s.cs2 = P.b02 * pow(s.r * P.ir0, P.beta);
+    C0q = 0.25 * ((P.EOS == 1 ? (1.0 - P.beta / s.e.G) : P.C0f) * s.cs2);
+  }
   s.irG = P.EOS == 1 ? P.iG : s.ir * P.iG;
   double E1 = q[1] * s.ir - 0.5 * (s.v[0] * s.v[0] + s.v[1] * s.v[1] + s.v[2] * s.v[2]) -
-              0.25 * C0 * s.devGsq;
+              C0q * s.devGsq;
   if (TH) {
     s.J[0] = q[14] * s.ir;
     s.J[1] = q[15] * s.ir;
     s.J[2] = q[16] * s.ir;
-    E1 -= 0.5 * P.calpha2 * (s.J[0] * s.J[0] + s.J[1] * s.J[1] + s.J[2] * s.J[2]);
+    E1 -= P.hca2 * (s.J[0] * s.J[0] + s.J[1] * s.J[1] + s.J[2] * s.J[2]);
   }
   // pressure_mg (mg.cpp:126-131), temperature_mg (mg.cpp:133-139)
   double rG = s.r * s.e.G;
   s.p = (E1 - s.e.er) * rG + s.e.pr;
-  s.T = s.e.phi * P.Tref + (s.p - s.e.pr) * s.irG * P.icv;
+  s.T = (s.p - s.e.pr) * s.irG * P.icv;
+  if (P.has_tref)
+    s.T = s.e.phi * P.Tref + s.T;
 }
 
-// sigma column d: -rho cs2 (A devG)^T A(:,d)   (state.cpp:23-29)
+// sigma column d: -rho cs2 (A devG)^T A(:,d) = -rho cs2 (devG A^T A)(:,d)
+// (state.cpp:23-29)
 template <bool TH>
-GPR_D void sigma_col(const double *q, const Prim<TH> &s, int d, double *sg) {
-  const double *A = q + 5;
+GPR_D void sigma_col(const double *, const Prim<TH> &s, int d, double *sg) {
   double f = -s.r * s.cs2;
 #pragma unroll
   for (int i = 0; i < 3; i++)
-    sg[i] = f * (s.AdG[i] * A[d] + s.AdG[3 + i] * A[3 + d] + s.AdG[6 + i] * A[6 + d]);
+    sg[i] = f * sym3(s.S, i, d);
 }
 
 // ret += F_d(Q)   (equations.cpp:11-48)
@@ -311,9 +363,7 @@ GPR_D void sigma_full(const double *q, const Prim<TH> &s, double *sf) {
 // theta1inv (sources.cpp:13-81)
 template <bool TH>
 GPR_D double theta1inv(const double *q, const Prim<TH> &s, const DevPar &P) {
-  double dA = det3(q + 5);
-  double cb = cbrt(dA);
-  double A53 = dA * cb * cb;  // det(A)^(5/3)
+  const double A53 = pow53(det3(q + 5));  // det(A)^(5/3)
   int SOLID = P.flags & GPR_SOLID, PL = P.flags & GPR_POWER_LAW, BING = P.flags & GPR_BINGHAM;
   if (!SOLID && !BING && !PL)
     return A53 * P.th1c;
@@ -345,16 +395,18 @@ GPR_D void source(const double *q, const Prim<TH> &s, const DevPar &P, double *S
 #pragma unroll
   for (int k = 0; k < V; k++)
     S[k] = 0.0;
-  S[2] = P.dp0 * scale;
-  S[3] = P.dp1 * scale;
-  S[4] = P.dp2 * scale;
+  if (P.has_dp) {
+    S[2] = P.dp0 * scale;
+    S[3] = P.dp1 * scale;
+    S[4] = P.dp2 * scale;
+  }
   double f = -s.cs2 * theta1inv(q, s, P) * scale;
 #pragma unroll
   for (int i = 0; i < 9; i++)
     S[5 + i] = s.AdG[i] * f;
   if (TH) {
     // -rho (calpha2 J) T / (kappa rho)
-    double g = -P.calpha2 * s.T * P.ikappa * scale;
+    double g = -P.ca2ik * s.T * scale;
 #pragma unroll
     for (int i = 0; i < 3; i++)
       S[14 + i] = g * s.J[i];
@@ -601,9 +653,7 @@ template <int n> GPR_D double max_abs_eig(double (&H)[n][n]) {
 // quotient).  Returns false when the certificate fails (complex roots of
 // larger modulus, a multiple largest root, no convergence); the caller then
 // runs the QR iteration, so the result is max |eig| either way.
-// Z: X[1][m-1] and X[2][m-1] are known zeros (the heat-conduction column of
-// the acoustic tensor), left out of the characteristic polynomial.
-template <int m, bool Z = false>
+template <int m>
 GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
   static_assert(m == 3 || m == 4, "3x3 or 4x4");
   double c1 = 0.0, c2 = 0.0, c3 = 0.0, c4 = 0.0;
@@ -629,27 +679,21 @@ GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
     auto mn = [](double a, double b, double c, double d) { return fma(a, b, -(c * d)); };
     auto s = [&](int a, int b) { return mn(X[0][a], X[1][b], X[0][b], X[1][a]); };
     auto t = [&](int a, int b) { return mn(X[r2][a], X[r3][b], X[r2][b], X[r3][a]); };
-    // with Z, X[1][3] = X[2][3] = 0 drop out of the minors that contain them
     const double s01 = s(0, 1), s02 = s(0, 2), s12 = s(1, 2);
-    const double s03 = Z ? -(X[0][r3] * X[1][0]) : s(0, 3);
-    const double s13 = Z ? -(X[0][r3] * X[1][1]) : s(1, 3);
-    const double s23 = Z ? -(X[0][r3] * X[1][r2]) : s(2, 3);
+    const double s03 = s(0, 3), s13 = s(1, 3), s23 = s(2, 3);
     const double t01 = t(0, 1), t02 = t(0, 2), t12 = t(1, 2);
-    const double t03 = Z ? X[r2][0] * X[r3][r3] : t(0, 3);
-    const double t13 = Z ? X[r2][1] * X[r3][r3] : t(1, 3);
-    const double t23 = Z ? X[r2][r2] * X[r3][r3] : t(2, 3);
+    const double t03 = t(0, 3), t13 = t(1, 3), t23 = t(2, 3);
     c2 = ((s01 + t23) + (mn(X[0][0], X[r2][r2], X[0][r2], X[r2][0]) +
                          mn(X[0][0], X[r3][r3], X[0][r3], X[r3][0]))) +
          (mn(X[1][1], X[r2][r2], X[1][r2], X[r2][1]) +
-          (Z ? X[1][1] * X[r3][r3] : mn(X[1][1], X[r3][r3], X[1][r3], X[r3][1])));
+          mn(X[1][1], X[r3][r3], X[1][r3], X[r3][1]));
     auto e3 = [](double a, double sa, double b, double sb, double c, double sc) {
       return fma(c, sc, fma(a, sa, -(b * sb)));
     };
     c3 = (e3(X[r2][r2], s01, X[r2][1], s02, X[r2][0], s12) +
           e3(X[r3][r3], s01, X[r3][1], s03, X[r3][0], s13)) +
          (e3(X[0][0], t23, X[0][r2], t03, X[0][r3], t02) +
-          (Z ? fma(X[1][1], t23, -(X[1][r2] * t13))
-             : e3(X[1][1], t23, X[1][r2], t13, X[1][r3], t12)));
+          e3(X[1][1], t23, X[1][r2], t13, X[1][r3], t12));
     c4 = (mn(s01, t23, s02, t13) + fma(s03, t12, s12 * t03)) - fma(s13, t02, -(s23 * t01));
   }
   // p(x) = x^m - c1 x^(m-1) + c2 x^(m-2) - c3 x^(m-3) [+ c4]
@@ -740,92 +784,267 @@ GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
          fabs(a0 * a0 - 1.0) > fabs(a0 * a2 - a1);
 }
 
+// The largest eigenvalue of the acoustic tensor by the general routines
+// (Laguerre in FP64 with its certificate, then QR): for the states that
+// top_root leaves (no real dominant root, or one within 1e-4 of another).
+// Out of line: the callers' registers are not sized for it.
+template <int m> __device__ __noinline__ double max_eig_general(const double *Xr) {
+  double X[m][m], l2;
+#pragma unroll
+  for (int i = 0; i < m; i++)
+#pragma unroll
+    for (int c = 0; c < m; c++)
+      X[i][c] = Xr[i * m + c];
+  if (!max_eig_laguerre<m>(X, l2))
+    l2 = max_abs_eig<m>(X);
+  return l2;
+}
+
+// The largest root of x^m - c[0] x^(m-1) + c[1] x^(m-2) - ... when it is real,
+// positive and simple (the squared fastest wave speed), with few FP64
+// instructions: everything that only has to be near runs in FP32 on the
+// polynomial scaled by a power of two (bit fields, no FP64 instruction), and
+// FP64 evaluates the residual p(x) alone.
+//  1. FP32: Laguerre's iteration from sqrt(c0^2 - 2 c1) (the 2-norm of a real
+//     spectrum, at least its largest root) down to ~1e-6, and p' there.
+//  2. FP32: certificate that p / (x - y) has its roots inside |z| < (1 - 1e-4)
+//     y (Jury's criterion, margins ten times the FP32 rounding).
+//  3. FP64: x <- x - p(x) / p'(y) with the FP32 derivative.  A step leaves the
+//     error times ~1e-6 (the FP32 error of p' and its change over a 1e-6
+//     interval); the ratio of two steps measures that factor, and the
+//     iteration stops when the factor times the last step is below 2^-56 x (or
+//     the step is at the rounding of p).
+// Returns false when any of it fails; the caller takes the general routine.
+// Against the previous FP64 Laguerre step with its FP64 certificate (two
+// divisions and a root in each, and six FP64 <-> FP32 conversions, which run on
+// the FP64 pipe) this issues about 13 FP64 instructions instead of about 110.
+template <int m> GPR_D bool top_root(const double (&c)[m], double &lam) {
+  const int hi = __double2hiint(c[0]);
+  const int sh = ((hi >> 20) & 0x7ff) - 1022;
+  if (hi < 0 || sh < -240 || sh > 240)
+    return false;
+  float a[m];  // coefficients of the scaled monic polynomial
+#pragma unroll
+  for (int k = 0; k < m; k++)
+    a[k] = ((k & 1) ? 1.0f : -1.0f) * f32_scaled(c[k], (k + 1) * sh);
+  const float b2 = fmaf(a[0], a[0], -2.0f * a[1]);
+  float y = sqrt32(b2) * 1.00001f, dp = 0.0f;
+  bool near = false;
+#pragma unroll 1
+  for (int it = 0; it < 12; it++) {
+    float p = 1.0f, d2p = 0.0f;
+    dp = 0.0f;
+#pragma unroll
+    for (int k = 0; k < m; k++) {
+      d2p = fmaf(d2p, y, 2.0f * dp);
+      dp = fmaf(dp, y, p);
+      p = fmaf(p, y, a[k]);
+    }
+    if (near)  // p' at the accepted y
+      break;
+    // Laguerre's step m p / (p' + sqrt((m-1)^2 p'^2 - m (m-1) p p''))
+    const float disc = fmaf((float)((m - 1) * (m - 1)) * dp, dp, -(float)(m * (m - 1)) * (p * d2p));
+    const float st = (float)m * p * rcp32(dp + copysignf(sqrt32(fmaxf(disc, 0.0f)), dp));
+    y -= st;
+    near = fabsf(st) <= 1e-3f * y;
+    if (!(y > 0.0f))
+      return false;
+  }
+  if (!near)
+    return false;
+  // certificate on the quotient, scaled by l = (1 - 1e-4) y
+  {
+    const float il = 1.0001f * rcp32(y);
+    const float q2 = a[0] + y, q1 = fmaf(y, q2, a[1]);
+    bool in;
+    if (m == 3) {
+      const float a1 = q2 * il, a0 = q1 * il * il;
+      in = fabsf(a0) < 1.0f - 1e-5f && fabsf(a1) < 1.0f + a0 - 1e-5f;
+    } else {
+      const float q0 = fmaf(y, q1, a[2]);
+      const float a2 = q2 * il, a1 = q1 * il * il, a0 = q0 * il * il * il;
+      in = 1.0f + a2 + a1 + a0 > 1e-5f && 1.0f - a2 + a1 - a0 > 1e-5f &&
+           fabsf(a0) < 1.0f - 1e-5f && fabsf(a0 * a0 - 1.0f) > fabsf(a0 * a2 - a1) + 1e-5f;
+    }
+    if (!in)
+      return false;
+  }
+  // p'(y) scales by 2^((m-1) sh)
+  const double ip = f64_scaled(rcp32(dp), -(m - 1) * sh);
+  double x = f64_scaled(y, sh);
+  float prev = 0.0f;
+#pragma unroll 1
+  for (int it = 0; it < 8; it++) {
+    double p = x - c[0];
+#pragma unroll
+    for (int k = 1; k < m; k++)
+      p = fma(p, x, (k & 1) ? c[k] : -c[k]);
+    const double st = p * ip;
+    x -= st;
+    const float s = fabsf(f32_scaled(st, sh));
+    if (s * s <= 1.4e-17f * y * prev || s <= 2e-15f * y) {
+      lam = x;
+      return true;
+    }
+    prev = s;
+  }
+  return false;
+}
+
 // max |eigenvalue| of the GPR system in direction d (system/eig.cpp:8-77):
 // |v_d| + sqrt(max |eig(Xi1 Xi2)|).  Xi1 (4x5) and Xi2 (5x4) are assembled
-// implicitly: Xi = Xi1 Xi2 is formed directly from its nonzero blocks.
+// implicitly: Xi = Xi1 Xi2 is formed directly from its nonzero blocks.  With
+// G = A^T A and S = devG G (both symmetric), the distortion part of Xi's
+// velocity block is (dsigma/dA A: state.cpp:43-56, A(:,d)^T A = G(d,:))
+//   cs2 (S + e_d S(d,:) + G(:,d) G(d,:) / 3 + G(d,d) G),
+// six entries and a row instead of two 3x3 products.
 // Xo (m x m, row-major) and l2o, when given, receive Xi and its dominant
 // eigenvalue (for the adjoint's wave-speed derivative).
 template <bool TH>
 GPR_D double max_abs_eigs(const double *q, const Prim<TH> &s, int d, const DevPar &P,
                           double *Xo = nullptr, double *l2o = nullptr) {
-  const double *A = q + 5;
   const double r = s.r, ir = s.ir;
-  // G = A^T A (row d only needed) and dsigma/dA (state.cpp:43-56):
-  // ret = A devG with column d doubled + 1/3 A(:,d) G(d,:) + G(d,d) A
-  double Gd[3];
+  const double cs2 = s.cs2;
+  double Gd[3], Sd[3], X[3][3];
 #pragma unroll
-  for (int j = 0; j < 3; j++)
-    Gd[j] = A[d] * A[j] + A[3 + d] * A[3 + j] + A[6 + d] * A[6 + j];
-  double ret[9];
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-      ret[3 * i + j] = (j == d ? 2.0 : 1.0) * s.AdG[3 * i + j] +
-                       (1.0 / 3.0) * A[3 * i + d] * Gd[j] + Gd[d] * A[3 * i + j];
-  // Xi1 top-right block: -dsigmadA/rho = cs2 ret^T  ->  Mt[i][j] = cs2 ret[j][i]
-  double sg[3];
-  sigma_col(q, s, d, sg);
-  // dsigma/drho = (1/rho + dcs2/drho / cs2) sigma = (1 + beta)/rho sigma
-  double fr = (1.0 + P.beta) * ir;
-  double dsr[3] = {fr * sg[0], fr * sg[1], fr * sg[2]};
-  // c0^2 = (p/rho^2 - dE/drho) / dE/dp   (waves/speeds.cpp:8-18)
-  const EosRho &e = s.e;
-  double rG = r * e.G, irG2 = s.irG * s.irG;
-  double dnum = e.dpr * rG + (e.G + r * e.dG) * (s.p - e.pr);
-  double dedr = e.der - dnum * irG2;
-  double cs2 = s.cs2;
-  double dC0 = 0.0;
-  if (P.beta != 0.0) {
-    double dcs2 = P.beta * ir * cs2;
-    dC0 = (1.0 - P.beta / e.G) * dcs2 + P.beta / (e.G * e.G) * e.dG * cs2;
+  for (int i = 0; i < 3; i++) {
+    Gd[i] = sym3(s.G, i, d);
+    Sd[i] = sym3(s.S, i, d);
   }
-  double dEdr = dedr + 0.25 * dC0 * s.devGsq;
-  double c02 = (s.p * ir * ir - dEdr) * rG;  // dE/dp = 1/(rho Gamma)
-  // Xi2 row 1: b = sigma - rho dsigma/drho + rho c0^2 e_d ; h = calpha2 T Gamma
-  double b[3] = {sg[0] - r * dsr[0], sg[1] - r * dsr[1], sg[2] - r * dsr[2]};
-  b[d] += r * c02;
-  constexpr int m = TH ? 4 : 3;
-  double X[m][m];
-  // rows 0..2, cols 0..2: rho a_i delta_c0 + delta_i0 b_c/rho + (Mt A)_ic
+  const double Gdd = d == 0 ? Gd[0] : (d == 1 ? Gd[1] : Gd[2]);
 #pragma unroll
-  for (int i = 0; i < 3; i++)
+  for (int i = 0; i < 3; i++) {
+    const double g3 = (1.0 / 3.0) * Gd[i];
+#pragma unroll
+    for (int c = i; c < 3; c++)
+      X[i][c] = fma(Gdd, sym3(s.G, i, c), fma(g3, Gd[c], sym3(s.S, i, c)));
+  }
+  // + e_d S(d,:), and with the reference's columns and rows 0: Xi1 column 0
+  // (-dsigma/drho / rho, dsigma/drho = (1 + beta) sigma / rho) and Xi2 row 1
+  // (b / rho with b = sigma - rho dsigma/drho + rho c0^2 e_d)
+  const double b1 = P.b1;
+  if (d == 0) {
+    X[0][0] = fma(2.0 * b1, Sd[0], X[0][0]);
+    X[0][1] = fma(b1, Sd[1], X[0][1]);
+    X[0][2] = fma(b1, Sd[2], X[0][2]);
+    X[1][0] = X[0][1];
+    X[2][0] = X[0][2];
+    X[2][1] = X[1][2];
+  } else {
+    X[1][0] = X[0][1];
+    X[2][0] = X[0][2];
+    X[2][1] = X[1][2];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      double acc = cs2 * (ret[i] * A[c] + ret[3 + i] * A[3 + c] + ret[6 + i] * A[6 + c]);
-      if (c == 0)
-        acc += -dsr[i];  // rho * (-dsigma_i/drho / rho)
-      if (i == 0)
-        acc += b[c] * ir;
-      X[i][c] = acc;
+      if (d == 1)
+        X[1][c] += Sd[c];
+      else
+        X[2][c] += Sd[c];
     }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      X[i][0] = fma(b1, Sd[i], X[i][0]);
+    if (P.has_beta) {
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        X[0][c] = fma(P.beta, Sd[c], X[0][c]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      X[i][c] *= cs2;
+  // c0^2 = (p/rho^2 - dE/drho) / dE/dp   (waves/speeds.cpp:8-18)
+  const EosRho &e = s.e;
+  const double rG = r * e.G, irG2 = s.irG * s.irG;
+  double dnum = e.G * (s.p - e.pr);
+  if (P.EOS != 0)
+    dnum = e.dpr * rG + (e.G + r * e.dG) * (s.p - e.pr);
+  double dEdr = e.der - dnum * irG2;
+  if (P.has_beta) {
+    const double dcs2 = P.beta * ir * cs2;
+    const double dC0 = (1.0 - P.beta / e.G) * dcs2 + P.beta / (e.G * e.G) * e.dG * cs2;
+    dEdr += 0.25 * dC0 * s.devGsq;
+  }
+  const double c02 = (s.p * ir * ir - dEdr) * rG;  // dE/dp = 1/(rho Gamma)
+  if (d == 0)
+    X[0][0] += c02;
+  else if (d == 1)
+    X[0][1] += c02;
+  else
+    X[0][2] += c02;
+  // The heat-conduction row and column (TH): Xi couples the impulse to
+  // velocity row 0 only (x03), and back through T's row (x3).
+  double x03 = 0.0, x3[3] = {0.0, 0.0, 0.0}, x33 = 0.0;
   if (TH) {
-    double h = P.calpha2 * s.T * e.G;
-    double tp = ir * s.irG * P.icv;  // dT/dp / rho
-    double dTr = -dnum * irG2 * P.icv;
-    X[0][m - 1] = h * ir;
-    X[1][m - 1] = 0.0;
-    X[2][m - 1] = 0.0;
-    X[m - 1][0] = dTr + tp * b[0];
-    X[m - 1][1] = tp * b[1];
-    X[m - 1][2] = tp * b[2];
-    X[m - 1][m - 1] = tp * h;
-  }
-  if (Xo) {
+    const double h = P.calpha2 * s.T * e.G;  // Xi2 row 1
+    const double rtp = s.irG * P.icv;        // dT/dp
+    x03 = h * ir;
+    x33 = rtp * ir * h;
+    const double dTr = -dnum * irG2 * P.icv;
+    x3[0] = d == 0 ? fma(rtp, c02, dTr) : dTr;
+    x3[1] = d == 1 ? rtp * c02 : 0.0;
+    x3[2] = d == 2 ? rtp * c02 : 0.0;
+    if (P.has_beta) {
+      const double f = rtp * P.beta * cs2;
 #pragma unroll
-    for (int i = 0; i < m; i++)
-#pragma unroll
-      for (int c = 0; c < m; c++)
-        Xo[i * m + c] = X[i][c];
+      for (int c = 0; c < 3; c++)
+        x3[c] = fma(f, Sd[c], x3[c]);
+    }
   }
+  // The characteristic polynomial: that of the velocity block Y by its minors,
+  // bordered: det(x - Xi) = (x - x33) chi_Y(x) - x03 x3 . adj(x - Y) e_0.
+  // (explicit fused multiply-adds: the same rounding in every kernel)
+  const double m12 = fma(X[1][1], X[2][2], -(X[1][2] * X[2][1]));
+  const double n1 = fma(X[1][2], X[2][0], -(X[1][0] * X[2][2]));
+  const double n2 = fma(X[1][0], X[2][1], -(X[2][0] * X[1][1]));
+  const double m01 = fma(X[0][0], X[1][1], -(X[0][1] * X[1][0]));
+  const double m02 = fma(X[0][0], X[2][2], -(X[0][2] * X[2][0]));
+  const double s12 = X[1][1] + X[2][2];
+  const double t1 = X[0][0] + s12, t2 = m12 + (m01 + m02);
+  const double t3 = fma(X[0][2], n2, fma(X[0][1], n1, X[0][0] * m12));
   double l2;
-  if (!max_eig_laguerre<m, TH>(X, l2))
-    l2 = max_abs_eig<m>(X);  // QR fallback: complex or multiple dominant roots
+  bool ok;
+  if (TH) {
+    double u2 = x3[0] * s12, u3 = x3[0] * m12;
+    if (d != 0 || P.has_beta) {
+      u2 = fma(-x3[2], X[2][0], fma(-x3[1], X[1][0], u2));
+      u3 = fma(x3[2], n2, fma(x3[1], n1, u3));
+    }
+    const double c[4] = {t1 + x33, fma(-x03, x3[0], fma(x33, t1, t2)),
+                         fma(-x03, u2, fma(x33, t2, t3)), fma(-x03, u3, x33 * t3)};
+    ok = top_root<4>(c, l2);
+  } else {
+    const double c[3] = {t1, t2, t3};
+    ok = top_root<3>(c, l2);
+  }
+  if (Xo || !ok) {
+    constexpr int m = TH ? 4 : 3;
+    double Xm[m * m];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        Xm[i * m + c] = X[i][c];
+      if (TH) {
+        Xm[i * m + m - 1] = i == 0 ? x03 : 0.0;
+        Xm[(m - 1) * m + i] = x3[i];
+      }
+    }
+    if (TH)
+      Xm[m * m - 1] = x33;
+    if (!ok)
+      l2 = max_eig_general<m>(Xm);
+    if (Xo) {
+#pragma unroll
+      for (int k = 0; k < m * m; k++)
+        Xo[k] = Xm[k];
+    }
+  }
   if (l2o)
     *l2o = l2;
-  double lam = sqrt(l2);
-  double vd = s.v[d];
-  return vd > 0 ? vd + lam : lam - vd;
+  return sqrt64(l2) + fabs(s.v[d]);
 }
 
 }  // namespace gpr
