@@ -1940,12 +1940,9 @@ __global__ void __launch_bounds__(128) k_adj_pred_post(
 #pragma unroll
   for (int k = 0; k < V; k++)
     y[k] = C.dgder[i][i] * mu[k] + C.dgder[1 - i][i] * other[k];
-  // R(q) at this node: dg_rhs_node with dt = 1 and W w = 0
-  double R[V], zero[V];
-#pragma unroll
-  for (int k = 0; k < V; k++)
-    zero[k] = 0.0;
-  dg_rhs_node<L, 1>(q, zero, R, t, i, 0, 1.0, idx, 1.0, P, C);
+  // R(q) at this node: the predictor's residual with weight W_t W_i
+  double R[V];
+  dg_residual<L, 1>(q, R, wn, i, 0, idx * C.derv[0][1], 0.0, P);
   double dtb = 0.0;
 #pragma unroll
   for (int k = 0; k < V; k++)

@@ -196,7 +196,7 @@ GPR_D void weno_point(const double *__restrict__ d0, long sd, double *__restrict
     // tL / (tL + tR): one division where the reference takes three (equal
     // side weights; the result moves by an ulp at most)
     static_assert(LAMS == 1.0, "equal side weights");
-    const double iden = 1.0 / (tL + tR);
+    const double iden = rcp64(tL + tR);
     out[0] = (wL0 * tR + wR0 * tL) * iden;
     out[so] = (wL1 * tR + wR1 * tL) * iden;
     return;
@@ -445,6 +445,14 @@ constexpr double PICARD_DIVERGE = 1e3;
 GPR_D unsigned long long fp_abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
 }
+// |x| in FP32 from its high word, truncated (relative error below 2^-20); 0
+// below the FP32 range, F32_TOP from 2^127 on (infinities and NaNs included).
+constexpr float F32_TOP = 1.7014118346046923e38f;  // 2^127
+GPR_D float f32_abs_hi(double x) {
+  int e = (__double2hiint(x) & 0x7fffffff) - (896 << 20);
+  e = e < 0x00100000 ? 0 : (e > 0x0fe00000 ? 0x0fe00000 : e);
+  return __int_as_float(e << 3);
+}
 
 template <int V>
 GPR_D void shfl_vec(const double *src, double *dst, int lanemask) {
@@ -453,100 +461,76 @@ GPR_D void shfl_vec(const double *src, double *dst, int lanemask) {
     dst[k] = __shfl_xor_sync(0xffffffffu, src[k], lanemask);
 }
 
-// rhs at this thread's node with time weight wt (W_t): r = dt R + Ww
-// (AFFINE) or r = R; q unchanged.  The spatial partners are the lanes
-// g ^ XB (x) and g ^ YB (y), as in both lane layouts that call it.
-template <class L, int ND, bool AFFINE = true>
-GPR_D void dg_rhs_node_w(const double *q, const double *Ww, double *r, double wt, int i, int j,
-                         double dt, double idx, double idy, const DevPar &P, const Consts &C) {
+// The system's pointwise residual at this thread's node, scaled:
+//   r = sg (S(q) - B_x dq/dx [- B_y dq/dy] - dF/dx [- dG/dy]),
+// the derivatives along the cell's node lines (S left out without SOURCE).
+// The rhs of the Picard map is W_t W_s times this with sg = dt: W_t W_s (S - B
+// dq) - W_t [W_j] DG_DER F / dx ..., since DG_DER(i, m) = W_i psi_m'(x_i).  With
+// two nodes a line's derivative is the same difference quotient at both,
+// (q1 - q0) / (x1 - x0), so it is one subtraction with the partner's value
+// and the quotient goes into the coefficient (sign by the lane's end).
+// hx, hy: 1 / (dx (x1 - x0)), 1 / (dy (x1 - x0)).  The spatial partners are the
+// lanes g ^ XB (x) and g ^ YB (y) in every lane layout that calls it.
+template <class L, int ND, bool SOURCE = true>
+GPR_D void dg_residual(const double *q, double *r, double sg, int i, int j, double hx, double hy,
+                       const DevPar &P) {
   constexpr int V = L::V;
   // lane bit layout: 1D g = 2t + i ; 2D g = 4t + 2i + j
   constexpr int XB = ND == 1 ? 1 : 2;  // flips i
   constexpr int YB = 1;                // flips j (2D)
-  double tmp[V], other[V];
   Prim<L::THERMAL> s;
   prim<L::THERMAL>(q, P, s);
-  // W (S - B dq/dx [- B dq/dy]): the node weight wn folded into the
-  // source's scalar factors and the derivative coefficients (B is linear)
-  const double wn = ND == 1 ? wt * C.w[i] : wt * C.w[i] * C.w[j];
-  source<L::THERMAL, V>(q, s, P, r, wn);
-  // x derivative: DERVALS[i][m] q(t, m, j) / dx
-  shfl_vec<V>(q, other, XB);
-  {
-    double a = C.derv[i][i] * idx * wn, b = C.derv[i][1 - i] * idx * wn;
+  if (SOURCE) {
+    source<L::THERMAL, V>(q, s, P, r, sg);
+  } else {
 #pragma unroll
     for (int k = 0; k < V; k++)
-      tmp[k] = a * q[k] + b * other[k];
-    double bd[V];
-    bdot<V, L::LSET>(s.v, tmp, 0, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      r[k] -= bd[k];
+      r[k] = 0.0;
   }
-  if (ND == 2) {
-    shfl_vec<V>(q, other, YB);
-    double a = C.derv[j][j] * idy * wn, b = C.derv[j][1 - j] * idy * wn;
+#pragma unroll
+  for (int d = 0; d < ND; d++) {
+    const int lm = d == 0 ? XB : YB;
+    const double c = sg * ((d == 0 ? i : j) ? -(d == 0 ? hx : hy) : (d == 0 ? hx : hy));
+    // - B_d dq: columns other than d of the distortion, and the level sets
+    const double vc[3] = {s.v[0] * c, s.v[1] * c, s.v[2] * c};
+#pragma unroll
+    for (int k = 5; k < V; k++) {
+      const bool lset = k >= V - L::LSET;
+      if (!lset && (k >= 14 || (k - 5) % 3 == d))
+        continue;
+      const double df = __shfl_xor_sync(0xffffffffu, q[k], lm) - q[k];
+      r[k] = fma(-vc[d], df, r[k]);
+      if (!lset) {
+        const int col = (k - 5) % 3, dst = k - col + d;
+        r[dst] = fma(vc[col], df, r[dst]);
+      }
+    }
+    double F[V];
+    flux_set<L::THERMAL, V>(q, s, d, P, F);
 #pragma unroll
     for (int k = 0; k < V; k++)
-      tmp[k] = a * q[k] + b * other[k];
-    double bd[V];
-    bdot<V, L::LSET>(s.v, tmp, 1, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      r[k] -= bd[k];
-  }
-  // - W_t [W_j] DG_DER(i, m) F(t, m, j) / dx, as two fused multiply-adds
-  flux_set<L::THERMAL, V>(q, s, 0, P, tmp);
-  shfl_vec<V>(tmp, other, XB);
-  {
-    double wx = (ND == 1 ? wt : wt * C.w[j]) * idx;
-    double a = wx * C.dgder[i][i], b = wx * C.dgder[i][1 - i];
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      if (flux_support<L::THERMAL>(k, 0))
-        r[k] = fma(-b, other[k], fma(-a, tmp[k], r[k]));
-  }
-  if (ND == 2) {
-    flux_set<L::THERMAL, V>(q, s, 1, P, tmp);
-    shfl_vec<V>(tmp, other, YB);
-    double wy = wt * C.w[i] * idy;
-    double a = wy * C.dgder[j][j], b = wy * C.dgder[j][1 - j];
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      if (flux_support<L::THERMAL>(k, 1))
-        r[k] = fma(-b, other[k], fma(-a, tmp[k], r[k]));
-  }
-  if (AFFINE) {
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      r[k] = r[k] * dt + Ww[k];
+      if (flux_support<L::THERMAL>(k, d))
+        r[k] = fma(-c, __shfl_xor_sync(0xffffffffu, F[k], lm) - F[k], r[k]);
   }
 }
 
-template <class L, int ND>
-GPR_D void dg_rhs_node(const double *q, const double *Ww, double *r, int t, int i, int j,
-                       double dt, double idx, double idy, const DevPar &P, const Consts &C) {
-  dg_rhs_node_w<L, ND, true>(q, Ww, r, C.w[t], i, j, dt, idx, idy, P, C);
-}
-
-// q_new(t, s) = sum_m DG_MATinv[t][m] r(m, s) / W_s
+// The Picard map at this node, q_new(t, s) = sum_m DG_MATinv[t][m] (ENDVALS[0][m]
+// W_s w + dt R(m, s)) / W_s = w + sum_m DG_MATinv[t][m] r_m: the initial
+// condition's part is w itself (DG_MATinv maps ENDVALS[0] to 1).  r holds the
+// residual at sg = dt W_t and is overwritten by q_new.
 template <int V, int ND>
-GPR_D void dg_solve_node(const double *r, double *qn, int t, int i, int j, const Consts &C) {
+GPR_D void dg_solve_node(double *r, const double *w, int t, const Consts &C) {
   constexpr int TB = ND == 1 ? 2 : 4;  // flips t
-  double other[V];
-  shfl_vec<V>(r, other, TB);
-  // 1 / W_s: 2 and 4 for the N = 2 weights (exact)
-  double iws = ND == 1 ? 1.0 / C.w[i] : 1.0 / (C.w[i] * C.w[j]);
-  double a = C.dgmatinv[t][t] * iws, b = C.dgmatinv[t][1 - t] * iws;
+  const double a = C.dgmatinv[t][t], b = C.dgmatinv[t][1 - t];
 #pragma unroll
   for (int k = 0; k < V; k++)
-    qn[k] = a * r[k] + b * other[k];
+    r[k] = fma(b, __shfl_xor_sync(0xffffffffu, r[k], TB), fma(a, r[k], w[k]));
 }
 
 // First Picard iteration.  From the standard initial guess q(t, s) = w(s)
 // (initial_guess.cpp:4-15) the rhs at the two time nodes differs only by the
 // weight W_t, so one thread per (cell, spatial node) evaluates it once (time
-// weight 1) and writes q1 = DG_U^-1 (W w + dt R(q0)) at both time nodes
+// weight 1) and writes q1 = w + DG_MATinv W r at both time nodes
 // into qh; k_predictor_picard (first = 1) takes that as its first iterate
 // and applies the reference's stopping test to it as usual.
 template <class L, int ND, bool BATCH = false>
@@ -579,23 +563,17 @@ __global__ void __launch_bounds__(128) k_predictor_first(
 #pragma unroll
   for (int k = 0; k < V; k++)
     q[k] = valid ? wc[k] : 1.0;
-  dg_rhs_node_w<L, ND, false>(q, nullptr, r, 1.0, i, j, dt, idx, idy, P, C);
+  dg_residual<L, ND>(q, r, dt, i, j, idx * C.derv[0][1], idy * C.derv[0][1], P);
   if (!active)
     return;
-  // r_t = dt W_t R + ENDVALS[0][t] W_s w ; q1_t = sum_m DG_MATinv[t][m] r_m / W_s
-  const double Ws = ND == 1 ? C.w[i] : C.w[i] * C.w[j];
-  const double iws = ND == 1 ? 1.0 / C.w[i] : 1.0 / (C.w[i] * C.w[j]);
-  const double d0 = dt * C.w[0], d1 = dt * C.w[1];
-  const double f0 = C.endv[0][0] * Ws, f1 = C.endv[0][1] * Ws;
-  const double a00 = C.dgmatinv[0][0] * iws, a01 = C.dgmatinv[0][1] * iws;
-  const double a10 = C.dgmatinv[1][0] * iws, a11 = C.dgmatinv[1][1] * iws;
+  // q1_t = w + sum_m DG_MATinv[t][m] W_m r
+  const double a0 = fma(C.dgmatinv[0][1], C.w[1], C.dgmatinv[0][0] * C.w[0]);
+  const double a1 = fma(C.dgmatinv[1][1], C.w[1], C.dgmatinv[1][0] * C.w[0]);
   double *o0 = qh + (c * NP + g) * V, *o1 = qh + (c * NP + NS + g) * V;
 #pragma unroll
   for (int k = 0; k < V; k++) {
-    const double r0 = r[k] * d0 + f0 * q[k];
-    const double r1 = r[k] * d1 + f1 * q[k];
-    o0[k] = a00 * r0 + a01 * r1;
-    o1[k] = a10 * r0 + a11 * r1;
+    o0[k] = fma(a0, r[k], q[k]);
+    o1[k] = fma(a1, r[k], q[k]);
   }
 }
 
@@ -640,14 +618,14 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
   bool active = valid && (mask == nullptr || mask[c]);
   int t = g / NS, sidx = g % NS;
   int i = ND == 1 ? sidx : sidx / NN, j = ND == 1 ? 0 : sidx % NN;
-  double w[V], Ww[V], q[V], r[V], qn[V];
+  double w[V], q[V], qn[V];
   long cc = valid ? c : 0;
   const double *wc = wh + (cc * NS + sidx) * V;
-  double f = C.endv[0][t] * (ND == 1 ? C.w[i] : C.w[i] * C.w[j]);
+  const double sg = dt * C.w[t], hx = idx * C.derv[0][1], hy = idy * C.derv[0][1];
+  const float tolf = (float)C.dg_tol;
 #pragma unroll
   for (int k = 0; k < V; k++) {
     w[k] = valid ? wc[k] : 1.0;
-    Ww[k] = f * w[k];
     q[k] = (R.in && valid) ? qh[(cc * NP + g) * V + k] : w[k];
   }
   // groups are aligned to NP lanes; the group shares the convergence decision
@@ -669,7 +647,7 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
   // iteration converges still converges by Picard.
   const bool resume = R.in != nullptr && valid;
   const int it0 = resume ? R.it[c] : 0;
-  double dmin = resume ? R.dmin[c] : 1e300;
+  float dmin = resume ? (float)R.dmin[c] : F32_TOP;
   bool failed = false, deferred = false;
   for (int kq = 0;; kq++) {
     const int it = it0 + kq;
@@ -701,42 +679,49 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
       for (int k = 0; k < V; k++)
         qn[k] = active ? src[k] : q[k];
     } else {
-      dg_rhs_node<L, ND>(q, Ww, r, t, i, j, dt, idx, idy, P, C);
-      dg_solve_node<V, ND>(r, qn, t, i, j, C);
+      dg_residual<L, ND>(q, qn, sg, i, j, hx, hy, P);
+      dg_solve_node<V, ND>(qn, w, t, C);
     }
-    // the reference's test |q1 - q0| > dg_tol (1 + |q0|) per entry, the
-    // comparisons and maxima on the IEEE bit patterns of the non-negative
-    // operands (integer order equals numeric order there; NaN patterns sort
-    // above infinity and are excluded as the floating-point forms exclude
-    // them), so that only the subtraction and the threshold use the FP64 pipe
-    bool big = false, hasnan = false;
-    unsigned long long dmaxb = 0;
+    // The reference's test |q1 - q0| > dg_tol (1 + |q0|) per entry.  Only the
+    // difference needs FP64; an entry is decided in FP32 from the high words
+    // (relative error of both sides below 3e-6) wherever the two sides differ
+    // by more than 1e-5, and a cell that no entry so decides as changing takes
+    // the FP64 test for the entries left open, so the decision is the FP64 one
+    // (17 subtractions against 51 FP64 instructions).  The largest update,
+    // which only the divergence test reads, is kept in FP32.
+    bool big = false, open = false, hasnan = false;
+    float dmax = 0.0f;
 #pragma unroll
     for (int k = 0; k < V; k++) {
-      const unsigned long long ddb = fp_abs_bits(qn[k] - q[k]);
-      const unsigned long long thb = fp_abs_bits(C.dg_tol * (1.0 + fabs(q[k])));
-      if (ddb > thb && ddb <= FP_INF_BITS && thb <= FP_INF_BITS)
-        big = true;
-      if (fp_abs_bits(qn[k]) > FP_INF_BITS)
-        hasnan = true;
-      if (ddb <= FP_INF_BITS && ddb > dmaxb)
-        dmaxb = ddb;
+      const float df = f32_abs_hi(qn[k] - q[k]), qf = f32_abs_hi(q[k]);
+      const float th = fmaf(tolf, qf, tolf);
+      const bool ok = fmaxf(df, qf) < F32_TOP;
+      big = big || (ok && df > th * 1.00001f);
+      open = open || !ok || df > th * 0.99999f;
+      dmax = fmaxf(dmax, df);
     }
-#pragma unroll
-    for (int o = 1; o < NP; o <<= 1) {
-      const unsigned long long x = __shfl_xor_sync(0xffffffffu, dmaxb, o);
-      dmaxb = x > dmaxb ? x : dmaxb;
-    }
-    const double dmax = __longlong_as_double((long long)dmaxb);
     unsigned bigm = __ballot_sync(0xffffffffu, big) & gmask;
-    unsigned nanm = __ballot_sync(0xffffffffu, hasnan) & gmask;
-    if (!done && bigm && it >= 3 && dmax > PICARD_DIVERGE * dmin) {
+    if (open && !bigm) {
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        if (fabs(qn[k] - q[k]) > C.dg_tol * (1.0 + fabs(q[k])))
+          big = true;
+        if (fp_abs_bits(qn[k]) > FP_INF_BITS)
+          hasnan = true;
+      }
+    }
+    bigm = __ballot_sync(0xffffffffu, big) & gmask;
+    const unsigned nanm = __ballot_sync(0xffffffffu, hasnan) & gmask;
+#pragma unroll
+    for (int o = 1; o < NP; o <<= 1)
+      dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+    if (!done && bigm && it >= 3 && dmax > (float)PICARD_DIVERGE * dmin) {
       nan_seen = true;  // hand over to the Newton pass
       done = true;
       iters = it + 1;
     }
     if (!done)
-      dmin = dmax < dmin ? dmax : dmin;
+      dmin = fminf(dmin, dmax);
     if (!done) {
       iters = it + 1;
       if (bigm) {
@@ -792,7 +777,6 @@ __global__ void __launch_bounds__(128) k_midstep(double *__restrict__ wh, long n
                                                  double idy, DevPar P, Consts C) {
   constexpr int V = L::V;
   constexpr int NS = ND == 1 ? NN : NN * NN;
-  constexpr int XB = ND == 1 ? 1 : 2, YB = 1;
   if (dt_dev)
     dt = *dt_dev;
   long gt = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -802,52 +786,16 @@ __global__ void __launch_bounds__(128) k_midstep(double *__restrict__ wh, long n
   const long cc = valid ? c : 0;
   const bool active = valid && (mask == nullptr || mask[cc]);
   const int a = ND == 1 ? g : g / NN, b = ND == 1 ? 0 : g % NN;
-  double w[V], F[V], other[V], dw[V], inc[V];
+  double w[V], r[V];
   double *wc = wh + (cc * NS + g) * V;
 #pragma unroll
   for (int k = 0; k < V; k++)
     w[k] = wc[k];
-  Prim<L::THERMAL> s;
-  prim<L::THERMAL>(w, P, s);
-#pragma unroll
-  for (int k = 0; k < V; k++)
-    F[k] = 0.0;
-  flux_add<L::THERMAL, V>(w, s, 0, P, F);
-  // x: d/dx of w and F over the x partner
-  {
-    const double ca = C.derv[a][a], cb = C.derv[a][1 - a];
-    shfl_vec<V>(w, other, XB);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      dw[k] = ca * w[k] + cb * other[k];
-    shfl_vec<V>(F, other, XB);
-    double bd[V];
-    bdot<V, L::LSET>(s.v, dw, 0, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      inc[k] = ((ca * F[k] + cb * other[k]) + bd[k]) * idx;
-  }
-  if (ND == 2) {
-    const double ca = C.derv[b][b], cb = C.derv[b][1 - b];
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      F[k] = 0.0;
-    flux_add<L::THERMAL, V>(w, s, 1, P, F);
-    shfl_vec<V>(w, other, YB);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      dw[k] = ca * w[k] + cb * other[k];
-    shfl_vec<V>(F, other, YB);
-    double bd[V];
-    bdot<V, L::LSET>(s.v, dw, 1, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      inc[k] += ((ca * F[k] + cb * other[k]) + bd[k]) * idy;
-  }
+  dg_residual<L, ND, false>(w, r, 0.5 * dt, a, b, idx * C.derv[0][1], idy * C.derv[0][1], P);
   if (active) {
 #pragma unroll
     for (int k = 0; k < V; k++)
-      wc[k] = w[k] - dt / 2 * inc[k];
+      wc[k] = w[k] + r[k];
   }
 }
 
@@ -1031,9 +979,7 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
   float *Jb = Jm + NJ * NJ;                   // 6
   const unsigned lane = threadIdx.x & 31u;
   const unsigned gmask = ((NP == 32) ? 0xffffffffu : ((1u << NP) - 1u)) << (lane & ~(NP - 1u));
-  const double f = C.endv[0][t] * (ND == 1 ? C.w[i] : C.w[i] * C.w[j]);
-  const double ws = ND == 1 ? C.w[i] : C.w[i] * C.w[j];
-  const double iws = 1.0 / ws;
+  const double f = C.endv[0][t];
   const double M0 = C.dgmat[t][t], M1 = C.dgmat[t][1 - t];
   const long cells_per_block = blockDim.x / NP;
   // persistent: blocks stride over the cells; the loop bound is uniform in
@@ -1053,12 +999,13 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
     const double dt = BATCH ? B.clk[5 * inst + 1] : dt_in;
     const double idx = BATCH ? B.idx[inst] : idx_in;
     const double a_t = dt * C.w[t];
-    double Ww[V], q[V], r[V], other[V];
+    const double hx = idx * C.derv[0][1], hy = idy * C.derv[0][1];
+    double fw[V], q[V], r[V], other[V];
     const double *wc = wh + (cc * NS + sidx) * V;
 #pragma unroll
     for (int k = 0; k < V; k++) {
       double w = active ? wc[k] : 1.0;
-      Ww[k] = f * w;
+      fw[k] = f * w;
       q[k] = w;
     }
     bool done = !active;
@@ -1067,12 +1014,13 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
     for (int it = 0; it < C.stiff_it; it++) {
       if (__all_sync(0xffffffffu, done))
         break;
-      dg_rhs_node<L, ND>(q, Ww, r, t, i, j, dt, idx, idy, P, C);
-      // residual g = r - W_s sum_m DG_MAT[t][m] q(m)
+      dg_residual<L, ND>(q, r, a_t, i, j, hx, hy, P);
+      // the fixed point's residual over W_s: r + ENDVALS[0][t] w - sum_m
+      // DG_MAT[t][m] q(m)
       shfl_vec<V>(q, other, TB);
 #pragma unroll
       for (int k = 0; k < V; k++)
-        r[k] -= ws * (M0 * q[k] + M1 * other[k]);
+        r[k] += fma(-M1, other[k], fma(-M0, q[k], fw[k]));
       if (!done) {
         Prim<L::THERMAL> st;
         prim<L::THERMAL>(q, P, st);
@@ -1083,11 +1031,11 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
                                         Jm + t * 3 * NJ + t * 3, NJ);
 #pragma unroll
         for (int a = 0; a < 9; a++)
-          Ab[t * 9 + a] = (float)(r[5 + a] * iws);
+          Ab[t * 9 + a] = (float)r[5 + a];
         if (L::THERMAL) {
 #pragma unroll
           for (int a = 0; a < 3; a++)
-            Jb[t * 3 + a] = (float)(r[14 + a] * iws);
+            Jb[t * 3 + a] = (float)r[14 + a];
         }
       }
       __syncwarp();
@@ -1151,10 +1099,10 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
           solved = smem_solve<3>(RJm, NJ, RJb);
       }
       __syncwarp();
-      // non-stiff variables: DG_MAT^-1 g / W_s (partner time node's residual)
+      // non-stiff variables: DG_MAT^-1 g (partner time node's residual)
       shfl_vec<V>(r, other, TB);
       double delta[V];
-      double ia = C.dgmatinv[t][t] * iws, ib = C.dgmatinv[t][1 - t] * iws;
+      const double ia = C.dgmatinv[t][t], ib = C.dgmatinv[t][1 - t];
 #pragma unroll
       for (int k = 0; k < V; k++)
         delta[k] = ia * r[k] + ib * other[k];
@@ -1498,7 +1446,7 @@ GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
   bool live = active && (time_dg || t == 0);
   int tt = time_dg ? t : 0;
   const double *qc = qh + ((cb * nt + tt) * NS + sidx) * V;
-  double q[V], other[V], dq[V], acc[V];
+  double q[V], acc[V];
 #pragma unroll
   for (int k = 0; k < V; k++)
     acc[k] = 0.0;
@@ -1514,29 +1462,25 @@ GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
     const double wn = ND == 1 ? wt * C.w[i] : wt * C.w[i] * C.w[j];
     if (sources)
       source<L::THERMAL, V>(q, s, P, acc, wn);
-    shfl_vec<V>(q, other, XB);
-    {
-      double a = C.derv[i][i] * idx * wn, b = C.derv[i][1 - i] * idx * wn;
+    // - B dq by the node lines' differences, as dg_residual
 #pragma unroll
-      for (int k = 0; k < V; k++)
-        dq[k] = a * q[k] + b * other[k];
-      double bd[V];
-      bdot<V, L::LSET>(s.v, dq, 0, bd);
+    for (int d = 0; d < ND; d++) {
+      const int lm = d == 0 ? XB : YB;
+      const double h = (d == 0 ? idx : idy) * C.derv[0][1];
+      const double cf = wn * ((d == 0 ? i : j) ? -h : h);
+      const double vc[3] = {s.v[0] * cf, s.v[1] * cf, s.v[2] * cf};
 #pragma unroll
-      for (int k = 0; k < V; k++)
-        acc[k] -= bd[k];
-    }
-    if (ND == 2) {
-      shfl_vec<V>(q, other, YB);
-      double a = C.derv[j][j] * idy * wn, b = C.derv[j][1 - j] * idy * wn;
-#pragma unroll
-      for (int k = 0; k < V; k++)
-        dq[k] = a * q[k] + b * other[k];
-      double bd[V];
-      bdot<V, L::LSET>(s.v, dq, 1, bd);
-#pragma unroll
-      for (int k = 0; k < V; k++)
-        acc[k] -= bd[k];
+      for (int k = 5; k < V; k++) {
+        const bool lset = k >= V - L::LSET;
+        if (!lset && (k >= 14 || (k - 5) % 3 == d))
+          continue;
+        const double df = __shfl_xor_sync(0xffffffffu, q[k], lm) - q[k];
+        acc[k] = fma(-vc[d], df, acc[k]);
+        if (!lset) {
+          const int col = (k - 5) % 3, dst = k - col + d;
+          acc[dst] = fma(vc[col], df, acc[dst]);
+        }
+      }
     }
 #pragma unroll
     for (int k = 0; k < V; k++)
