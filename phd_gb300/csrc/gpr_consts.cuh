@@ -12,6 +12,7 @@
 namespace gpr {
 
 constexpr int NN = 2;  // Gauss nodes / basis functions (the reference's N)
+constexpr double GAUSS_W = 0.5;  // both weights of the two-point rule on [0, 1]
 
 struct Consts {
   double nodes[NN], w[NN];       // Gauss-Legendre on [0, 1]
@@ -37,7 +38,7 @@ inline Consts make_consts() {
   const double s = 1.0 / sqrt(3.0);
   c.nodes[0] = (1.0 - s) / 2.0;
   c.nodes[1] = (1.0 + s) / 2.0;
-  c.w[0] = c.w[1] = 0.5;
+  c.w[0] = c.w[1] = GAUSS_W;
   const double x0 = c.nodes[0], x1 = c.nodes[1];
   const double h = x1 - x0;
   // psi_0 = (x1 - x)/h, psi_1 = (x - x0)/h

@@ -325,7 +325,9 @@ template <int n, int G> struct GroupReduceScatter {
 
 // The face contributions kk (b + f) (left cell) and kk (b - f) (right cell)
 // summed over the G quadrature lanes of a face (r = lane within the face)
-// and written to out[0..V-1] / out[V..2V-1] by the lanes that hold them.
+// and written to out[0..V-1] / out[V..2V-1] by the lanes that hold them.  The
+// two-point rule's weights are equal, so kk is the same on every lane of a face
+// and multiplies the 2 V / G sums a lane ends with, not its 2 V terms.
 template <int V, int G>
 GPR_D void face_reduce_store(const double *b, const double *f, double kk, bool active,
                              bool valid, int r, double *out) {
@@ -333,8 +335,8 @@ GPR_D void face_reduce_store(const double *b, const double *f, double kk, bool a
   double v[2 * NPR * G];
 #pragma unroll
   for (int k = 0; k < NPR * G; k++) {
-    v[2 * k] = (active && k < V) ? kk * b[k] : 0.0;
-    v[2 * k + 1] = (active && k < V) ? kk * f[k] : 0.0;
+    v[2 * k] = (active && k < V) ? b[k] : 0.0;
+    v[2 * k + 1] = (active && k < V) ? f[k] : 0.0;
   }
   GroupReduceScatter<2 * NPR * G, G>::run(v, r);
   if (!valid)
@@ -343,8 +345,8 @@ GPR_D void face_reduce_store(const double *b, const double *f, double kk, bool a
   for (int p = 0; p < NPR; p++) {
     const int k = r * NPR + p;
     if (k < V) {
-      out[k] = v[2 * p] + v[2 * p + 1];
-      out[V + k] = v[2 * p] - v[2 * p + 1];
+      out[k] = kk * (v[2 * p] + v[2 * p + 1]);
+      out[V + k] = kk * (v[2 * p] - v[2 * p + 1]);
     }
   }
 }
@@ -361,8 +363,8 @@ GPR_D void face_reduce_apply(const double *b, const double *f, double kk, bool a
   double v[2 * NPR * G];
 #pragma unroll
   for (int k = 0; k < NPR * G; k++) {
-    v[2 * k] = (active && k < V) ? kk * b[k] : 0.0;
-    v[2 * k + 1] = (active && k < V) ? kk * f[k] : 0.0;
+    v[2 * k] = (active && k < V) ? b[k] : 0.0;
+    v[2 * k + 1] = (active && k < V) ? f[k] : 0.0;
   }
   GroupReduceScatter<2 * NPR * G, G>::run(v, r);
   if (!face_on)
@@ -372,9 +374,9 @@ GPR_D void face_reduce_apply(const double *b, const double *f, double kk, bool a
     const int k = r * NPR + p;
     if (k < V) {
       if (uL)
-        uL[k] -= v[2 * p] + v[2 * p + 1];
+        uL[k] = fma(-kk, v[2 * p] + v[2 * p + 1], uL[k]);
       if (uR)
-        uR[k] -= v[2 * p] - v[2 * p + 1];
+        uR[k] = fma(-kk, v[2 * p] - v[2 * p + 1], uR[k]);
     }
   }
 }
@@ -1179,41 +1181,50 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
 // of a face reduce with shuffles.  Face results: fb[face][0][k] (to the left
 // cell, subtracted) and fb[face][1][k] (to the right cell).
 
-template <class L>
-GPR_D void interface_point(const double *ql, const double *qr, int d, const DevPar &P,
-                           const Consts &C, double *f, double *b) {
+// Bint = sum_n W_n B_d(qL + x_n dq) dq, dq = qR - qL (fluxes.cpp:9-20).  B_d
+// is linear in the velocity and needs nothing else of the state, so the path
+// nodes' velocities are averaged first and one product taken; b is written on
+// the rows where it can be nonzero and zeroed elsewhere.
+template <class L, int NQ>
+GPR_D void path_product(const double *ql, const double *dq, int d, const double *nodes,
+                        const double *wts, double *b) {
+  double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int n = 0; n < NQ; n++) {
+    const double wr = wts[n] * rcp64(fma(nodes[n], dq[0], ql[0]));
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      v[c] = fma(wr, fma(nodes[n], dq[2 + c], ql[2 + c]), v[c]);
+  }
+  bdot<L::V, L::LSET>(v, dq, d, b);
+}
+
+// Rusanov interface terms at one point: f = D + F(qL) + F(qR) and b = Bint.
+template <class L, int NQ>
+GPR_D void rusanov_point(const double *ql, const double *qr, int d, const DevPar &P,
+                         const double *nodes, const double *wts, double *f, double *b) {
   constexpr int V = L::V;
   Prim<L::THERMAL> sl, sr;
   prim<L::THERMAL>(ql, P, sl);
   prim<L::THERMAL>(qr, P, sr);
-  double m1 = max_abs_eigs<L::THERMAL>(ql, sl, d, P);
-  double m2 = max_abs_eigs<L::THERMAL>(qr, sr, d, P);
-  double m = m1 > m2 ? m1 : m2;  // std::max(m1, m2)
-#pragma unroll
-  for (int k = 0; k < V; k++)
-    f[k] = m * (ql[k] - qr[k]);
-  flux_add<L::THERMAL, V>(ql, sl, d, P, f);
-  flux_add<L::THERMAL, V>(qr, sr, d, P, f);
-  // Bint: sum_i W_i B(qL + x_i dq) dq, dq = qR - qL; B needs only v
-  double dq[V];
+  const double m1 = max_abs_eigs<L::THERMAL>(ql, sl, d, P);
+  const double m2 = max_abs_eigs<L::THERMAL>(qr, sr, d, P);
+  const double m = m1 > m2 ? m1 : m2;  // std::max(m1, m2)
+  double fl[V], dq[V];
+  flux_set<L::THERMAL, V>(ql, sl, d, P, fl);
+  flux_set<L::THERMAL, V>(qr, sr, d, P, f);
 #pragma unroll
   for (int k = 0; k < V; k++) {
     dq[k] = qr[k] - ql[k];
-    b[k] = 0.0;
+    f[k] = flux_support<L::THERMAL>(k, d) ? fma(-m, dq[k], fl[k] + f[k]) : -m * dq[k];
   }
-#pragma unroll
-  for (int n = 0; n < NN; n++) {
-    double rho = ql[0] + C.nodes[n] * dq[0];
-    double ir = 1.0 / rho;
-    double v[3] = {(ql[2] + C.nodes[n] * dq[2]) * ir, (ql[3] + C.nodes[n] * dq[3]) * ir,
-                   (ql[4] + C.nodes[n] * dq[4]) * ir};
-    double bd[V];
-    bdot<V, L::LSET>(v, dq, d, bd);
-#pragma unroll
-    for (int k = 5; k < V; k++)  // B x is zero outside the distortion and level-set rows
-      if (k < 14 || k >= V - L::LSET)
-        b[k] += C.w[n] * bd[k];
-  }
+  path_product<L, NQ>(ql, dq, d, nodes, wts, b);
+}
+
+template <class L>
+GPR_D void interface_point(const double *ql, const double *qr, int d, const DevPar &P,
+                           const Consts &C, double *f, double *b) {
+  rusanov_point<L, NN>(ql, qr, d, P, C.nodes, C.w, f, b);
 }
 
 // 1D faces i = 0..nx between predictor cells i and i+1.  NQ = N lanes per
@@ -1221,7 +1232,7 @@ GPR_D void interface_point(const double *ql, const double *qr, int d, const DevP
 template <class L, bool BATCH = false>
 __global__ void __launch_bounds__(128) k_faces1d(
     double *__restrict__ fb, const double *__restrict__ qh, long nface,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double idx,
     int time_dg, DevPar Pv, Consts C, Batch B) {
   constexpr int V = L::V;
   constexpr int NQ = NN;
@@ -1239,7 +1250,7 @@ __global__ void __launch_bounds__(128) k_faces1d(
   if (BATCH) {
     fi = B.off_b[inst] + (fo - B.off_f[inst]);
     dt = B.clk[5 * inst + 1];
-    dx = 1.0 / B.idx[inst];
+    idx = B.idx[inst];
   }
   bool active = valid && (mask == nullptr || (mask[fi] && mask[fi + 1])) && (time_dg || t == 0);
   int nt = time_dg ? NN : 1;
@@ -1251,7 +1262,7 @@ __global__ void __launch_bounds__(128) k_faces1d(
     ql[k] = C.endv[1][0] * ql_[k] + C.endv[1][1] * ql_[V + k];
     qr[k] = C.endv[0][0] * qr_[k] + C.endv[0][1] * qr_[V + k];
   }
-  double kk = (time_dg ? dt * C.w[t] : dt) / (2.0 * dx);
+  const double kk = dt * idx * (time_dg ? 0.5 * GAUSS_W : 0.5);
   if (active) {
     interface_point<L>(ql, qr, 0, P, C, f, b);
   } else {
@@ -1271,7 +1282,7 @@ __global__ void __launch_bounds__(128) k_faces1d(
 template <class L, bool BATCH>
 GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict__ qh,
                               long nface, const uint8_t *__restrict__ mask, double dt,
-                              double dx, int time_dg, const DevPar &Pv, const Consts &C,
+                              double idx, int time_dg, const DevPar &Pv, const Consts &C,
                               const Batch &B, long face, int lq, bool inrange, long fbase) {
   constexpr int V = L::V;
   static_assert(NN == 2, "two time nodes and two path nodes");
@@ -1285,7 +1296,7 @@ GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict_
   if (BATCH) {
     fi = B.off_b[inst] + (fo - B.off_f[inst]);
     dt = B.clk[5 * inst + 1];
-    dx = 1.0 / B.idx[inst];
+    idx = B.idx[inst];
   }
   bool active = valid && (mask == nullptr || (mask[fi] && mask[fi + 1])) && (time_dg || t == 0);
   int nt = time_dg ? NN : 1;
@@ -1297,9 +1308,8 @@ GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict_
     ql[k] = C.endv[1][0] * ql_[k] + C.endv[1][1] * ql_[V + k];
     qr[k] = C.endv[0][0] * qr_[k] + C.endv[0][1] * qr_[V + k];
     dq[k] = qr[k] - ql[k];
-    b[k] = 0.0;
   }
-  const double kk = (time_dg ? dt * C.w[t] : dt) / (2.0 * dx);
+  const double kk = dt * idx * (time_dg ? 0.5 * GAUSS_W : 0.5);
   const double *qs = side ? qr : ql;
   Prim<L::THERMAL> ps;
   prim<L::THERMAL>(qs, P, ps);
@@ -1308,23 +1318,18 @@ GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict_
   const double m1 = side ? lo : lam, m2 = side ? lam : lo;  // lambda(qL), lambda(qR)
   const double m = m1 > m2 ? m1 : m2;                        // std::max(m1, m2)
   flux_set<L::THERMAL, V>(qs, ps, 0, P, f);
-  if (side == 0) {
+  // the dissipation -m dq once per point (side 0)
+  const double ms = side == 0 ? -m : 0.0;
 #pragma unroll
-    for (int k = 0; k < V; k++)
-      f[k] += m * (ql[k] - qr[k]);
-  }
+  for (int k = 0; k < V; k++)
+    f[k] = flux_support<L::THERMAL>(k, 0) ? fma(ms, dq[k], f[k]) : ms * dq[k];
   // Bint node `side`: W_n B(qL + x_n dq) dq   (fluxes.cpp:9-20)
   {
-    const double xn = C.nodes[side], wn = C.w[side];
-    double ir = 1.0 / (ql[0] + xn * dq[0]);
-    double v[3] = {(ql[2] + xn * dq[2]) * ir, (ql[3] + xn * dq[3]) * ir,
-                   (ql[4] + xn * dq[4]) * ir};
-    double bd[V];
-    bdot<V, L::LSET>(v, dq, 0, bd);
-#pragma unroll
-    for (int k = 5; k < V; k++)
-      if (k < 14 || k >= V - L::LSET)
-        b[k] = wn * bd[k];
+    const double xn = C.nodes[side];
+    const double wr = GAUSS_W * rcp64(fma(xn, dq[0], ql[0]));
+    const double v[3] = {fma(xn, dq[2], ql[2]) * wr, fma(xn, dq[3], ql[3]) * wr,
+                         fma(xn, dq[4], ql[4]) * wr};
+    bdot<V, L::LSET>(v, dq, 0, b);
   }
   face_reduce_store<V, 4>(b, f, kk, active, valid, lq, fb + (fo - fbase) * 2 * V);
 }
@@ -1332,26 +1337,27 @@ GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict_
 template <class L, bool BATCH = false>
 __global__ void __launch_bounds__(128) k_faces1d_split(
     double *__restrict__ fb, const double *__restrict__ qh, long nface,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double idx,
     int time_dg, DevPar Pv, Consts C, Batch B) {
   if (dt_dev)
     dt = *dt_dev;
   long gt = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  faces1d_split_body<L, BATCH>(fb, qh, nface, mask, dt, dx, time_dg, Pv, C, B, gt / 4,
+  faces1d_split_body<L, BATCH>(fb, qh, nface, mask, dt, idx, time_dg, Pv, C, B, gt / 4,
                                threadIdx.x % 4, true, 0);
 }
 
-// 2D faces: direction dir, faces (i, j) of the (nx+1) x (ny+1) face grid,
-// between predictor cells (i, j) and (i+1, j) (dir 0) or (i, j+1) (dir 1);
-// NQ = N*N lanes per face (time node t, transverse node s).  parity < 0:
+// 2D faces: direction DIR (compile-time: a run-time axis makes the
+// kernel keep 1.3 KB of its state in local memory), faces (i, j) of the (nx+1) x (ny+1) face grid,
+// between predictor cells (i, j) and (i+1, j) (DIR 0) or (i, j+1) (DIR 1);
+// ih = 1 / dx_DIR; NQ = N*N lanes per face (time node t, transverse node s).  parity < 0:
 // every face, contributions written to fb[face][2][V] (the face-flux
-// entry points); parity 0 / 1: the faces of that parity along dir, applied
+// entry points); parity 0 / 1: the faces of that parity along DIR, applied
 // to u (passed as fb) in place, the conservative update of interfs2.
-template <class L>
+template <class L, int DIR>
 __global__ void __launch_bounds__(128) k_faces2d(
-    double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny, int dir,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
-    double dy, int time_dg, DevPar P, Consts C, int parity = -1) {
+    double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double ih,
+    int time_dg, DevPar P, Consts C, int parity = -1) {
   constexpr int V = L::V;
   constexpr int NQ = NN * NN;
   if (dt_dev)
@@ -1359,13 +1365,13 @@ __global__ void __launch_bounds__(128) k_faces2d(
   long gt = blockIdx.x * (long)blockDim.x + threadIdx.x;
   int lq = threadIdx.x % NQ;
   int t = lq / NN, s = lq % NN;
-  const Face2 F = face2_of(gt / NQ, nx, ny, dir, parity);
+  const Face2 F = face2_of(gt / NQ, nx, ny, DIR, parity);
   const bool valid = F.valid;
   const long fi = F.fi;
   const int i = F.i, j = F.j;
   long cb = (long)i * (ny + 2) + j;
-  long cn = dir == 0 ? cb + (ny + 2) : cb + 1;
-  bool geo = dir == 0 ? (j > 0) : (i > 0);
+  long cn = DIR == 0 ? cb + (ny + 2) : cb + 1;
+  bool geo = DIR == 0 ? (j > 0) : (i > 0);
   const bool face_on = valid && geo && (mask == nullptr || (mask[cb] && mask[cn]));
   bool active = face_on && (time_dg || t == 0);
   int nt = time_dg ? NN : 1;
@@ -1373,18 +1379,18 @@ __global__ void __launch_bounds__(128) k_faces2d(
   const double *q0 = qh + (cb * nt + tt) * NN * NN * V;
   const double *q1 = qh + (cn * nt + tt) * NN * NN * V;
   double ql[V], qr[V], f[V], b[V];
-  // endpts2d (evaluations.cpp:20-35): dir 0 -> nodes (m, s); dir 1 -> (s, m)
-  long o0 = dir == 0 ? (long)s * V : (long)s * NN * V;
-  long st = dir == 0 ? (long)NN * V : (long)V;
+  // endpts2d (evaluations.cpp:20-35): DIR 0 -> nodes (m, s); DIR 1 -> (s, m)
+  long o0 = DIR == 0 ? (long)s * V : (long)s * NN * V;
+  long st = DIR == 0 ? (long)NN * V : (long)V;
 #pragma unroll
   for (int k = 0; k < V; k++) {
     ql[k] = C.endv[1][0] * q0[o0 + k] + C.endv[1][1] * q0[o0 + st + k];
     qr[k] = C.endv[0][0] * q1[o0 + k] + C.endv[0][1] * q1[o0 + st + k];
   }
-  double wt = time_dg ? dt * C.w[t] : dt;
-  double kk = wt / (2.0 * (dir == 0 ? dx : dy)) * C.w[s];
+  // W_t W_s dt / (2 h)
+  const double kk = dt * ih * (time_dg ? 0.5 * GAUSS_W * GAUSS_W : 0.5 * GAUSS_W);
   if (active) {
-    interface_point<L>(ql, qr, dir, P, C, f, b);
+    interface_point<L>(ql, qr, DIR, P, C, f, b);
   } else {
 #pragma unroll
     for (int k = 0; k < V; k++)
@@ -1394,7 +1400,7 @@ __global__ void __launch_bounds__(128) k_faces2d(
     face_reduce_store<V, NQ>(b, f, kk, active, valid, lq, fb + fi * 2 * V);
   } else {
     double *uL, *uR;
-    face2_cells(fb, i, j, nx, ny, dir, V, uL, uR);
+    face2_cells(fb, i, j, nx, ny, DIR, V, uL, uR);
     face_reduce_apply<V, NQ>(b, f, kk, active, face_on, lq, uL, uR);
   }
 }
@@ -1406,15 +1412,16 @@ constexpr int FV_CENTERS = 1, FV_INTERFS = 2, FV_BOTH = 3;
 
 // Cell pass: one thread per (cell, space-time node): the volume term
 // w_t w_s (S - B dq/dx [- B dq/dy]) (fv.cpp:11-109), reduced over the cell's
-// NP lanes, then u += volume - face contributions (the parts selected).
+// NP lanes, then u += volume - face contributions (the parts selected).  hx,
+// hy: 1 / (dx (x1 - x0)), 1 / (dy (x1 - x0)), as in dg_residual.
 // The body for cell c (u index), lane g of its NP lanes; fbx[(fo - fbase)]
 // holds the 1D face on the cell's left (fbase: the first face of a tile
 // staged in shared memory, else 0).
 template <class L, int ND, bool BATCH>
 GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
                       const double *__restrict__ fbx, const double *__restrict__ fby, long nx,
-                      int ny, const uint8_t *__restrict__ mask, double dt, double dx,
-                      double dy, int sources, int time_dg, const DevPar &Pv, const Consts &C,
+                      int ny, const uint8_t *__restrict__ mask, double dt, double hx,
+                      double hy, int sources, int time_dg, const DevPar &Pv, const Consts &C,
                       const Batch &B, int parts, long c, int g, bool inrange, long fbase) {
   constexpr int V = L::V;
   constexpr int NS = ND == 1 ? NN : NN * NN;
@@ -1426,8 +1433,6 @@ GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
   long cc = valid ? c : 0;
   const int inst = BATCH ? B.inst_u[cc] : 0;
   const DevPar &P = BATCH ? B.P[inst] : Pv;
-  double idx = 1.0 / dx;
-  const double idy = 1.0 / dy;
   long ci = ND == 1 ? cc : (cc / ny);
   int cj = ND == 1 ? 0 : (int)(cc % ny);
   long cb = ND == 1 ? ci + 1 : (long)(ci + 1) * (ny + 2) + (cj + 1);
@@ -1437,7 +1442,7 @@ GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
     cb = B.off_b[inst] + li + 1;
     fo = B.off_f[inst] + li;
     dt = B.clk[5 * inst + 1];
-    idx = B.idx[inst];
+    hx = B.idx[inst] * C.derv[0][1];
   }
   bool active = valid && (mask == nullptr || mask[cb]);
   int t = g / NS, sidx = g % NS;
@@ -1458,15 +1463,14 @@ GPR_D void cells_body(double *__restrict__ u, const double *__restrict__ qh,
     prim<L::THERMAL>(q, P, s);
     // wn (S - B dq/dx [- B dq/dy]), wn folded into the source's scalar
     // factors and the derivative coefficients (B is linear)
-    const double wt = time_dg ? dt * C.w[t] : dt;
-    const double wn = ND == 1 ? wt * C.w[i] : wt * C.w[i] * C.w[j];
+    const double wn = dt * ((time_dg ? GAUSS_W : 1.0) * (ND == 1 ? GAUSS_W : GAUSS_W * GAUSS_W));
     if (sources)
       source<L::THERMAL, V>(q, s, P, acc, wn);
     // - B dq by the node lines' differences, as dg_residual
 #pragma unroll
     for (int d = 0; d < ND; d++) {
       const int lm = d == 0 ? XB : YB;
-      const double h = (d == 0 ? idx : idy) * C.derv[0][1];
+      const double h = d == 0 ? hx : hy;
       const double cf = wn * ((d == 0 ? i : j) ? -h : h);
       const double vc[3] = {s.v[0] * cf, s.v[1] * cf, s.v[2] * cf};
 #pragma unroll
@@ -1550,13 +1554,13 @@ template <class L, int ND, bool BATCH = false>
 __global__ void __launch_bounds__(128) k_cells(
     double *__restrict__ u, const double *__restrict__ qh, const double *__restrict__ fbx,
     const double *__restrict__ fby, long nx, int ny, const uint8_t *__restrict__ mask,
-    double dt, const double *__restrict__ dt_dev, double dx, double dy, int sources,
+    double dt, const double *__restrict__ dt_dev, double hx, double hy, int sources,
     int time_dg, DevPar Pv, Consts C, Batch B, int parts) {
   constexpr int NP = NN * (ND == 1 ? NN : NN * NN);
   if (dt_dev)
     dt = *dt_dev;
   long gt = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  cells_body<L, ND, BATCH>(u, qh, fbx, fby, nx, ny, mask, dt, dx, dy, sources, time_dg, Pv, C,
+  cells_body<L, ND, BATCH>(u, qh, fbx, fby, nx, ny, mask, dt, hx, hy, sources, time_dg, Pv, C,
                            B, parts, gt / NP, threadIdx.x % NP, true, 0);
 }
 
@@ -1575,7 +1579,7 @@ constexpr int FV1_TILE_SMALL = 7;
 template <class L, int TILE = FV1_TILE>
 __global__ void __launch_bounds__(128) k_fv1d(
     double *__restrict__ u, const double *__restrict__ qh, long nx,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double idx,
     int sources, int time_dg, DevPar P, Consts C, int parts) {
   constexpr int V = L::V;
   static_assert(NN == 2 && 4 * (TILE + 1) <= 128 && (TILE + 1) % 8 == 0,
@@ -1586,11 +1590,11 @@ __global__ void __launch_bounds__(128) k_fv1d(
   const long c0 = (long)blockIdx.x * TILE;  // first cell, and first face, of the tile
   const int slot = threadIdx.x >> 2, lq = threadIdx.x & 3;
   if (parts & FV_INTERFS)
-    faces1d_split_body<L, false>(sfb, qh, nx + 1, mask, dt, dx, time_dg, P, C, Batch{},
+    faces1d_split_body<L, false>(sfb, qh, nx + 1, mask, dt, idx, time_dg, P, C, Batch{},
                                  c0 + slot, lq, true, c0);
   __syncthreads();
-  cells_body<L, 1, false>(u, qh, sfb, nullptr, nx, 1, mask, dt, dx, 1.0, sources, time_dg, P, C,
-                          Batch{}, parts, c0 + slot, lq, slot < TILE, c0);
+  cells_body<L, 1, false>(u, qh, sfb, nullptr, nx, 1, mask, dt, idx * C.derv[0][1], 0.0,
+                          sources, time_dg, P, C, Batch{}, parts, c0 + slot, lq, slot < TILE, c0);
 }
 
 // ---------------------------------------------------------------------------
@@ -1599,7 +1603,7 @@ __global__ void __launch_bounds__(128) k_fv1d(
 // unsigned integers); NaN cells are skipped as std::max skips them.
 template <class L>
 __global__ void __launch_bounds__(256) k_cfl_max(const double *__restrict__ u, long ncell,
-                                                 int nd, double dx, double dy,
+                                                 int nd, double idx, double idy,
                                                  unsigned long long *__restrict__ out,
                                                  DevPar P) {
   constexpr int V = L::V;
@@ -1612,9 +1616,9 @@ __global__ void __launch_bounds__(256) k_cfl_max(const double *__restrict__ u, l
       q[k] = u[c * V + k];
     Prim<L::THERMAL> s;
     prim<L::THERMAL>(q, P, s);
-    double tmp = max_abs_eigs<L::THERMAL>(q, s, 0, P) / dx;
+    double tmp = max_abs_eigs<L::THERMAL>(q, s, 0, P) * idx;
     if (nd == 2)
-      tmp += max_abs_eigs<L::THERMAL>(q, s, 1, P) / dy;
+      tmp = fma(max_abs_eigs<L::THERMAL>(q, s, 1, P), idy, tmp);
     if (tmp > m)
       m = tmp;
   }

@@ -287,15 +287,17 @@ template <class L> struct Ops {
     const Consts &C = consts();
     int nx = nX[0];
     const bool faces = parts & FV_INTERFS;
+    const double idx = 1.0 / dX[0], idy = nd == 2 ? 1.0 / dX[1] : 0.0;
+    const double hx = idx * C.derv[0][1], hy = idy * C.derv[0][1];
     if (nd == 1) {
       if (flux == GPR_FLUX_RUSANOV || !faces) {
         // faces, volume term and update in one launch (k_fv1d)
         if (blocks(nx, FV1_TILE) < 2 * sm_count())
           k_fv1d<L, FV1_TILE_SMALL><<<blocks(nx, FV1_TILE_SMALL), 4 * (FV1_TILE_SMALL + 1), 0,
-                                      st>>>(u, qh, nx, mask, dt, dt_dev, dX[0], sources,
+                                      st>>>(u, qh, nx, mask, dt, dt_dev, idx, sources,
                                             time_dg, P, C, parts);
         else
-          k_fv1d<L><<<blocks(nx, FV1_TILE), 128, 0, st>>>(u, qh, nx, mask, dt, dt_dev, dX[0],
+          k_fv1d<L><<<blocks(nx, FV1_TILE), 128, 0, st>>>(u, qh, nx, mask, dt, dt_dev, idx,
                                                           sources, time_dg, P, C, parts);
         return cuda_rc();
       }
@@ -307,7 +309,7 @@ template <class L> struct Ops {
           scratch, qh, (long)nx + 1, mask, dt, dt_dev, dX[0], time_dg, flux, P, C, Batch{});
       long nc = (long)nx * NN * NN;
       k_cells<L, 1><<<GPR_SPREAD(nc, 128), 0, st>>>(u, qh, scratch, nullptr, nx, 1, mask, dt,
-                                                     dt_dev, dX[0], 1.0, sources, time_dg, P,
+                                                     dt_dev, hx, hy, sources, time_dg, P,
                                                      C, Batch{}, parts);
       return cuda_rc();
     }
@@ -321,14 +323,13 @@ template <class L> struct Ops {
       // buffer.
       if (parts & FV_CENTERS)
         k_cells<L, 2><<<blocks(nc, 128), 128, 0, st>>>(u, qh, nullptr, nullptr, nx, ny, mask,
-                                                        dt, dt_dev, dX[0], dX[1], sources,
+                                                        dt, dt_dev, hx, hy, sources,
                                                         time_dg, P, C, Batch{}, FV_CENTERS);
       if (faces)
         for (int dir = 0; dir < 2; dir++)
           for (int par = 0; par < 2; par++) {
-            long nf = face2_count(nx, ny, dir, par);
-            k_faces2d<L><<<blocks(nf * NN * NN, 128), 128, 0, st>>>(
-                u, qh, nx, ny, dir, mask, dt, dt_dev, dX[0], dX[1], time_dg, P, C, par);
+            launch_faces2d(u, qh, nx, ny, dir, par, mask, dt, dt_dev, dir ? idy : idx, time_dg,
+                           P, C, st);
           }
       return cuda_rc();
     }
@@ -340,8 +341,8 @@ template <class L> struct Ops {
     faces2d_eig(fbx, pp, qh, nx, ny, 0, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
     faces2d_eig(fby, pp, qh, nx, ny, 1, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
     k_cells<L, 2><<<blocks(nc, 128), 128, 0, st>>>(u, qh, fbx, fby, nx, ny, mask, dt, dt_dev,
-                                                    dX[0], dX[1], sources, time_dg, P, C,
-                                                    Batch{}, parts);
+                                                    hx, hy, sources, time_dg, P, C, Batch{},
+                                                    parts);
     return cuda_rc();
   }
 
@@ -356,7 +357,7 @@ template <class L> struct Ops {
       long nf = (long)(nx + 1) * NN;
       if (flux == GPR_FLUX_RUSANOV)
         k_faces1d_split<L><<<GPR_SPREAD(nf * 2, 128), 0, st>>>(
-            fb, qh, (long)nx + 1, mask, dt, nullptr, dX[0], time_dg, P, C, Batch{});
+            fb, qh, (long)nx + 1, mask, dt, nullptr, 1.0 / dX[0], time_dg, P, C, Batch{});
       else
         k_faces1d_eigw<L><<<(unsigned)(nx + 1), 32 * EIG_WARPS, 0, st>>>(
             fb, qh, (long)nx + 1, mask, dt, nullptr, dX[0], time_dg, flux, P, C, Batch{});
@@ -371,13 +372,23 @@ template <class L> struct Ops {
                   C, st);
       return cuda_rc();
     }
-    k_faces2d<L><<<blocks(nf * NN * NN, 128), 128, 0, st>>>(fb, qh, nx, ny, 0, mask, dt,
-                                                             nullptr, dX[0], dX[1], time_dg,
-                                                             P, C);
-    k_faces2d<L><<<blocks(nf * NN * NN, 128), 128, 0, st>>>(fb + nf * 2 * V, qh, nx, ny, 1,
-                                                             mask, dt, nullptr, dX[0], dX[1],
-                                                             time_dg, P, C);
+    launch_faces2d(fb, qh, nx, ny, 0, -1, mask, dt, nullptr, 1.0 / dX[0], time_dg, P, C, st);
+    launch_faces2d(fb + nf * 2 * V, qh, nx, ny, 1, -1, mask, dt, nullptr, 1.0 / dX[1], time_dg,
+                   P, C, st);
     return cuda_rc();
+  }
+
+  // One k_faces2d pass: direction dir, parity par, ih = 1 / dx_dir.
+  static void launch_faces2d(double *fb, const double *qh, int nx, int ny, int dir, int par,
+                             const uint8_t *mask, double dt, const double *dt_dev, double ih,
+                             int time_dg, const DevPar &P, const Consts &C, cudaStream_t st) {
+    const int nb = blocks(face2_count(nx, ny, dir, par) * NN * NN, 128);
+    if (dir == 0)
+      k_faces2d<L, 0><<<nb, 128, 0, st>>>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg, P, C,
+                                          par);
+    else
+      k_faces2d<L, 1><<<nb, 128, 0, st>>>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg, P, C,
+                                          par);
   }
 
   // Osher / Roe faces of one direction on a 2D grid: one thread per face
@@ -398,8 +409,8 @@ template <class L> struct Ops {
                       double *scratch, cudaStream_t st) {
     unsigned long long *mx = (unsigned long long *)scratch;
     cudaMemsetAsync(mx, 0, sizeof(unsigned long long), st);
-    k_cfl_max<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, nd, dX[0],
-                                                      nd == 2 ? dX[1] : 1.0, mx, P);
+    k_cfl_max<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, nd, 1.0 / dX[0],
+                                                      nd == 2 ? 1.0 / dX[1] : 0.0, mx, P);
     k_cfl_finalize<<<1, 1, 0, st>>>(mx, cfl, t, tf, count, dt_out);
     return cuda_rc();
   }
@@ -474,8 +485,8 @@ template <class L> struct Ops {
   // first step.
   static void step_head(const double *u, long ncell, int nd, const double *dX, const DevPar &P,
                         unsigned long long *mx, double *clk, cudaStream_t st) {
-    k_cfl_max<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, nd, dX[0],
-                                                      nd == 2 ? dX[1] : 1.0, mx, P);
+    k_cfl_max<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, nd, 1.0 / dX[0],
+                                                      nd == 2 ? 1.0 / dX[1] : 0.0, mx, P);
     k_clock_finalize<<<1, 1, 0, st>>>(mx, clk, (int *)(mx + 1));
   }
   static void step_tail(double *u, long ncell, const DevPar &P, double tol,

@@ -164,8 +164,8 @@ template <class L, int NO> struct OpsN {
     const long ncell = g.ncell();
     for (int s = 0; s < nsteps; s++) {
       cudaMemsetAsync(mx, 0, sizeof(unsigned long long), st);
-      k_cfl_max<L><<<blocks(ncell, 256), 256, 0, st>>>(u, ncell, g.nd, dX[0],
-                                                        g.nd == 2 ? dX[1] : 1.0, mx, P);
+      k_cfl_max<L><<<blocks(ncell, 256), 256, 0, st>>>(u, ncell, g.nd, 1.0 / dX[0],
+                                                        g.nd == 2 ? 1.0 / dX[1] : 0.0, mx, P);
       k_clock_finalize<<<1, 1, 0, st>>>(mx, clk);
       int rc = boundaries(u, ub, g, bcs, st);
       if (!rc)

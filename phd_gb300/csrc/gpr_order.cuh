@@ -789,42 +789,21 @@ template <class L, int NO, bool EIG = false>
 GPR_D void interface_point_n(const double *ql, const double *qr, int d, const DevPar &P,
                              const ConstsN<NO> &C, double *f, double *b, int flux = 0) {
   constexpr int V = L::V;
+  if (!EIG) {
+    rusanov_point<L, NO>(ql, qr, d, P, C.nodes, C.w, f, b);
+    return;
+  }
   Prim<L::THERMAL> sl, sr;
   prim<L::THERMAL>(ql, P, sl);
   prim<L::THERMAL>(qr, P, sr);
-  double dq[V];
-  if (EIG) {
-    eig_dissipation_qd<L, NO>(ql, qr, d, flux, P, C.nodes, C.w, f);
-#pragma unroll
-    for (int k = 0; k < V; k++) {
-      dq[k] = qr[k] - ql[k];
-      b[k] = 0.0;
-    }
-  } else {
-    const double m1 = max_abs_eigs<L::THERMAL>(ql, sl, d, P);
-    const double m2 = max_abs_eigs<L::THERMAL>(qr, sr, d, P);
-    const double m = m1 > m2 ? m1 : m2;
-#pragma unroll
-    for (int k = 0; k < V; k++) {
-      f[k] = m * (ql[k] - qr[k]);
-      dq[k] = qr[k] - ql[k];
-      b[k] = 0.0;
-    }
-  }
+  eig_dissipation_qd<L, NO>(ql, qr, d, flux, P, C.nodes, C.w, f);
   flux_add<L::THERMAL, V>(ql, sl, d, P, f);
   flux_add<L::THERMAL, V>(qr, sr, d, P, f);
+  double dq[V];
 #pragma unroll
-  for (int n = 0; n < NO; n++) {
-    const double ir = 1.0 / (ql[0] + C.nodes[n] * dq[0]);
-    double v[3] = {(ql[2] + C.nodes[n] * dq[2]) * ir, (ql[3] + C.nodes[n] * dq[3]) * ir,
-                   (ql[4] + C.nodes[n] * dq[4]) * ir};
-    double bd[V];
-    bdot<V, L::LSET>(v, dq, d, bd);
-#pragma unroll
-    for (int k = 5; k < V; k++)
-      if (k < 14 || k >= V - L::LSET)
-        b[k] += C.w[n] * bd[k];
-  }
+  for (int k = 0; k < V; k++)
+    dq[k] = qr[k] - ql[k];
+  path_product<L, NO>(ql, dq, d, C.nodes, C.w, b);
 }
 
 // Face terms (interfs1 / interfs2, fv.cpp:111-279): one thread per (face,

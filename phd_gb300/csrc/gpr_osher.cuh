@@ -825,22 +825,9 @@ GPR_D void interface_point_eig(const double *ql, const double *qr, int flux, con
   flux_add<L::THERMAL, V>(qr, sr, d, P, f);
   double dq[V];
 #pragma unroll
-  for (int k = 0; k < V; k++) {
+  for (int k = 0; k < V; k++)
     dq[k] = qr[k] - ql[k];
-    b[k] = 0.0;
-  }
-#pragma unroll
-  for (int n = 0; n < NN; n++) {
-    const double rho = ql[0] + C.nodes[n] * dq[0];
-    const double ir = 1.0 / rho;
-    const double v[3] = {(ql[2] + C.nodes[n] * dq[2]) * ir, (ql[3] + C.nodes[n] * dq[3]) * ir,
-                         (ql[4] + C.nodes[n] * dq[4]) * ir};
-    double bd[V];
-    bdot<V, L::LSET>(v, dq, d, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      b[k] += C.w[n] * bd[k];
-  }
+  path_product<L, NN>(ql, dq, d, C.nodes, C.w, b);
 }
 
 // ---------------------------------------------------------------------------
