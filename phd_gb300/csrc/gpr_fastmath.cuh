@@ -54,6 +54,15 @@ GPR_D double sqrt64(double x) {
   return g;
 }
 
+// 1 / sqrt(x) for normal x well inside the range: one third-order step
+// (Householder) from the special-function start, truncation below 2^-58.
+GPR_D double rsqrt64(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
 // x^(5/3) (sign of x), the distortion's det(A)^(5/3).  With y ~ |x|^(-1/3)
 // from FP32 (of the mantissa times 2^(exponent mod 3): relative error below
 // 2^-20), u = |x| y^2 and e = 1 - u y, |x|^(-1/3) = y (1 - e)^(-1/3) = y (1 +

@@ -1353,11 +1353,13 @@ __global__ void __launch_bounds__(128) k_faces1d_split(
 // every face, contributions written to fb[face][2][V] (the face-flux
 // entry points); parity 0 / 1: the faces of that parity along DIR, applied
 // to u (passed as fb) in place, the conservative update of interfs2.
-template <class L, int DIR>
-__global__ void __launch_bounds__(128) k_faces2d(
-    double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double ih,
-    int time_dg, DevPar P, Consts C, int parity = -1) {
+// point(ql, qr) evaluates f and b at one quadrature point.
+template <class L, int DIR, class Point>
+GPR_D void faces2d_body(double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny,
+                        const uint8_t *__restrict__ mask, double dt,
+                        const double *__restrict__ dt_dev, double ih, int time_dg,
+                        const Consts &C, int parity, double (&f)[L::V], double (&b)[L::V],
+                        Point point) {
   constexpr int V = L::V;
   constexpr int NQ = NN * NN;
   if (dt_dev)
@@ -1378,7 +1380,7 @@ __global__ void __launch_bounds__(128) k_faces2d(
   int tt = time_dg ? t : 0;
   const double *q0 = qh + (cb * nt + tt) * NN * NN * V;
   const double *q1 = qh + (cn * nt + tt) * NN * NN * V;
-  double ql[V], qr[V], f[V], b[V];
+  double ql[V], qr[V];
   // endpts2d (evaluations.cpp:20-35): DIR 0 -> nodes (m, s); DIR 1 -> (s, m)
   long o0 = DIR == 0 ? (long)s * V : (long)s * NN * V;
   long st = DIR == 0 ? (long)NN * V : (long)V;
@@ -1390,7 +1392,7 @@ __global__ void __launch_bounds__(128) k_faces2d(
   // W_t W_s dt / (2 h)
   const double kk = dt * ih * (time_dg ? 0.5 * GAUSS_W * GAUSS_W : 0.5 * GAUSS_W);
   if (active) {
-    interface_point<L>(ql, qr, DIR, P, C, f, b);
+    point(ql, qr);
   } else {
 #pragma unroll
     for (int k = 0; k < V; k++)
@@ -1403,6 +1405,18 @@ __global__ void __launch_bounds__(128) k_faces2d(
     face2_cells(fb, i, j, nx, ny, DIR, V, uL, uR);
     face_reduce_apply<V, NQ>(b, f, kk, active, face_on, lq, uL, uR);
   }
+}
+
+template <class L, int DIR>
+__global__ void __launch_bounds__(128) k_faces2d(
+    double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double ih,
+    int time_dg, DevPar P, Consts C, int parity = -1) {
+  double f[L::V], b[L::V];
+  faces2d_body<L, DIR>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg, C, parity, f, b,
+                       [&](const double *ql, const double *qr) {
+                         interface_point<L>(ql, qr, DIR, P, C, f, b);
+                       });
 }
 
 // Parts of the FV update k_cells applies: the volume term (centers1 /

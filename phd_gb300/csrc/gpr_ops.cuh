@@ -301,12 +301,8 @@ template <class L> struct Ops {
                                                           sources, time_dg, P, C, parts);
         return cuda_rc();
       }
-      // Osher / Roe: the faces' eigen-decompositions, one warp each, write
-      // the face sums to scratch (a 1D grid has few faces, so one launch over
-      // all of them keeps the decompositions' latency to one), then the cell
-      // pass applies them
-      k_faces1d_eigw<L><<<(unsigned)(nx + 1), 32 * EIG_WARPS, 0, st>>>(
-          scratch, qh, (long)nx + 1, mask, dt, dt_dev, dX[0], time_dg, flux, P, C, Batch{});
+      // Osher / Roe: the face sums to scratch, then the cell pass
+      faces1d_eig(scratch, qh, nx, mask, dt, dt_dev, dX[0], time_dg, flux, P, C, st);
       long nc = (long)nx * NN * NN;
       k_cells<L, 1><<<GPR_SPREAD(nc, 128), 0, st>>>(u, qh, scratch, nullptr, nx, 1, mask, dt,
                                                      dt_dev, hx, hy, sources, time_dg, P,
@@ -315,8 +311,8 @@ template <class L> struct Ops {
     }
     int ny = nX[1];
     const long nc = (long)nx * ny * NN * NN * NN;
-    if (flux == GPR_FLUX_RUSANOV || !faces) {
-      // Rusanov: the volume term first (centers2), then the face terms
+    if (flux == GPR_FLUX_RUSANOV || osher_closed(flux, P) || !faces) {
+      // Rusanov, Osher: the volume term first (centers2), then the face terms
       // applied to u in place by four passes (x / y faces, even / odd index
       // along the direction; two faces of one pass never share a cell), as
       // interfs2 updates u inside its face loop (fv.cpp:162-279).  No face
@@ -329,12 +325,12 @@ template <class L> struct Ops {
         for (int dir = 0; dir < 2; dir++)
           for (int par = 0; par < 2; par++) {
             launch_faces2d(u, qh, nx, ny, dir, par, mask, dt, dt_dev, dir ? idy : idx, time_dg,
-                           P, C, st);
+                           flux, P, C, st);
           }
       return cuda_rc();
     }
-    // Osher / Roe: the per-thread eigen-decompositions write the face sums
-    // of each direction to scratch, then the cell pass applies the volume
+    // Roe: the per-thread eigen-decompositions write the face sums of each
+    // direction to scratch, then the cell pass applies the volume
     // and face terms
     long nf = (long)(nx + 1) * (ny + 1);
     double *fbx = scratch, *fby = scratch + nf * 2 * V, *pp = scratch + 2 * nf * 2 * V;
@@ -359,31 +355,58 @@ template <class L> struct Ops {
         k_faces1d_split<L><<<GPR_SPREAD(nf * 2, 128), 0, st>>>(
             fb, qh, (long)nx + 1, mask, dt, nullptr, 1.0 / dX[0], time_dg, P, C, Batch{});
       else
-        k_faces1d_eigw<L><<<(unsigned)(nx + 1), 32 * EIG_WARPS, 0, st>>>(
-            fb, qh, (long)nx + 1, mask, dt, nullptr, dX[0], time_dg, flux, P, C, Batch{});
+        faces1d_eig(fb, qh, nx, mask, dt, nullptr, dX[0], time_dg, flux, P, C, st);
       return cuda_rc();
     }
     int ny = nX[1];
     long nf = (long)(nx + 1) * (ny + 1);
-    if (flux != GPR_FLUX_RUSANOV) {
+    if (flux != GPR_FLUX_RUSANOV && !osher_closed(flux, P)) {
       double *pp = fb + 2 * nf * 2 * V;
       faces2d_eig(fb, pp, qh, nx, ny, 0, mask, dt, nullptr, dX, time_dg, flux, P, C, st);
       faces2d_eig(fb + nf * 2 * V, pp, qh, nx, ny, 1, mask, dt, nullptr, dX, time_dg, flux, P,
                   C, st);
       return cuda_rc();
     }
-    launch_faces2d(fb, qh, nx, ny, 0, -1, mask, dt, nullptr, 1.0 / dX[0], time_dg, P, C, st);
+    launch_faces2d(fb, qh, nx, ny, 0, -1, mask, dt, nullptr, 1.0 / dX[0], time_dg, flux, P, C,
+                   st);
     launch_faces2d(fb + nf * 2 * V, qh, nx, ny, 1, -1, mask, dt, nullptr, 1.0 / dX[1], time_dg,
-                   P, C, st);
+                   flux, P, C, st);
     return cuda_rc();
   }
 
-  // One k_faces2d pass: direction dir, parity par, ih = 1 / dx_dir.
+  // The Osher dissipation has its closed form (abs_apply_acoustic) for the
+  // material; with heat conduction and beta != 0 no point would take it.
+  static bool osher_closed(int flux, const DevPar &P) {
+    return flux == GPR_FLUX_OSHER && !(L::THERMAL && P.has_beta);
+  }
+
+  // Osher / Roe faces of a 1D grid into fb.
+  static void faces1d_eig(double *fb, const double *qh, int nx, const uint8_t *mask, double dt,
+                          const double *dt_dev, double dx, int time_dg, int flux,
+                          const DevPar &P, const Consts &C, cudaStream_t st) {
+    const int closed = osher_closed(flux, P);
+    if (closed)
+      k_faces1d_osher<L><<<GPR_SPREAD(4L * (nx + 1), 128), 0, st>>>(
+          fb, qh, (long)nx + 1, mask, dt, dt_dev, 1.0 / dx, time_dg, P, C);
+    k_faces1d_eigw<L><<<(unsigned)(nx + 1), 32 * EIG_WARPS, 0, st>>>(
+        fb, qh, (long)nx + 1, mask, dt, dt_dev, dx, time_dg, flux, P, C, Batch{}, closed);
+  }
+
+  // One face pass of k_faces2d or k_faces2d_osher: direction dir, parity par,
+  // ih = 1 / dx_dir.
   static void launch_faces2d(double *fb, const double *qh, int nx, int ny, int dir, int par,
                              const uint8_t *mask, double dt, const double *dt_dev, double ih,
-                             int time_dg, const DevPar &P, const Consts &C, cudaStream_t st) {
+                             int time_dg, int flux, const DevPar &P, const Consts &C,
+                             cudaStream_t st) {
     const int nb = blocks(face2_count(nx, ny, dir, par) * NN * NN, 128);
-    if (dir == 0)
+    if (flux == GPR_FLUX_OSHER) {
+      if (dir == 0)
+        k_faces2d_osher<L, 0><<<nb, 128, 0, st>>>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg,
+                                                  P, C, par);
+      else
+        k_faces2d_osher<L, 1><<<nb, 128, 0, st>>>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg,
+                                                  P, C, par);
+    } else if (dir == 0)
       k_faces2d<L, 0><<<nb, 128, 0, st>>>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg, P, C,
                                           par);
     else

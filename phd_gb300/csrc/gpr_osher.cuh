@@ -703,6 +703,333 @@ template <int n> GPR_D bool abs_apply(double *M, const double *dq, double w, dou
   return true;
 }
 
+// ---------------------------------------------------------------------------
+// |M| of one state in closed form (Osher-Solomon).  In primitive variables (rho,
+// p, v, A, J) the system matrix along x is v + N, where N couples only y =
+// (v, J_x) with z = (rho, p, A): y' = Xi1 z, z' = Xi2 y (the energy equation's
+// heat terms cancel but for h dJ_x).  So N^2 on y is the acoustic tensor Xi =
+// Xi1 Xi2, the eigenvalues of M are v (nine-fold) and v +- c_k with c_k^2
+// those of Xi, and for any eigenvectors
+//   |M| (y, z) = (E(Xi) y + O(Xi) Xi1 z,  |v| z + Xi2 (K(Xi) Xi1 z + O(Xi) y)),
+// E = max(c, |v|), O = sgn(v) min(c, |v|) / c, K = max(c - |v|, 0) / c^2.
+// Along x the velocity block of Xi is symmetric and the heat row and column
+// meet it at v_x only, so a diagonal scaling makes Xi symmetric and E, O, K
+// follow from its 3 x 3 or 4 x 4 symmetric eigenproblem (Jacobi): about 1300
+// FP64 instructions per path node in registers, where the 17 x 17
+// eigen-decomposition with its vectors and complex solve takes about 1e5 in
+// local memory.  An orthogonal decomposition has no loss at equal wave speeds.
+
+// H = W diag(H) W^T by cyclic Jacobi rotations, H symmetric positive definite
+// (its upper triangle is used, and holds the eigenvalues on the diagonal at
+// the end).  A rotation's tangent only has to bring the entry down by a few
+// digits, so it is taken in FP32 from the exact FP64 difference of the
+// diagonal; cosine and sine are then formed in FP64, so each rotation is
+// orthogonal to rounding, and the rotated entry keeps what is left of it.
+// Entries below 6e-16 of the geometric mean of their diagonal, or below 2e-17 of
+// the trace (a rounding of the largest entries), are skipped; the
+// sweeps end when a whole sweep skipped (4 x 4 acoustic tensors: 3 - 5).
+template <int m> GPR_D bool jacobi_sym(double (&H)[m][m], double (&W)[m][m]) {
+#pragma unroll
+  for (int i = 0; i < m; i++)
+#pragma unroll
+    for (int j = 0; j < m; j++)
+      W[i][j] = i == j ? 1.0 : 0.0;
+  double tr = H[0][0];
+#pragma unroll
+  for (int i = 1; i < m; i++)
+    tr += H[i][i];
+  const int sh = fp_exponent(tr) - 1023;
+  if (__double2hiint(tr) < 0 || sh < -500 || sh > 500)
+    return false;
+#pragma unroll 1
+  for (int sweep = 0; sweep < 12; sweep++) {
+    bool rotated = false;
+#pragma unroll
+    for (int p = 0; p < m - 1; p++)
+#pragma unroll
+      for (int q = p + 1; q < m; q++) {
+        const float e = f32_scaled(H[p][q], sh);
+        const float a = f32_scaled(H[p][p], sh), b = f32_scaled(H[q][q], sh);
+        if (fabsf(e) <= 2e-17f || e * e <= 4e-31f * (a * b))
+          continue;
+        rotated = true;
+        const float th = 0.5f * f32_scaled(H[q][q] - H[p][p], sh) * rcp32(e);
+        const float tf = copysignf(rcp32(fabsf(th) + sqrt32(fmaf(th, th, 1.0f))), th);
+        const double t = f64_scaled(tf, 0);
+        const double c = rsqrt64(fma(t, t, 1.0)), s = c * t;
+        const double u1 = fma(c, H[p][p], -(s * H[p][q])), u2 = fma(c, H[p][q], -(s * H[q][q]));
+        const double u3 = fma(s, H[p][p], c * H[p][q]), u4 = fma(s, H[p][q], c * H[q][q]);
+        H[p][p] = fma(c, u1, -(s * u2));
+        H[p][q] = fma(s, u1, c * u2);
+        H[q][q] = fma(s, u3, c * u4);
+#pragma unroll
+        for (int r = 0; r < m; r++) {
+          if (r != p && r != q) {
+            double &x = r < p ? H[r][p] : H[p][r], &y = r < q ? H[r][q] : H[q][r];
+            const double xp = fma(c, x, -(s * y));
+            y = fma(s, x, c * y);
+            x = xp;
+          }
+          const double wp = fma(c, W[r][p], -(s * W[r][q]));
+          W[r][q] = fma(s, W[r][p], c * W[r][q]);
+          W[r][p] = wp;
+        }
+      }
+    if (!rotated)
+      return true;
+  }
+  return false;
+}
+
+// f += w |M(q)| dq along x.  Returns false, with f unchanged, where the form
+// does not apply (wave speeds that are not real and positive, a heat coupling
+// that no scaling makes symmetric): the caller then takes the general
+// eigen-decomposition.
+template <class L>
+GPR_D bool abs_apply_acoustic(const double *q, const double *dq, double w, const DevPar &P,
+                              double *f) {
+  constexpr int V = L::V;
+  constexpr bool TH = L::THERMAL;
+  constexpr int m = TH ? 4 : 3;
+  Prim<TH> s;
+  prim<TH>(q, P, s);
+  const double *A = q + 5;
+  const double *dA = dq + 5;
+  const EosRho &e = s.e;
+  const double r = s.r, ir = s.ir, cs2 = s.cs2;
+  const double rG = r * e.G, irG2 = s.irG * s.irG;
+  double dnum = e.G * (s.p - e.pr);
+  if (P.EOS != 0)
+    dnum = e.dpr * rG + (e.G + r * e.dG) * (s.p - e.pr);
+  double Er = e.der - dnum * irG2;
+  double C0 = cs2;
+  if (P.has_beta) {
+    if (TH)
+      return false;  // the impulse then couples to all of v
+    const double dcs2 = P.beta * ir * cs2;
+    Er += 0.25 * ((1.0 - P.beta / e.G) * dcs2 + P.beta / (e.G * e.G) * e.dG * cs2) * s.devGsq;
+    C0 = (P.EOS == 1 ? (1.0 - P.beta / e.G) : P.C0f) * cs2;
+  }
+  const double c02 = (s.p * ir * ir - Er) * rG;
+  const double eR = fma(q[1], ir, r * Er);  // d(rho E)/drho at fixed p, v, A, J
+  const double rC0 = r * C0;
+  // dq in primitive variables (dP/dQ, equations.cpp:130-167)
+  const double rho = dq[0];
+  double vp[3], Jp[3] = {0.0, 0.0, 0.0}, AGdA = 0.0;
+  double pp = fma(-eR, rho, dq[1]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    vp[i] = fma(-s.v[i], rho, dq[2 + i]);
+    pp = fma(-s.v[i], vp[i], pp);
+    vp[i] *= ir;
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++)
+    AGdA = fma(s.AdG[k], dA[k], AGdA);
+  pp = fma(-rC0, AGdA, pp);
+  if (TH) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      Jp[i] = fma(-s.J[i], rho, dq[14 + i]);
+      pp = fma(-P.calpha2 * s.J[i], Jp[i], pp);
+      Jp[i] *= ir;
+    }
+  }
+  pp *= e.G;
+  // Xi1 z: (dp e_x - dsigma_x) / rho and dT / rho, with dsigma_x = (1 + beta)
+  // sigma_x drho / rho - rho cs2 (dG devG + devG dG ... )(:,x), dG = dA^T A + A^T dA
+  double y[m], a[m];
+  {
+    double dG[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      const int i = k < 3 ? k : (k == 5 ? 1 : 0), j = k < 3 ? k : (k == 3 ? 1 : 2);
+      double x = 0.0;
+#pragma unroll
+      for (int n = 0; n < 3; n++)
+        x = fma(dA[3 * n + i], A[3 * n + j], fma(A[3 * n + i], dA[3 * n + j], x));
+      dG[k] = x;
+    }
+    const double t3 = (s.G[0] + s.G[1] + s.G[2]) * (1.0 / 3.0);
+    const double dt3 = (dG[0] + dG[1] + dG[2]) * (1.0 / 3.0);
+    const double fr = P.b1 * rho * ir;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      // S(i, x) = (G^2 - t3 G)(i, x): dS = dG G + G dG - dt3 G - t3 dG
+      double x = fma(-dt3, sym3(s.G, i, 0), -(t3 * sym3(dG, i, 0)));
+#pragma unroll
+      for (int n = 0; n < 3; n++)
+        x = fma(sym3(dG, i, n), sym3(s.G, n, 0), fma(sym3(s.G, i, n), sym3(dG, n, 0), x));
+      a[i] = cs2 * fma(fr, sym3(s.S, i, 0), x);
+      y[i] = vp[i];
+    }
+    a[0] = fma(ir, pp, a[0]);
+  }
+  // the acoustic tensor (max_abs_eigs, d = 0), symmetric after scaling the
+  // impulse by del = sqrt(x30 / x03)
+  double H[m][m], W[m][m];
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double g3 = (1.0 / 3.0) * sym3(s.G, i, 0);
+#pragma unroll
+    for (int c = i; c < 3; c++) {
+      double x = fma(s.G[0], sym3(s.G, i, c), fma(g3, sym3(s.G, c, 0), sym3(s.S, i, c)));
+      if (i == 0)
+        x = fma(c == 0 ? 2.0 * P.b1 : P.b1, sym3(s.S, 0, c), x);
+      H[i][c] = cs2 * x;
+    }
+  }
+  H[0][0] += c02;
+  double h = 0.0, del = 1.0, idel = 1.0;
+  if (TH) {
+    h = P.calpha2 * s.T * e.G;
+    const double rtp = s.irG * P.icv;
+    const double dTr = -dnum * irG2 * P.icv;
+    const double x03 = h * ir, x30 = fma(rtp, c02, dTr);
+    const double pr = x03 * x30;
+    if (!(pr > 0.0))
+      return false;
+    H[0][m - 1] = copysign(sqrt64(pr), x03);
+    H[1][m - 1] = H[2][m - 1] = 0.0;
+    H[m - 1][m - 1] = rtp * ir * h;
+    del = fabs(H[0][m - 1] * rcp64(x03));
+    idel = rcp64(del);
+    y[m - 1] = Jp[0] * idel;
+    a[m - 1] = ir * fma(rtp, pp, dTr * rho) * idel;
+  }
+  if (!jacobi_sym<m>(H, W))
+    return false;
+  bool pos = true;
+#pragma unroll
+  for (int k = 0; k < m; k++)
+    pos = pos && H[k][k] > 0.0;
+  if (!pos)
+    return false;
+  const double av = fabs(s.v[0]);
+  double yo[m], wo[m];
+#pragma unroll
+  for (int i = 0; i < m; i++)
+    yo[i] = wo[i] = 0.0;
+#pragma unroll
+  for (int k = 0; k < m; k++) {
+    const double c = sqrt64(H[k][k]), ic = rcp64(c);
+    const bool sub = c > av;
+    const double E = sub ? c : av;
+    const double O = sub ? s.v[0] * ic : copysign(1.0, s.v[0]);
+    const double K = sub ? (c - av) * ic * ic : 0.0;
+    double yk = 0.0, ak = 0.0;
+#pragma unroll
+    for (int i = 0; i < m; i++) {
+      yk = fma(W[i][k], y[i], yk);
+      ak = fma(W[i][k], a[i], ak);
+    }
+    const double ey = fma(E, yk, O * ak), ew = fma(K, ak, O * yk);
+#pragma unroll
+    for (int i = 0; i < m; i++) {
+      yo[i] = fma(W[i][k], ey, yo[i]);
+      wo[i] = fma(W[i][k], ew, wo[i]);
+    }
+  }
+  // z: |v| z + Xi2 w, b = -beta sigma_x + rho c0^2 e_x
+  const double rho_o = fma(r, wo[0], av * rho);
+  double pw = r * c02 * wo[0];
+  if (P.has_beta) {
+    const double fb = P.beta * r * cs2;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      pw = fma(fb * sym3(s.S, i, 0), wo[i], pw);
+  }
+  if (TH)
+    pw = fma(h * del, wo[m - 1], pw);
+  const double p_o = fma(av, pp, pw);
+  // back to conserved variables (dQ/dP)
+  double en = fma(eR, rho_o, p_o * r * s.irG), AG = 0.0;
+  f[0] = fma(w, rho_o, f[0]);
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double mi = fma(s.v[i], rho_o, r * yo[i]);
+    en = fma(r * s.v[i], yo[i], en);
+    f[2 + i] = fma(w, mi, f[2 + i]);
+  }
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    double x = av * dA[k];
+    if (k % 3 == 0) {
+#pragma unroll
+      for (int j = 0; j < 3; j++)
+        x = fma(A[k + j], wo[j], x);
+    }
+    AG = fma(s.AdG[k], x, AG);
+    f[5 + k] = fma(w, x, f[5 + k]);
+  }
+  en = fma(rC0, AG, en);
+  if (TH) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const double Jo = i == 0 ? del * yo[m - 1] : av * Jp[i];
+      en = fma(P.calpha2 * r * s.J[i], Jo, en);
+      f[14 + i] = fma(w, fma(s.J[i], rho_o, r * Jo), f[14 + i]);
+    }
+  }
+  f[1] = fma(w, en, f[1]);
+#pragma unroll
+  for (int k = V - L::LSET; k < V; k++)
+    f[k] = fma(w * av, dq[k], f[k]);
+  return true;
+}
+
+// f += w |M(q)| dq by the general eigen-decomposition (out of line: the
+// callers' registers and code are those of the closed form).
+template <class L>
+__device__ __noinline__ bool abs_apply_general(const double *q, const double *dq, double w,
+                                               const DevPar &P, double *f) {
+  constexpr int V = L::V;
+  double M[V * V];
+  Prim<L::THERMAL> s;
+  prim<L::THERMAL>(q, P, s);
+  system_matrix<L::THERMAL, V>(q, s, P, M);
+  return abs_apply<V>(M, dq, w, f);
+}
+
+// Eigen part of D_OSH along x into f (overwritten): sum_i w_i |M(q_i)| dq
+// over the NQ Gauss nodes of the path qR -> qL; NaN if a general
+// eigen-decomposition is needed and fails.
+template <class L, int NQ>
+GPR_D void osher_dissipation(const double *ql, const double *qr, const DevPar &P,
+                             const double *nodes, const double *wts, double *f) {
+  constexpr int V = L::V;
+  double dq[V], q[V];
+  bool flat = true;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    dq[k] = ql[k] - qr[k];
+    f[k] = 0.0;
+    flat = flat && (__double_as_longlong(dq[k]) << 1) == 0;
+  }
+  // qL = qR (a uniform region): |M| dq is exactly zero
+  if (flat)
+    return;
+#pragma unroll 1
+  for (int i = 0; i < NQ; i++) {
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      q[k] = fma(nodes[i], dq[k], qr[k]);
+    if (!abs_apply_acoustic<L>(q, dq, wts[i], P, f)) {
+      double qm[V], dm[V], fm[V];
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        qm[k] = q[k];
+        dm[k] = dq[k];
+        fm[k] = f[k];
+      }
+      const bool ok = abs_apply_general<L>(qm, dm, wts[i], P, fm);
+#pragma unroll
+      for (int k = 0; k < V; k++)
+        f[k] = ok ? fm[k] : __longlong_as_double(0x7ff8000000000000ll);
+    }
+  }
+}
+
 // Eigen part of D_OSH (flux 2) / D_ROE (flux 1) at one interface into f
 // (overwritten); NaN if the eigen-decomposition fails (fluxes.cpp:22-64).
 // The path qR -> qL takes the scheme's NQ Gauss nodes (nodes, wts on [0, 1]).
@@ -710,7 +1037,11 @@ template <class L, int NQ>
 GPR_D void eig_dissipation_q(const double *ql, const double *qr, int flux, const DevPar &P,
                              const double *nodes, const double *wts, double *f) {
   constexpr int V = L::V;
-  double dq[V], q[V], M[V * V];
+  if (flux == GPR_FLUX_OSHER) {
+    osher_dissipation<L, NQ>(ql, qr, P, nodes, wts, f);
+    return;
+  }
+  double dq[V], q[V], M[V * V], Mi[V * V];
   bool flat = true;
 #pragma unroll
   for (int k = 0; k < V; k++) {
@@ -722,38 +1053,22 @@ GPR_D void eig_dissipation_q(const double *ql, const double *qr, int flux, const
   // eigen-decomposition
   if (flat)
     return;
-  bool ok = true;
-  if (flux == GPR_FLUX_OSHER) {
 #pragma unroll 1
-    for (int i = 0; i < NQ; i++) {
+  for (int i = 0; i < V * V; i++)
+    M[i] = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < NQ; i++) {
 #pragma unroll
-      for (int k = 0; k < V; k++)
-        q[k] = qr[k] + nodes[i] * dq[k];
-      Prim<L::THERMAL> s;
-      prim<L::THERMAL>(q, P, s);
-      system_matrix<L::THERMAL, V>(q, s, P, M);
-      ok = ok && abs_apply<V>(M, dq, wts[i], f);
-    }
-  } else {
-    double Mi[V * V];
+    for (int k = 0; k < V; k++)
+      q[k] = qr[k] + nodes[i] * dq[k];
+    Prim<L::THERMAL> s;
+    prim<L::THERMAL>(q, P, s);
+    system_matrix<L::THERMAL, V>(q, s, P, Mi);
 #pragma unroll 1
-    for (int i = 0; i < V * V; i++)
-      M[i] = 0.0;
-#pragma unroll 1
-    for (int i = 0; i < NQ; i++) {
-#pragma unroll
-      for (int k = 0; k < V; k++)
-        q[k] = qr[k] + nodes[i] * dq[k];
-      Prim<L::THERMAL> s;
-      prim<L::THERMAL>(q, P, s);
-      system_matrix<L::THERMAL, V>(q, s, P, Mi);
-#pragma unroll 1
-      for (int k = 0; k < V * V; k++)
-        M[k] += wts[i] * Mi[k];
-    }
-    ok = abs_apply<V>(M, dq, 1.0, f);
+    for (int k = 0; k < V * V; k++)
+      M[k] += wts[i] * Mi[k];
   }
-  if (!ok) {
+  if (!abs_apply<V>(M, dq, 1.0, f)) {
 #pragma unroll
     for (int k = 0; k < V; k++)
       f[k] = __longlong_as_double(0x7ff8000000000000ll);
@@ -766,21 +1081,21 @@ GPR_D void eig_dissipation(const double *ql, const double *qr, int flux, const D
   eig_dissipation_q<L, NN>(ql, qr, flux, P, C.nodes, C.w, f);
 }
 
+GPR_HD constexpr int axis_swap_index(int a, int d) { return a == 0 ? d : (a == d ? 0 : a); }
 // Index of state entry k with spatial axes 0 and d exchanged: velocity and
 // thermal impulse components, and both indices of A (as the reference's
 // rotate_tensors, system/multi/rotations.cpp:37-47).  The GPR system is
 // invariant under this relabelling, so the system matrix along d is that
 // along x of the relabelled state, relabelled back: exact, a permutation.
-template <class L> GPR_D int axis_swap(int k, int d) {
+template <class L> GPR_HD constexpr int axis_swap(int k, int d) {
   if (d == 0)
     return k;
-  auto sw = [d](int a) { return a == 0 ? d : (a == d ? 0 : a); };
   if (k >= 2 && k < 5)
-    return 2 + sw(k - 2);
+    return 2 + axis_swap_index(k - 2, d);
   if (k >= 5 && k < 14)
-    return 5 + 3 * sw((k - 5) / 3) + sw((k - 5) % 3);
+    return 5 + 3 * axis_swap_index((k - 5) / 3, d) + axis_swap_index((k - 5) % 3, d);
   if (L::THERMAL && k >= 14 && k < 17)
-    return 14 + sw(k - 14);
+    return 14 + axis_swap_index(k - 14, d);
   return k;
 }
 
@@ -1402,18 +1717,124 @@ template <class L> GPR_D void w_system_matrix(EigWS<L::V> &ws, const DevPar &P, 
   __syncwarp();
 }
 
+// Osher interface terms at one point along D: f = D + F(qL) + F(qR), b = Bint.
+template <class L, int D>
+GPR_D void osher_point(const double *ql, const double *qr, const DevPar &P, const Consts &C,
+                       double *f, double *b) {
+  constexpr int V = L::V;
+  eig_dissipation_qd<L, NN>(ql, qr, D, GPR_FLUX_OSHER, P, C.nodes, C.w, f);
+  Prim<L::THERMAL> sl, sr;
+  prim<L::THERMAL>(ql, P, sl);
+  prim<L::THERMAL>(qr, P, sr);
+  flux_add<L::THERMAL, V>(ql, sl, D, P, f);
+  flux_add<L::THERMAL, V>(qr, sr, D, P, f);
+  double dq[V];
+#pragma unroll
+  for (int k = 0; k < V; k++)
+    dq[k] = qr[k] - ql[k];
+  path_product<L, NN>(ql, dq, D, C.nodes, C.w, b);
+}
+
+// 2D faces with the Osher dissipation in closed form: the lanes, passes and
+// in-place update of k_faces2d.
+template <class L, int DIR>
+__global__ void __launch_bounds__(128) k_faces2d_osher(
+    double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double ih,
+    int time_dg, DevPar P, Consts C, int parity) {
+  constexpr int V = L::V;
+  double f[V], b[V];
+  faces2d_body<L, DIR>(fb, qh, nx, ny, mask, dt, dt_dev, ih, time_dg, C, parity, f, b,
+                       [&](const double *ql, const double *qr) {
+                         osher_point<L, DIR>(ql, qr, P, C, f, b);
+                       });
+}
+
+// 1D faces with the Osher dissipation in closed form, one lane per (face,
+// time node, side) as k_faces1d_split: side 0 (1) evaluates the flux of qL (qR)
+// and path node 0 (1) of the dissipation and of Bint.  A face with a point the
+// closed form declines gets OSHER_MARK in its first entry, and the
+// warp-cooperative k_faces1d_eigw, launched next, evaluates the marked faces
+// (on the device: whether there are any is not known to the host; the launch
+// of blocks that return at once takes ~3 us).  The general routine per thread
+// would give this kernel an 18 KB stack, which a caller that cannot let the
+// device allocate must not meet.
+constexpr unsigned long long OSHER_MARK = 0x7ff8000000000badull;
+template <class L>
+__global__ void __launch_bounds__(128) k_faces1d_osher(
+    double *__restrict__ fb, const double *__restrict__ qh, long nface,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double idx,
+    int time_dg, DevPar P, Consts C) {
+  constexpr int V = L::V;
+  static_assert(NN == 2, "two time nodes and two path nodes");
+  if (dt_dev)
+    dt = *dt_dev;
+  const long face = (blockIdx.x * (long)blockDim.x + threadIdx.x) / 4;
+  const int lq = threadIdx.x % 4, t = lq >> 1, side = lq & 1;
+  const bool valid = face < nface;
+  const long fi = valid ? face : 0;
+  const bool on = valid && (mask == nullptr || (mask[fi] && mask[fi + 1]));
+  const bool active = on && (time_dg || t == 0);
+  const int nt = time_dg ? NN : 1, tt = time_dg ? t : 0;
+  const double *ql_ = qh + (fi * nt + tt) * NN * V, *qr_ = qh + ((fi + 1) * nt + tt) * NN * V;
+  double ql[V], qr[V], dq[V], f[V], b[V];
+  bool flat = true;
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    ql[k] = C.endv[1][0] * ql_[k] + C.endv[1][1] * ql_[V + k];
+    qr[k] = C.endv[0][0] * qr_[k] + C.endv[0][1] * qr_[V + k];
+    dq[k] = ql[k] - qr[k];
+    f[k] = 0.0;
+    flat = flat && (__double_as_longlong(dq[k]) << 1) == 0;
+  }
+  bool ok = true;
+  if (active && !flat) {
+    double q[V];
+    const double xn = C.nodes[side];
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      q[k] = fma(xn, dq[k], qr[k]);
+    ok = abs_apply_acoustic<L>(q, dq, GAUSS_W, P, f);
+  }
+  {
+    double qs[V];
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+      qs[k] = side ? qr[k] : ql[k];
+      dq[k] = -dq[k];
+    }
+    Prim<L::THERMAL> s;
+    prim<L::THERMAL>(qs, P, s);
+    flux_add<L::THERMAL, V>(qs, s, 0, P, f);
+    const double xn = C.nodes[side];
+    const double wr = GAUSS_W * rcp64(fma(xn, dq[0], ql[0]));
+    const double v[3] = {fma(xn, dq[2], ql[2]) * wr, fma(xn, dq[3], ql[3]) * wr,
+                         fma(xn, dq[4], ql[4]) * wr};
+    bdot<V, L::LSET>(v, dq, 0, b);
+  }
+  const double kk = dt * idx * (time_dg ? 0.5 * GAUSS_W : 0.5);
+  face_reduce_store<V, 4>(b, f, kk, active, valid, lq, fb + fi * 2 * V);
+  const unsigned lane = threadIdx.x & 31u;
+  const bool bad = (__ballot_sync(0xffffffffu, !ok) >> (lane & ~3u)) & 0xfu;
+  __syncwarp();
+  // lane 0 of the face holds entry 0 after the reduction
+  if (valid && bad && lq == 0)
+    fb[fi * 2 * V] = __longlong_as_double((long long)OSHER_MARK);
+}
+
 // 1D faces with the Osher or Roe dissipation: one block per face, one warp
 // per eigen-decomposition: warp w = t * NPATH + i handles time node t and,
 // for Osher, path node i (NPATH = 2; Roe averages the path's matrices in one
 // warp, NPATH = 1).  The contributions are summed in the serial order (path
-// nodes, then time nodes); output as k_faces1d.
+// nodes, then time nodes); output as k_faces1d.  Roe's flux, and the Osher
+// points that the closed form declines (marked != 0).
 constexpr int EIG_WARPS = 4;
 
 template <class L, bool BATCH = false>
 __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
     double *__restrict__ fb, const double *__restrict__ qh, long nface,
     const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
-    int time_dg, int flux, DevPar Pv, Consts C, Batch B) {
+    int time_dg, int flux, DevPar Pv, Consts C, Batch B, int marked) {
   constexpr int V = L::V;
   __shared__ EigWS<V> wsa[EIG_WARPS];
   __shared__ double part[NN][2][V];
@@ -1423,6 +1844,11 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
   const long face = blockIdx.x;
   if (face >= nface)
     return;  // block-uniform
+  // marked: only the faces k_faces1d_osher left (block-uniform: the block
+  // writes the entry after its last barrier)
+  if (marked &&
+      (unsigned long long)__double_as_longlong(fb[face * 2 * V]) != OSHER_MARK)
+    return;
   long fi = face;
   const int inst = BATCH ? B.inst_f[face] : 0;
   const DevPar &P = BATCH ? B.P[inst] : Pv;
