@@ -272,10 +272,10 @@ template <class L> struct Ops {
   static long fv_scratch(const int32_t *nX, int nd) {
     if (nd == 1)
       return (long)(nX[0] + 1) * 2 * V;
-    // x and y face sums, then the per-point terms of one direction (Osher /
-    // Roe, k_faces2d_eigp)
+    // x and y face sums, then the per-point terms of both directions (Roe,
+    // k_faces2d_eigp)
     const long nf = (long)(nX[0] + 1) * (nX[1] + 1);
-    return 2L * nf * 2 * V + nf * NN * NN * 2 * V;
+    return 2L * nf * 2 * V + 2L * nf * NN * NN * 2 * V;
   }
 
   // parts: FV_BOTH (fv_launcher), FV_CENTERS (centers1/2: the volume term,
@@ -334,8 +334,7 @@ template <class L> struct Ops {
     // and face terms
     long nf = (long)(nx + 1) * (ny + 1);
     double *fbx = scratch, *fby = scratch + nf * 2 * V, *pp = scratch + 2 * nf * 2 * V;
-    faces2d_eig(fbx, pp, qh, nx, ny, 0, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
-    faces2d_eig(fby, pp, qh, nx, ny, 1, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
+    faces2d_eig(fbx, pp, qh, nx, ny, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
     k_cells<L, 2><<<blocks(nc, 128), 128, 0, st>>>(u, qh, fbx, fby, nx, ny, mask, dt, dt_dev,
                                                     hx, hy, sources, time_dg, P, C, Batch{},
                                                     parts);
@@ -362,9 +361,7 @@ template <class L> struct Ops {
     long nf = (long)(nx + 1) * (ny + 1);
     if (flux != GPR_FLUX_RUSANOV && !osher_closed(flux, P)) {
       double *pp = fb + 2 * nf * 2 * V;
-      faces2d_eig(fb, pp, qh, nx, ny, 0, mask, dt, nullptr, dX, time_dg, flux, P, C, st);
-      faces2d_eig(fb + nf * 2 * V, pp, qh, nx, ny, 1, mask, dt, nullptr, dX, time_dg, flux, P,
-                  C, st);
+      faces2d_eig(fb, pp, qh, nx, ny, mask, dt, nullptr, dX, time_dg, flux, P, C, st);
       return cuda_rc();
     }
     launch_faces2d(fb, qh, nx, ny, 0, -1, mask, dt, nullptr, 1.0 / dX[0], time_dg, flux, P, C,
@@ -414,17 +411,17 @@ template <class L> struct Ops {
                                           par);
   }
 
-  // Osher / Roe faces of one direction on a 2D grid: one thread per face
-  // quadrature point into the per-point buffer pp (nf x 4 x 2V doubles),
-  // then the face sums into fb.
-  static void faces2d_eig(double *fb, double *pp, const double *qh, int nx, int ny, int dir,
+  // Roe faces of a 2D grid (k_faces2d_eigp): one thread per quadrature point
+  // of both directions into pp (2 x nf x 4 x 2V doubles), then the face sums
+  // into fb (2 x nf x 2V).
+  static void faces2d_eig(double *fb, double *pp, const double *qh, int nx, int ny,
                           const uint8_t *mask, double dt, const double *dt_dev, const double *dX,
                           int time_dg, int flux, const DevPar &P, const Consts &C,
                           cudaStream_t st) {
     long nf = (long)(nx + 1) * (ny + 1);
-    k_faces2d_eigp<L><<<blocks(nf * NN * NN, 64), 64, 0, st>>>(
-        pp, qh, nx, ny, dir, mask, dt, dt_dev, dX[0], dX[1], time_dg, flux, P, C);
-    k_faces2d_eigsum<V><<<blocks(nf * 2 * V, 256), 256, 0, st>>>(fb, pp, nf);
+    k_faces2d_eigp<L><<<dim3(blocks(nf * NN * NN, 64), 2), 64, 0, st>>>(
+        pp, qh, nx, ny, mask, dt, dt_dev, dX[0], dX[1], time_dg, flux, P, C);
+    k_faces2d_eigsum<V><<<blocks(2 * nf * 2 * V, 256), 256, 0, st>>>(fb, pp, 2 * nf);
   }
 
   static int timestep(const double *u, long ncell, const double *dX, int nd, double cfl,

@@ -597,8 +597,9 @@ GPR_D void schur_vectors(const double *T, const double *Z, const double *wr, con
   }
 }
 
-// Complex Gaussian elimination with partial pivoting: (Cr + i Ci) x = b,
-// b = (br + i bi) overwritten by x.  Returns false if singular.
+// Complex Gaussian elimination with partial pivoting: (Cr + i Ci) x = b for
+// two right-hand sides b = (br + i bi)[2][n], overwritten by x.  Returns false
+// if singular.
 template <int n> GPR_D bool csolve_n(double *Cr, double *Ci, double *br, double *bi) {
 #pragma unroll 1
   for (int c = 0; c < n; c++) {
@@ -615,21 +616,21 @@ template <int n> GPR_D bool csolve_n(double *Cr, double *Ci, double *br, double 
     if (best == 0.0)
       return false;
     if (p != c) {
+      auto swap = [](double &x, double &y) {
+        const double t = x;
+        x = y;
+        y = t;
+      };
 #pragma unroll 1
       for (int j = 0; j < n; j++) {
-        double t = Cr[c * n + j];
-        Cr[c * n + j] = Cr[p * n + j];
-        Cr[p * n + j] = t;
-        t = Ci[c * n + j];
-        Ci[c * n + j] = Ci[p * n + j];
-        Ci[p * n + j] = t;
+        swap(Cr[c * n + j], Cr[p * n + j]);
+        swap(Ci[c * n + j], Ci[p * n + j]);
       }
-      double t = br[c];
-      br[c] = br[p];
-      br[p] = t;
-      t = bi[c];
-      bi[c] = bi[p];
-      bi[p] = t;
+#pragma unroll 1
+      for (int h = 0; h < 2 * n; h += n) {
+        swap(br[h + c], br[h + p]);
+        swap(bi[h + c], bi[h + p]);
+      }
     }
     const double pr = Cr[c * n + c], pi = Ci[c * n + c];
     const double den = pr * pr + pi * pi;
@@ -643,63 +644,248 @@ template <int n> GPR_D bool csolve_n(double *Cr, double *Ci, double *br, double 
         Cr[r * n + j] -= fr * xr - fi * xi;
         Ci[r * n + j] -= fr * xi + fi * xr;
       }
-      br[r] -= fr * br[c] - fi * bi[c];
-      bi[r] -= fr * bi[c] + fi * br[c];
+#pragma unroll 1
+      for (int h = 0; h < 2 * n; h += n) {
+        const double xr = br[h + c], xi = bi[h + c];
+        br[h + r] -= fr * xr - fi * xi;
+        bi[h + r] -= fr * xi + fi * xr;
+      }
     }
   }
 #pragma unroll 1
-  for (int r = n - 1; r >= 0; r--) {
-    double sr = br[r], si = bi[r];
+  for (int h = 0; h < 2 * n; h += n)
 #pragma unroll 1
-    for (int j = r + 1; j < n; j++) {
-      sr -= Cr[r * n + j] * br[j] - Ci[r * n + j] * bi[j];
-      si -= Cr[r * n + j] * bi[j] + Ci[r * n + j] * br[j];
+    for (int r = n - 1; r >= 0; r--) {
+      double sr = br[h + r], si = bi[h + r];
+#pragma unroll 1
+      for (int j = r + 1; j < n; j++) {
+        sr -= Cr[r * n + j] * br[h + j] - Ci[r * n + j] * bi[h + j];
+        si -= Cr[r * n + j] * bi[h + j] + Ci[r * n + j] * br[h + j];
+      }
+      const double pr = Cr[r * n + r], pi = Ci[r * n + r];
+      const double den = pr * pr + pi * pi;
+      br[h + r] = (sr * pr + si * pi) / den;
+      bi[h + r] = (si * pr - sr * pi) / den;
     }
-    const double pr = Cr[r * n + r], pi = Ci[r * n + r];
-    const double den = pr * pr + pi * pi;
-    br[r] = (sr * pr + si * pi) / den;
-    bi[r] = (si * pr - sr * pi) / den;
-  }
   return true;
 }
 
-// acc += w R |Lambda| R^-1 dq for M (n x n row-major, destroyed).
-template <int n> GPR_D bool abs_apply(double *M, const double *dq, double w, double *acc) {
-  double Z[n * n], wr[n], wi[n], Rr[n * n], Ri[n * n], Cr[n * n], Ci[n * n];
+// The system matrix along x, or an average of it over states, leaves six
+// distortion entries (A_k1, A_k2) and the level sets as they are but for the
+// advection velocity vb on their diagonal:
+//   M = [[C, B], [0, vb I]],   |M| (w, a) = (|C| w + g(C) B a, |vb| a),
+// g(x) = (|x| - |vb|) / (x - vb), so only C is decomposed: 11 x 11 with heat
+// conduction, else 8 x 8 (in place of 17 x 17 and 14 x 14: a quarter and a
+// fifth of the work and of the local memory).  Entry r of the active part is
+// state entry active_entry(r).
+template <class L> constexpr int ACTIVE_N = L::THERMAL ? 11 : 8;
+GPR_HD constexpr int active_entry(int r) {
+  return r < 5 ? r : (r < 8 ? 5 + 3 * (r - 5) : 14 + (r - 8));
+}
+template <class L> GPR_HD constexpr bool passive_entry(int k) {
+  return (k >= 5 && k < 14 && (k - 5) % 3 != 0) || k >= L::V - L::LSET;
+}
+
+// |l| and g(l) of one eigenvalue l = lr + i li.  For a real l of vb's sign g is
+// that sign whatever l - vb (a semisimple l = vb included).
+GPR_D void abs_factors(double lr, double li, double vb, double &fa, double &gr, double &gi) {
+  gi = 0.0;
+  if (li == 0.0) {
+    fa = fabs(lr);
+    if ((lr >= 0.0) == (vb >= 0.0))
+      gr = vb >= 0.0 ? 1.0 : -1.0;
+    else
+      gr = (fa - fabs(vb)) / (lr - vb);
+    return;
+  }
+  fa = hypot(lr, li);
+  const double dr = lr - vb, den = dr * dr + li * li, num = fa - fabs(vb);
+  gr = num * dr / den;
+  gi = -num * li / den;
+}
+
+// C (ld n) and Ba of wt times the system matrix of q along x, added to C and
+// Ba; returns wt v_x.  dF/dP and dP/dQ have a few nonzeros per row, known at
+// compile time: the products are written for those (about 300 in place of
+// V^3 = 4913).
+template <class L>
+GPR_D double system_active(const double *q, const double *a, double wt, const DevPar &P,
+                           double *C, double *Ba) {
+  constexpr int V = L::V, n = ACTIVE_N<L>;
+  double F[V * V], D[V * V];
+#pragma unroll
+  for (int i = 0; i < V * V; i++)
+    F[i] = D[i] = 0.0;
+  Prim<L::THERMAL> s;
+  prim<L::THERMAL>(q, P, s);
+  system_fd<L::THERMAL, V>(q, s, P, F, D);
+#pragma unroll
+  for (int r = 0; r < n; r++) {
+    const int R = active_entry(r);
+    double ba = 0.0;
+#pragma unroll
+    for (int j = 0; j < V - L::LSET; j++) {
+      // row R of dF/dP: entry 1 (pressure) for E, m_x and J_x only
+      const bool press = R == 1 || R == 2 || R == 14;
+      double x = j == 1 ? 0.0 : F[R * V + j] * D[j * V + j];
+      if (press)
+        x = fma(F[R * V + 1], D[V + j], x);
+      if (j == 0) {
+#pragma unroll
+        for (int k = 2; k < 5; k++)
+          x = fma(F[R * V + k], D[k * V], x);
+        if (L::THERMAL) {
+#pragma unroll
+          for (int k = 14; k < 17; k++)
+            x = fma(F[R * V + k], D[k * V], x);
+        }
+      }
+      // B_x: v_x on the distortion's diagonal, -v_j in the x rows
+      if (R >= 5 && R < 14) {
+        if (j == R)
+          x += s.v[0];
+        if (j >= R && j < R + 3)
+          x -= s.v[j - R];
+      }
+      if (passive_entry<L>(j)) {
+        ba = fma(x, a[j], ba);
+      } else {
+        const int c = j < 5 ? j : (j < 14 ? 5 + (j - 5) / 3 : j - 6);
+        C[r * n + c] = fma(wt, x, C[r * n + c]);
+      }
+    }
+    Ba[r] = fma(wt, ba, Ba[r]);
+  }
+  return wt * s.v[0];
+}
+
+// acc += w |M| dq for M given by C (n x n row-major, destroyed), Ba = B a (a the
+// passive part of dq) and vb.  With a real spectrum the eigenvectors are Z Y, Y
+// unit upper triangular (back-substitution on the Schur form), so R^-1 is Z^T
+// and a triangular solve; complex eigenvalues take the complex elimination.
+template <class L>
+GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, double w,
+                     double *acc) {
+  constexpr int V = L::V, n = ACTIVE_N<L>;
+  double Z[n * n], wr[n], wi[n], y[n];
 #pragma unroll 1
   for (int i = 0; i < n * n; i++)
     Z[i] = (i % (n + 1) == 0) ? 1.0 : 0.0;
-  hess_reduce<n>(M, Z);
-  if (!hqr_schur<n>(M, Z, wr, wi))
+  hess_reduce<n>(C, Z);
+  if (!hqr_schur<n>(C, Z, wr, wi))
     return false;
-  schur_vectors<n>(M, Z, wr, wi, Rr, Ri);
+  bool real = true;
 #pragma unroll 1
-  for (int i = 0; i < n * n; i++) {
-    Cr[i] = Rr[i];
-    Ci[i] = Ri[i];
+  for (int k = 0; k < n; k++)
+    real = real && wi[k] == 0.0;
+  double dw[n];
+#pragma unroll
+  for (int r = 0; r < n; r++)
+    dw[r] = dq[active_entry(r)];
+  if (real) {
+    double norm = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < n; i++)
+#pragma unroll 1
+      for (int j = i; j < n; j++)
+        norm += fabs(C[i * n + j]);
+    const double tol = OSH_MULT_TOL * norm;
+    double Y[n * n], c2[n];  // Y by columns
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+      double x1 = 0.0, x2 = 0.0;
+#pragma unroll 1
+      for (int i = 0; i < n; i++) {
+        x1 += Z[i * n + k] * dw[i];
+        x2 += Z[i * n + k] * Ba[i];
+      }
+      y[k] = x1;
+      c2[k] = x2;
+      Y[k * n + k] = 1.0;
+#pragma unroll 1
+      for (int i = k - 1; i >= 0; i--) {
+        double sum = 0.0;
+#pragma unroll 1
+        for (int j = i + 1; j <= k; j++)
+          sum += C[i * n + j] * Y[k * n + j];
+        const double d = C[i * n + i] - wr[k];
+        // the same eigenvalue: an independent Schur vector
+        Y[k * n + i] = fabs(d) <= tol ? 0.0 : -sum / d;
+      }
+    }
+#pragma unroll 1
+    for (int k = n - 1; k >= 0; k--) {
+#pragma unroll 1
+      for (int i = 0; i < k; i++) {
+        y[i] -= Y[k * n + i] * y[k];
+        c2[i] -= Y[k * n + i] * c2[k];
+      }
+      double fa, gr, gi;
+      abs_factors(wr[k], 0.0, vb, fa, gr, gi);
+      y[k] = fa * y[k] + gr * c2[k];
+    }
+    // Y y (column by column, downwards in place), then Z
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+      double sum = y[i];
+#pragma unroll 1
+      for (int k = i + 1; k < n; k++)
+        sum += Y[k * n + i] * y[k];
+      y[i] = sum;
+    }
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+      double sum = 0.0;
+#pragma unroll 1
+      for (int k = 0; k < n; k++)
+        sum += Z[i * n + k] * y[k];
+      c2[i] = sum;
+    }
+#pragma unroll
+    for (int r = 0; r < n; r++)
+      acc[active_entry(r)] += w * c2[r];
+  } else {
+    double Rr[n * n], Ri[n * n], br[2 * n], bi[2 * n];
+    schur_vectors<n>(C, Z, wr, wi, Rr, Ri);
+    // C and Z are free: the elimination's copy of R
+#pragma unroll 1
+    for (int i = 0; i < n * n; i++) {
+      C[i] = Rr[i];
+      Z[i] = Ri[i];
+    }
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+      br[k] = dw[k];
+      br[n + k] = Ba[k];
+      bi[k] = bi[n + k] = 0.0;
+    }
+    if (!csolve_n<n>(C, Z, br, bi))
+      return false;
+#pragma unroll 1
+    for (int k = 0; k < n; k++) {
+      double fa, gr, gi;
+      abs_factors(wr[k], wi[k], vb, fa, gr, gi);
+      const double xr = fa * br[k] + (gr * br[n + k] - gi * bi[n + k]);
+      bi[k] = fa * bi[k] + (gr * bi[n + k] + gi * br[n + k]);
+      br[k] = xr;
+    }
+#pragma unroll 1
+    for (int i = 0; i < n; i++) {
+      double sum = 0.0;
+#pragma unroll 1
+      for (int k = 0; k < n; k++)
+        sum += Rr[i * n + k] * br[k] - Ri[i * n + k] * bi[k];
+      y[i] = sum;
+    }
+#pragma unroll
+    for (int r = 0; r < n; r++)
+      acc[active_entry(r)] += w * y[r];
   }
-  double br[n], bi[n];
-#pragma unroll 1
-  for (int k = 0; k < n; k++) {
-    br[k] = dq[k];
-    bi[k] = 0.0;
-  }
-  if (!csolve_n<n>(Cr, Ci, br, bi))
-    return false;
-#pragma unroll 1
-  for (int k = 0; k < n; k++) {
-    const double a = hypot(wr[k], wi[k]);
-    br[k] *= a;
-    bi[k] *= a;
-  }
-#pragma unroll 1
-  for (int i = 0; i < n; i++) {
-    double s = 0.0;
-#pragma unroll 1
-    for (int k = 0; k < n; k++)
-      s += Rr[i * n + k] * br[k] - Ri[i * n + k] * bi[k];
-    acc[i] += w * s;
-  }
+  const double av = w * fabs(vb);
+#pragma unroll
+  for (int k = 5; k < V; k++)
+    if (passive_entry<L>(k))
+      acc[k] = fma(av, dq[k], acc[k]);
   return true;
 }
 
@@ -983,12 +1169,16 @@ GPR_D bool abs_apply_acoustic(const double *q, const double *dq, double w, const
 template <class L>
 __device__ __noinline__ bool abs_apply_general(const double *q, const double *dq, double w,
                                                const DevPar &P, double *f) {
-  constexpr int V = L::V;
-  double M[V * V];
-  Prim<L::THERMAL> s;
-  prim<L::THERMAL>(q, P, s);
-  system_matrix<L::THERMAL, V>(q, s, P, M);
-  return abs_apply<V>(M, dq, w, f);
+  constexpr int n = ACTIVE_N<L>;
+  double C[n * n], Ba[n];
+#pragma unroll 1
+  for (int i = 0; i < n * n; i++)
+    C[i] = 0.0;
+#pragma unroll
+  for (int i = 0; i < n; i++)
+    Ba[i] = 0.0;
+  const double vb = system_active<L>(q, dq, 1.0, P, C, Ba);
+  return abs_apply<L>(C, Ba, vb, dq, w, f);
 }
 
 // Eigen part of D_OSH along x into f (overwritten): sum_i w_i |M(q_i)| dq
@@ -1041,7 +1231,8 @@ GPR_D void eig_dissipation_q(const double *ql, const double *qr, int flux, const
     osher_dissipation<L, NQ>(ql, qr, P, nodes, wts, f);
     return;
   }
-  double dq[V], q[V], M[V * V], Mi[V * V];
+  constexpr int n = ACTIVE_N<L>;
+  double dq[V], q[V], C[n * n], Ba[n];
   bool flat = true;
 #pragma unroll
   for (int k = 0; k < V; k++) {
@@ -1054,21 +1245,20 @@ GPR_D void eig_dissipation_q(const double *ql, const double *qr, int flux, const
   if (flat)
     return;
 #pragma unroll 1
-  for (int i = 0; i < V * V; i++)
-    M[i] = 0.0;
+  for (int i = 0; i < n * n; i++)
+    C[i] = 0.0;
+#pragma unroll
+  for (int i = 0; i < n; i++)
+    Ba[i] = 0.0;
+  double vb = 0.0;
 #pragma unroll 1
   for (int i = 0; i < NQ; i++) {
 #pragma unroll
     for (int k = 0; k < V; k++)
       q[k] = qr[k] + nodes[i] * dq[k];
-    Prim<L::THERMAL> s;
-    prim<L::THERMAL>(q, P, s);
-    system_matrix<L::THERMAL, V>(q, s, P, Mi);
-#pragma unroll 1
-    for (int k = 0; k < V * V; k++)
-      M[k] += wts[i] * Mi[k];
+    vb += system_active<L>(q, dq, wts[i], P, C, Ba);
   }
-  if (!abs_apply<V>(M, dq, 1.0, f)) {
+  if (!abs_apply<L>(C, Ba, vb, dq, 1.0, f)) {
 #pragma unroll
     for (int k = 0; k < V; k++)
       f[k] = __longlong_as_double(0x7ff8000000000000ll);
@@ -1153,14 +1343,15 @@ GPR_D void interface_point_eig(const double *ql, const double *qr, int flux, con
 // eigenvectors are one lane each; the complex solve eliminates one row per
 // lane.  The arithmetic of every element update is the serial one.
 
-// Per-warp workspace.  After the eigenvectors are formed, H and Z (the
-// Schur form and vectors) are no longer needed and hold the copy of the
-// eigenvector matrix that the complex solve factorises; before the
-// eigen-decomposition Rr and Ri hold dF/dP and dP/dQ.
-template <int n> struct EigWS {
-  double H[n * n], Z[n * n], Rr[n * n], Ri[n * n];
-  double wr[n], wi[n], v[n], br[n], bi[n];
-  double q[n], ql[n], qr[n], dq[n], f[n];
+// Per-warp workspace.  H and Z are the active matrix and its Schur vectors;
+// Rr and Ri hold dF/dP and dP/dQ before the eigen-decomposition, then the
+// eigenvectors (Y in Rr for a real spectrum; for a complex one H and Z
+// afterwards hold the copy that the complex solve factorises).
+template <class L> struct EigWS {
+  static constexpr int V = L::V, n = ACTIVE_N<L>;
+  double H[n * n], Z[n * n], Rr[V * V], Ri[V * V];
+  double wr[n], wi[n], v[n > 3 ? n : 3], br[2 * n], bi[2 * n], Ba[n], vb;
+  double q[V], ql[V], qr[V], dq[V], f[V];
 };
 
 GPR_D double warp_sum(double x) {
@@ -1594,13 +1785,14 @@ GPR_D bool w_csolve(double *Cr, double *Ci, double *br, double *bi, int lane) {
         Ci[c * n + j] = Ci[p * n + j];
         Ci[p * n + j] = t;
       }
-      if (lane == 0) {
-        double t = br[c];
-        br[c] = br[p];
-        br[p] = t;
-        t = bi[c];
-        bi[c] = bi[p];
-        bi[p] = t;
+      if (lane < 2) {
+        const int h = lane * n;
+        double t = br[h + c];
+        br[h + c] = br[h + p];
+        br[h + p] = t;
+        t = bi[h + c];
+        bi[h + c] = bi[h + p];
+        bi[h + p] = t;
       }
     }
     __syncwarp();
@@ -1614,34 +1806,38 @@ GPR_D bool w_csolve(double *Cr, double *Ci, double *br, double *bi, int lane) {
         Cr[r * n + j] -= fr * xr - fi * xi;
         Ci[r * n + j] -= fr * xi + fi * xr;
       }
-      br[r] -= fr * br[c] - fi * bi[c];
-      bi[r] -= fr * bi[c] + fi * br[c];
+      for (int h = 0; h < 2 * n; h += n) {
+        const double xr = br[h + c], xi = bi[h + c];
+        br[h + r] -= fr * xr - fi * xi;
+        bi[h + r] -= fr * xi + fi * xr;
+      }
     }
     __syncwarp();
   }
+  // back-substitution, one right-hand side per lane
+  if (lane < 2) {
+    const int h = lane * n;
 #pragma unroll 1
-  for (int r = n - 1; r >= 0; r--) {
-    double sr = 0.0, si = 0.0;
-    for (int j = r + 1 + lane; j < n; j += 32) {
-      sr += Cr[r * n + j] * br[j] - Ci[r * n + j] * bi[j];
-      si += Cr[r * n + j] * bi[j] + Ci[r * n + j] * br[j];
-    }
-    sr = warp_sum(sr);
-    si = warp_sum(si);
-    if (lane == 0) {
-      const double xr = br[r] - sr, xi = bi[r] - si;
+    for (int r = n - 1; r >= 0; r--) {
+      double sr = br[h + r], si = bi[h + r];
+      for (int j = r + 1; j < n; j++) {
+        sr -= Cr[r * n + j] * br[h + j] - Ci[r * n + j] * bi[h + j];
+        si -= Cr[r * n + j] * bi[h + j] + Ci[r * n + j] * br[h + j];
+      }
       const double pr = Cr[r * n + r], pi = Ci[r * n + r];
       const double den = pr * pr + pi * pi;
-      br[r] = (xr * pr + xi * pi) / den;
-      bi[r] = (xi * pr - xr * pi) / den;
+      br[h + r] = (sr * pr + si * pi) / den;
+      bi[h + r] = (si * pr - sr * pi) / den;
     }
-    __syncwarp();
   }
+  __syncwarp();
   return true;
 }
 
-// ws.f += w R |Lambda| R^-1 ws.dq for the matrix in ws.H (destroyed)
-template <int n> GPR_D bool w_abs_apply(EigWS<n> &ws, double w, int lane) {
+// ws.f += w |M| ws.dq for M given by ws.H (C, destroyed), ws.Ba and ws.vb, as
+// abs_apply.
+template <class L> GPR_D bool w_abs_apply(EigWS<L> &ws, double w, int lane) {
+  constexpr int V = L::V, n = ACTIVE_N<L>;
   for (int e = lane; e < n * n; e += 32)
     ws.Z[e] = (e % (n + 1) == 0) ? 1.0 : 0.0;
   __syncwarp();
@@ -1649,45 +1845,104 @@ template <int n> GPR_D bool w_abs_apply(EigWS<n> &ws, double w, int lane) {
   if (!w_hqr<n>(ws.H, ws.Z, ws.wr, ws.wi, lane))
     return false;
   __syncwarp();
-  w_schur_vectors<n>(ws.H, ws.Z, ws.wr, ws.wi, ws.Rr, ws.Ri, lane);
-  double *Cr = ws.H, *Ci = ws.Z;
-  for (int e = lane; e < n * n; e += 32) {
-    Cr[e] = ws.Rr[e];
-    Ci[e] = ws.Ri[e];
+  const bool real = __all_sync(0xffffffffu, lane >= n || ws.wi[lane < n ? lane : 0] == 0.0);
+  double out = 0.0;  // entry `lane` of the active result
+  if (real) {
+    double nrm = 0.0;
+    for (int e = lane; e < n * n; e += 32)
+      if (e % n >= e / n)
+        nrm += fabs(ws.H[e]);
+    const double tol = OSH_MULT_TOL * warp_sum(nrm);
+    double *Y = ws.Rr, *y = ws.br, *c2 = ws.br + n;  // Y by columns
+    if (lane < n) {
+      const int k = lane;
+      double x1 = 0.0, x2 = 0.0;
+      for (int i = 0; i < n; i++) {
+        x1 += ws.Z[i * n + k] * ws.dq[active_entry(i)];
+        x2 += ws.Z[i * n + k] * ws.Ba[i];
+      }
+      y[k] = x1;
+      c2[k] = x2;
+      Y[k * n + k] = 1.0;
+      for (int i = k - 1; i >= 0; i--) {
+        double sum = 0.0;
+        for (int j = i + 1; j <= k; j++)
+          sum += ws.H[i * n + j] * Y[k * n + j];
+        const double d = ws.H[i * n + i] - ws.wr[k];
+        Y[k * n + i] = fabs(d) <= tol ? 0.0 : -sum / d;
+      }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int k = n - 1; k > 0; k--) {
+      if (lane < k) {
+        y[lane] -= Y[k * n + lane] * y[k];
+        c2[lane] -= Y[k * n + lane] * c2[k];
+      }
+      __syncwarp();
+    }
+    if (lane < n) {
+      double fa, gr, gi;
+      abs_factors(ws.wr[lane], 0.0, ws.vb, fa, gr, gi);
+      y[lane] = fa * y[lane] + gr * c2[lane];
+    }
+    __syncwarp();
+    double sum = 0.0;
+    if (lane < n)
+      for (int k = lane; k < n; k++)
+        sum += Y[k * n + lane] * y[k];
+    if (lane < n)
+      c2[lane] = sum;
+    __syncwarp();
+    if (lane < n)
+      for (int k = 0; k < n; k++)
+        out += ws.Z[lane * n + k] * c2[k];
+  } else {
+    w_schur_vectors<n>(ws.H, ws.Z, ws.wr, ws.wi, ws.Rr, ws.Ri, lane);
+    double *Cr = ws.H, *Ci = ws.Z;
+    for (int e = lane; e < n * n; e += 32) {
+      Cr[e] = ws.Rr[e];
+      Ci[e] = ws.Ri[e];
+    }
+    if (lane < n) {
+      ws.br[lane] = ws.dq[active_entry(lane)];
+      ws.br[n + lane] = ws.Ba[lane];
+      ws.bi[lane] = ws.bi[n + lane] = 0.0;
+    }
+    __syncwarp();
+    if (!w_csolve<n>(Cr, Ci, ws.br, ws.bi, lane))
+      return false;
+    if (lane < n) {
+      double fa, gr, gi;
+      abs_factors(ws.wr[lane], ws.wi[lane], ws.vb, fa, gr, gi);
+      const double b2r = ws.br[n + lane], b2i = ws.bi[n + lane];
+      ws.br[lane] = fa * ws.br[lane] + (gr * b2r - gi * b2i);
+      ws.bi[lane] = fa * ws.bi[lane] + (gr * b2i + gi * b2r);
+    }
+    __syncwarp();
+    if (lane < n)
+      for (int k = 0; k < n; k++)
+        out += ws.Rr[lane * n + k] * ws.br[k] - ws.Ri[lane * n + k] * ws.bi[k];
   }
-  for (int k = lane; k < n; k += 32) {
-    ws.br[k] = ws.dq[k];
-    ws.bi[k] = 0.0;
-  }
-  __syncwarp();
-  if (!w_csolve<n>(Cr, Ci, ws.br, ws.bi, lane))
-    return false;
-  for (int k = lane; k < n; k += 32) {
-    const double a = hypot(ws.wr[k], ws.wi[k]);
-    ws.br[k] *= a;
-    ws.bi[k] *= a;
-  }
-  __syncwarp();
-  for (int i = lane; i < n; i += 32) {
-    double s = 0.0;
-    for (int k = 0; k < n; k++)
-      s += ws.Rr[i * n + k] * ws.br[k] - ws.Ri[i * n + k] * ws.bi[k];
-    ws.f[i] += w * s;
-  }
+  if (lane < n)
+    ws.f[active_entry(lane)] += w * out;
+  for (int k = 5 + lane; k < V; k += 32)
+    if (passive_entry<L>(k))
+      ws.f[k] += w * fabs(ws.vb) * ws.dq[k];
   __syncwarp();
   return true;
 }
 
-// ws.H = M(ws.q) (system matrix); F and D are built in ws.Rr / ws.Ri by lane
-// 0, their product formed by all lanes.
-template <class L> GPR_D void w_system_matrix(EigWS<L::V> &ws, const DevPar &P, int lane) {
-  constexpr int V = L::V;
+// wt times the system matrix of ws.q added to ws.H, ws.Ba and ws.vb (as
+// system_active): F and D are built in ws.Rr / ws.Ri by lane 0, the products
+// formed by all lanes.
+template <class L> GPR_D void w_system_active(EigWS<L> &ws, double wt, const DevPar &P, int lane) {
+  constexpr int V = L::V, n = ACTIVE_N<L>;
   for (int e = lane; e < V * V; e += 32) {
     ws.Rr[e] = 0.0;
     ws.Ri[e] = 0.0;
   }
   __syncwarp();
-  double vloc[3];
   if (lane == 0) {
     double q[V];
 #pragma unroll
@@ -1701,19 +1956,37 @@ template <class L> GPR_D void w_system_matrix(EigWS<L::V> &ws, const DevPar &P, 
     ws.v[2] = s.v[2];
   }
   __syncwarp();
-  for (int e = lane; e < V * V; e += 32) {
-    const int i = e / V, j = e % V;
-    double acc = 0.0;
-    for (int k = 0; k < V; k++)
-      acc += ws.Rr[i * V + k] * ws.Ri[k * V + j];
-    ws.H[e] = acc;
+  const double *F = ws.Rr, *D = ws.Ri;
+  auto entry = [&](int R, int j) {  // M(R, j) of the active row R
+    double x = F[R * V + 1] * D[V + j];
+    if (j != 1)
+      x += F[R * V + j] * D[j * V + j];
+    if (j == 0) {
+      for (int k = 2; k < 5; k++)
+        x += F[R * V + k] * D[k * V];
+      if (L::THERMAL)
+        for (int k = 14; k < 17; k++)
+          x += F[R * V + k] * D[k * V];
+    }
+    if (R >= 5 && R < 14) {
+      if (j == R)
+        x += ws.v[0];
+      if (j >= R && j < R + 3)
+        x -= ws.v[j - R];
+    }
+    return x;
+  };
+  for (int e = lane; e < n * n; e += 32)
+    ws.H[e] += wt * entry(active_entry(e / n), active_entry(e % n));
+  if (lane < n) {
+    double ba = 0.0;
+    for (int j = 5; j < 14; j++)
+      if (passive_entry<L>(j))
+        ba += entry(active_entry(lane), j) * ws.dq[j];
+    ws.Ba[lane] += wt * ba;
   }
-  vloc[0] = ws.v[0];
-  vloc[1] = ws.v[1];
-  vloc[2] = ws.v[2];
-  __syncwarp();
   if (lane == 0)
-    system_block<V, L::LSET>(vloc, ws.H);
+    ws.vb += wt * ws.v[0];
   __syncwarp();
 }
 
@@ -1836,7 +2109,7 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
     const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
     int time_dg, int flux, DevPar Pv, Consts C, Batch B, int marked) {
   constexpr int V = L::V;
-  __shared__ EigWS<V> wsa[EIG_WARPS];
+  __shared__ EigWS<L> wsa[EIG_WARPS];
   __shared__ double part[NN][2][V];
   if (dt_dev)
     dt = *dt_dev;
@@ -1862,7 +2135,7 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
   const int npath = flux == GPR_FLUX_OSHER ? NN : 1;
   const int t = wid / npath, ip = wid % npath;
   const bool mine = active && t < nt;  // warp-uniform
-  EigWS<V> &ws = wsa[wid];
+  EigWS<L> &ws = wsa[wid];
   if (mine) {
     const double *ql_ = qh + (fi * nt + t) * NN * V;
     const double *qr_ = qh + ((fi + 1) * nt + t) * NN * V;
@@ -1880,31 +2153,24 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
       flat = flat && ws.dq[k] == 0.0;
     flat = __all_sync(0xffffffffu, flat);
     bool ok = true;
-    if (flat) {
-    } else if (flux == GPR_FLUX_OSHER) {
-      for (int k = lane; k < V; k += 32)
-        ws.q[k] = ws.qr[k] + C.nodes[ip] * ws.dq[k];
-      __syncwarp();
-      w_system_matrix<L>(ws, P, lane);
-      ok = w_abs_apply<V>(ws, C.w[ip], lane);
-    } else {
-      // Roe: the path-averaged matrix, accumulated in Z
-      for (int e = lane; e < V * V; e += 32)
-        ws.Z[e] = 0.0;
+    if (!flat) {
+      // Osher: this warp's path node; Roe: the path-averaged matrix
+      constexpr int n = ACTIVE_N<L>;
+      for (int e = lane; e < n * n; e += 32)
+        ws.H[e] = 0.0;
+      if (lane < n)
+        ws.Ba[lane] = 0.0;
+      if (lane == 0)
+        ws.vb = 0.0;
+      const bool osher = flux == GPR_FLUX_OSHER;
 #pragma unroll 1
-      for (int i = 0; i < NN; i++) {
+      for (int i = osher ? ip : 0; i < (osher ? ip + 1 : NN); i++) {
         for (int k = lane; k < V; k += 32)
           ws.q[k] = ws.qr[k] + C.nodes[i] * ws.dq[k];
         __syncwarp();
-        w_system_matrix<L>(ws, P, lane);
-        for (int e = lane; e < V * V; e += 32)
-          ws.Z[e] += C.w[i] * ws.H[e];
-        __syncwarp();
+        w_system_active<L>(ws, osher ? 1.0 : C.w[i], P, lane);
       }
-      for (int e = lane; e < V * V; e += 32)
-        ws.H[e] = ws.Z[e];
-      __syncwarp();
-      ok = w_abs_apply<V>(ws, 1.0, lane);
+      ok = w_abs_apply<L>(ws, osher ? C.w[ip] : 1.0, lane);
     }
     if (!ok) {
       for (int k = lane; k < V; k += 32)
@@ -1972,27 +2238,21 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
   }
 }
 
-// 2D Osher / Roe faces in two launches.  k_faces2d_eigp: one thread per face
-// quadrature point (time node t, transverse node s), as the pointwise
-// interface-terms kernel: it evaluates D_OSH / D_ROE + F(qL) + F(qR) and
-// the path integral of B, and stores kk (b + f) and kk (b - f) to
-// pp[face][lane][2][V].  k_faces2d_eigsum adds each face's four points as
-// a butterfly over the lanes would, (l0 + l1) + (l2 + l3), into
-// fb[face][2][V].  A one-kernel form (the four points of a face in
-// neighbouring lanes, summed by shuffles) gave, on two-material (V = 15)
-// grids, faces that differed from the oracle by up to 4e-2 (Osher only)
-// while the same states through the pointwise kernel matched it to 2e-15,
-// also under 1e-15 noise; this form keeps the per-point evaluation in the
-// pointwise kernel's shape.  With millions of independent eigenproblems in
-// a 512 x 512 step, one thread per eigenproblem beats a warp per
-// eigenproblem (k_faces1d_eigw, built for the few faces of a 1D grid).
+// 2D Roe faces (and Osher's where its closed form does not hold) in two
+// launches.  k_faces2d_eigp: one thread per face quadrature point (time node t,
+// transverse node s) of both directions (blockIdx.y): a point is one thread's
+// serial chain, so on grids of some thousand faces the two directions side by
+// side halve the time.  It stores kk (b + f) and kk (b - f) to
+// pp[dir][face][lane][2][V]; k_faces2d_eigsum adds each face's four points into
+// fb[dir][face][2][V].
 template <class L>
 __global__ void __launch_bounds__(64) k_faces2d_eigp(
-    double *__restrict__ pp, const double *__restrict__ qh, int nx, int ny, int dir,
+    double *__restrict__ pp, const double *__restrict__ qh, int nx, int ny,
     const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
     double dy, int time_dg, int flux, DevPar P, Consts C) {
   constexpr int V = L::V;
   constexpr int NQ = NN * NN;
+  const int dir = blockIdx.y;
   if (dt_dev)
     dt = *dt_dev;
   const long gt = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -2006,7 +2266,7 @@ __global__ void __launch_bounds__(64) k_faces2d_eigp(
   const long cn = dir == 0 ? cb + (ny + 2) : cb + 1;
   const bool geo = dir == 0 ? (j > 0) : (i > 0);
   const bool active = geo && (mask == nullptr || (mask[cb] && mask[cn])) && (time_dg || t == 0);
-  double *o = pp + gt * 2 * V;
+  double *o = pp + (dir * nf * NQ + gt) * 2 * V;
   if (!active) {
 #pragma unroll
     for (int k = 0; k < 2 * V; k++)
