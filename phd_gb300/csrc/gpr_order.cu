@@ -79,16 +79,28 @@ template <class L, int NO> struct OpsN {
     const double idx = 1.0 / dX[0], idy = g.nd == 2 ? 1.0 / dX[1] : 1.0;
     const ConstsN<NO> &C = consts_n<NO>();
     if (g.nd == 1) {
-      using NB = NodeBlock<NO, 1>;
-      k_predictor_n<L, NO, 1><<<(unsigned)((ncb + NB::CPB - 1) / NB::CPB), 128, 0, st>>>(
-          qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, stiff, P, C);
+      if (!stiff)
+        k_predictor_first_n<L, NO, 1>
+            <<<node_blocks<NodeBlock<NO, 1>::NS>(ncb, NodeBlock<NO, 1>::NW),
+               32 * NodeBlock<NO, 1>::NW, 0, st>>>(
+                qh, wh, ncb, mask, dt, dt_dev, idx, idy, P, C);
+      k_predictor_n<L, NO, 1>
+          <<<node_blocks<NodeBlock<NO, 1>::NP>(ncb, NodeBlock<NO, 1>::NW),
+             32 * NodeBlock<NO, 1>::NW, 0, st>>>(
+              qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, stiff, P, C);
       k_predictor_stiff_n<L, NO, 1><<<stiff_grid(k_predictor_stiff_n<L, NO, 1>, ncb), 32, 0,
                                       st>>>(qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, P,
                                             C);
     } else {
-      using NB = NodeBlock<NO, 2>;
-      k_predictor_n<L, NO, 2><<<(unsigned)((ncb + NB::CPB - 1) / NB::CPB), 128, 0, st>>>(
-          qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, stiff, P, C);
+      if (!stiff)
+        k_predictor_first_n<L, NO, 2>
+            <<<node_blocks<NodeBlock<NO, 2>::NS>(ncb, NodeBlock<NO, 2>::NW),
+               32 * NodeBlock<NO, 2>::NW, 0, st>>>(
+                qh, wh, ncb, mask, dt, dt_dev, idx, idy, P, C);
+      k_predictor_n<L, NO, 2>
+          <<<node_blocks<NodeBlock<NO, 2>::NP>(ncb, NodeBlock<NO, 2>::NW),
+             32 * NodeBlock<NO, 2>::NW, 0, st>>>(
+              qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, stiff, P, C);
       k_predictor_stiff_n<L, NO, 2><<<stiff_grid(k_predictor_stiff_n<L, NO, 2>, ncb), 32, 0,
                                       st>>>(qh, wh, ncb, mask, status, dt, dt_dev, idx, idy, P,
                                             C);
@@ -111,33 +123,33 @@ template <class L, int NO> struct OpsN {
                     const uint8_t *mask, cudaStream_t st) {
     const ConstsN<NO> &C = consts_n<NO>();
     const long n = g.nface() * (ND == 1 ? NO : NO * NO);
-    const double dy = g.nd == 2 ? dX[1] : 1.0;
+    const double ih = 1.0 / dX[dir];
     if (flux == GPR_FLUX_RUSANOV)
       k_faces_n<L, NO, ND><<<blocks(n, 128), 128, 0, st>>>(fb, qh, g.nx, g.ny, dir, mask, dt,
-                                                           dt_dev, dX[0], dy, P, C);
+                                                           dt_dev, ih, P, C);
     else
       k_faces_n<L, NO, ND, true><<<blocks(n, 64), 64, 0, st>>>(
-          fb, qh, g.nx, g.ny, dir, mask, dt, dt_dev, dX[0], dy, P, C, flux);
+          fb, qh, g.nx, g.ny, dir, mask, dt, dt_dev, ih, P, C, flux);
   }
   static int fv(double *u, const double *qh, const Grid &g, double dt, const double *dt_dev,
                 const double *dX, int flux, const DevPar &P, const uint8_t *mask, double *fb,
                 cudaStream_t st) {
     const ConstsN<NO> &C = consts_n<NO>();
     const long nf = g.nface();
-    const double dy = g.nd == 2 ? dX[1] : 1.0;
+    const double idx = 1.0 / dX[0], idy = g.nd == 2 ? 1.0 / dX[1] : 0.0;
     if (g.nd == 1) {
       using NB = NodeBlock<NO, 1>;
       faces<1>(fb, qh, g, 0, dt, dt_dev, dX, flux, P, mask, st);
-      k_cells_n<L, NO, 1><<<(unsigned)((g.nx + NB::CPB - 1) / NB::CPB), 128, 0, st>>>(
-          u, qh, fb, nullptr, g.nx, 1, mask, dt, dt_dev, dX[0], dy, P, C);
+      k_cells_n<L, NO, 1><<<node_blocks<NB::NP>(g.nx, NB::NW), 32 * NB::NW, 0, st>>>(
+          u, qh, fb, nullptr, g.nx, 1, mask, dt, dt_dev, idx, idy, P, C);
       return cuda_rc();
     }
     using NB = NodeBlock<NO, 2>;
     double *fby = fb + nf * NO * NO * 2 * V;
     for (int d = 0; d < 2; d++)
       faces<2>(d ? fby : fb, qh, g, d, dt, dt_dev, dX, flux, P, mask, st);
-    k_cells_n<L, NO, 2><<<(unsigned)((g.ncell() + NB::CPB - 1) / NB::CPB), 128, 0, st>>>(
-        u, qh, fb, fby, g.nx, g.ny, mask, dt, dt_dev, dX[0], dy, P, C);
+    k_cells_n<L, NO, 2><<<node_blocks<NB::NP>(g.ncell(), NB::NW), 32 * NB::NW, 0, st>>>(
+        u, qh, fb, fby, g.nx, g.ny, mask, dt, dt_dev, idx, idy, P, C);
     return cuda_rc();
   }
   // scratch: wh, qh, face terms

@@ -2,10 +2,9 @@
 // Gauss nodes NO (the reference's compile-time N, options.h:15), used for
 // NO = 3 (third order: degree-2 polynomials in space and time).  The N = 2
 // kernels in gpr_kernels.cuh map a cell's N^(d+1) = 4 / 8 space-time nodes
-// onto aligned lane groups and exchange values with warp shuffles; 9 or 27
-// nodes per cell do not align with a warp, so these kernels keep one thread
-// per space-time node and exchange a cell's node values through shared
-// memory.
+// onto aligned lane groups and exchange values with warp shuffles; here a warp
+// takes whole cells (one of 27 nodes, three of 9), one lane per space-time
+// node, and exchanges a cell's node values through its part of shared memory.
 //
 // Restates for general N: etc/grid.cpp:12-170 (ghost cells), weno/weno.cpp:
 // 4-124 (WENO with the central stencil of odd N, LAMC = 1e5), dg/dg1.cpp:
@@ -397,190 +396,261 @@ __global__ void k_weno2d_y_n(double *__restrict__ wh, const double *__restrict__
                    wh + (((long)i * nyp + j) * NO * NO + ii * NO) * V + k, V, j, nyp, gap, C);
 }
 
-// Node kernels: one thread per space-time node, NP = N^(d+1) per cell,
-// g = t NS + s with s = i (1D) or i N + j (2D, x-node major), NS = N^d.
+// Node kernels: one lane per node, whole cells per warp: CPW cells of PER nodes
+// (PER = NP = N^(d+1) space-time nodes, g = t NS + s with s = i (1D) or i N + j
+// (2D, x-node major), or PER = NS = N^d spatial nodes).  No barrier but the
+// warp's own, and a warp ends with its own cells.
 template <int NO, int ND> struct NodeBlock {
   static constexpr int NS = ND == 1 ? NO : NO * NO;
   static constexpr int NP = NO * NS;
-  static constexpr int CPB = 128 / NP;
-  static constexpr int THREADS = CPB * NP;
+  // warps per block: (1 + ND) V doubles per lane in 48 KB of shared memory
+  static constexpr int NW = NO == 2 && ND == 2 ? 2 : 4;
 };
+template <int PER> struct WarpCells {
+  static constexpr int CPW = 32 / PER;
+  int cell, g;   // cell within the warp and node within the cell
+  bool on;       // the lane holds a node (the spare lanes read node 0's data)
+  long c;        // the cell's index in the launch
+  GPR_D WarpCells() {
+    const int lane = threadIdx.x & 31;
+    on = lane < CPW * PER;
+    cell = on ? lane / PER : 0;
+    g = on ? lane % PER : 0;
+    c = ((long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * CPW + cell;
+  }
+  // this warp's cells in shared memory of `words` doubles per node
+  GPR_D double *nodes(double *sm, int words) const {
+    return sm + ((threadIdx.x >> 5) * CPW + cell) * (long)PER * words;
+  }
+};
+template <int PER> inline unsigned node_blocks(long ncell, int warps) {
+  const long per = (long)warps * WarpCells<PER>::CPW;
+  return (unsigned)((ncell + per - 1) / per);
+}
 
-// r = W w + dt R(q) at one space-time node (the Picard right-hand side,
-// dg1.cpp:75-89, dg2.cpp:115-150): R = W (S - B dq/dx [- B dq/dy]) - W_t
-// [W_j] DG_DER F_x / dx [- W_t W_i DG_DER F_y / dy].  The cell's node values
-// pass through sq (NP x V doubles); every thread of the block calls it (it
-// synchronises the block) and threads without a node (in_block false) read
-// zeros.
+// The system's pointwise residual at one node, scaled (as dg_residual):
+//   r = sg (S(q) - B_x dq/dx [- B_y dq/dy] - dF/dx [- dG/dy]),
+// the derivatives by DERVALS along the cell's node lines (DG_DER(i, m) is W_i
+// psi_m'(x_i), so the node weight cancels against DG_U^-1).  The cell's q, F [and
+// G] pass through sq: (1 + ND) V doubles per node, node n of the cell at sq + n
+// (1 + ND) V.  Every lane of the warp calls it; only `on` lanes write.
 template <class L, int NO, int ND>
-GPR_D void picard_rhs_n(const double *q, const double *Ww, double *r, double (*sq)[L::V],
-                        bool in_block, int g, int t, int i, int j, double wn, double dt,
-                        double idx, double idy, const DevPar &P, const ConstsN<NO> &C) {
+GPR_D void dg_residual_n(const double *q, double *r, double *sq, bool on, int g, int t, int i,
+                         int j, double sg, double idx, double idy, const DevPar &P,
+                         const ConstsN<NO> &C) {
   constexpr int V = L::V;
   constexpr int NS = NodeBlock<NO, ND>::NS;
-  // the partner node of this one with the x (y) index replaced by m
-  auto nx_of = [&](int m) { return ND == 1 ? t * NS + m : t * NS + m * NO + j; };
-  auto ny_of = [&](int m) { return t * NS + i * NO + m; };
+  constexpr int W = (1 + ND) * V;
   Prim<L::THERMAL> s;
   prim<L::THERMAL>(q, P, s);
-  // W (S - B dq/dx [- B dq/dy]) with the node weight in the source's factors
-  source<L::THERMAL, V>(q, s, P, r, wn);
-  if (in_block) {
+  source<L::THERMAL, V>(q, s, P, r, sg);
+  __syncwarp();
+  if (on) {
 #pragma unroll
     for (int k = 0; k < V; k++)
-      sq[g][k] = q[k];
+      sq[g * W + k] = q[k];
   }
-  __syncthreads();
 #pragma unroll
-  for (int dir = 0; dir < ND; dir++) {
-    const int e = dir == 0 ? i : j;
-    const double h = dir == 0 ? idx : idy;
-    double dq[V];
-#pragma unroll
-    for (int k = 0; k < V; k++) {
-      double a = 0.0;
-#pragma unroll
-      for (int m = 0; m < NO; m++)
-        a += C.derv[e][m] * (in_block ? sq[dir == 0 ? nx_of(m) : ny_of(m)][k] : 0.0);
-      dq[k] = a * h * wn;
-    }
-    double bd[V];
-    bdot<V, L::LSET>(s.v, dq, dir, bd);
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      r[k] -= bd[k];
-  }
-  // - W_t [W_j] DG_DER(i, m) F_x(t, m, j) / dx [- W_t W_i DG_DER(j, m) F_y(t, i, m) / dy]
-#pragma unroll
-  for (int dir = 0; dir < ND; dir++) {
+  for (int d = 0; d < ND; d++) {
     double F[V];
-    flux_set<L::THERMAL, V>(q, s, dir, P, F);
-    __syncthreads();
-    if (in_block) {
+    flux_set<L::THERMAL, V>(q, s, d, P, F);
+    if (on) {
 #pragma unroll
       for (int k = 0; k < V; k++)
-        sq[g][k] = F[k];
-    }
-    __syncthreads();
-    const int e = dir == 0 ? i : j;
-    const double wx = dir == 0 ? C.w[t] * (ND == 1 ? 1.0 : C.w[j]) * idx
-                               : C.w[t] * C.w[i] * idy;
-#pragma unroll
-    for (int k = 0; k < V; k++) {
-      if (!flux_support<L::THERMAL>(k, dir))
-        continue;
-      double a = 0.0;
-#pragma unroll
-      for (int m = 0; m < NO; m++)
-        a += C.dgder[e][m] * (in_block ? sq[dir == 0 ? nx_of(m) : ny_of(m)][k] : 0.0);
-      r[k] -= wx * a;
+        if (flux_support<L::THERMAL>(k, d))
+          sq[g * W + (1 + d) * V + k] = F[k];
     }
   }
+  __syncwarp();
+#pragma unroll
+  for (int d = 0; d < ND; d++) {
+    const int e = d == 0 ? i : j;
+    const double c = sg * (d == 0 ? idx : idy);
+    double a[NO];
+    const double *line[NO];  // the nodes of this one's line along d
+#pragma unroll
+    for (int m = 0; m < NO; m++) {
+      a[m] = c * C.derv[e][m];
+      line[m] = sq + (ND == 1 ? t * NS + m : (d == 0 ? t * NS + m * NO + j : t * NS + i * NO + m)) * W;
+    }
+    // - B_d dq: columns other than d of the distortion, and the level sets
+#pragma unroll
+    for (int k = 5; k < V; k++) {
+      const bool lset = k >= V - L::LSET;
+      if (!lset && (k >= 14 || (k - 5) % 3 == d))
+        continue;
+      double df = a[0] * line[0][k];
+#pragma unroll
+      for (int m = 1; m < NO; m++)
+        df = fma(a[m], line[m][k], df);
+      r[k] = fma(-s.v[d], df, r[k]);
+      if (!lset) {
+        const int col = (k - 5) % 3, dst = k - col + d;
+        r[dst] = fma(s.v[col], df, r[dst]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      if (flux_support<L::THERMAL>(k, d)) {
+#pragma unroll
+        for (int m = 0; m < NO; m++)
+          r[k] = fma(-a[m], line[m][(1 + d) * V + k], r[k]);
+      }
+  }
+}
+
+// r <- w + sum_m DG_MATinv[t][m] r(m, s), the Picard map from the residuals at
+// sg = dt W_t (as dg_solve_node), through the q part of sq.
+template <int V, int NO, int NS, int W>
+GPR_D void dg_solve_n(double *r, const double *w, double *sq, bool on, int g, int t, int sidx,
+                      const ConstsN<NO> &C) {
+  __syncwarp();
+  if (on) {
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      sq[g * W + k] = r[k];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < V; k++) {
+    double x = w[k];
+#pragma unroll
+    for (int m = 0; m < NO; m++)
+      x = fma(C.dgmatinv[t][m], sq[(m * NS + sidx) * W + k], x);
+    r[k] = x;
+  }
+}
+
+// First Picard iteration, as k_predictor_first: the initial guess is the same
+// at every time node, so its residual is evaluated once per spatial node (three
+// 2D cells to a warp) and q1 = w + DG_MATinv W r written at all of them.
+template <class L, int NO, int ND>
+__global__ void __launch_bounds__(32 * NodeBlock<NO, ND>::NW) k_predictor_first_n(
+    double *__restrict__ qh, const double *__restrict__ wh, long ncb,
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double idx,
+    double idy, DevPar P, ConstsN<NO> C) {
+  constexpr int V = L::V;
+  constexpr int NS = NodeBlock<NO, ND>::NS, NP = NodeBlock<NO, ND>::NP;
+  constexpr int W = (1 + ND) * V;
+  __shared__ double sm[NodeBlock<NO, ND>::NW * WarpCells<NS>::CPW * NS * W];
+  if (dt_dev)
+    dt = *dt_dev;
+  const WarpCells<NS> wc;
+  const bool valid = wc.on && wc.c < ncb;
+  const long cc = valid ? wc.c : 0;
+  const int i = ND == 1 ? wc.g : wc.g / NO, j = ND == 1 ? 0 : wc.g % NO;
+  double q[V], r[V];
 #pragma unroll
   for (int k = 0; k < V; k++)
-    r[k] = r[k] * dt + Ww[k];
+    q[k] = wh[(cc * NS + wc.g) * V + k];
+  dg_residual_n<L, NO, ND>(q, r, wc.nodes(sm, W), wc.on, wc.g, 0, i, j, dt, idx, idy, P, C);
+  if (!valid || !(mask == nullptr || mask[wc.c]))
+    return;
+#pragma unroll
+  for (int t = 0; t < NO; t++) {
+    double a = 0.0;
+#pragma unroll
+    for (int m = 0; m < NO; m++)
+      a = fma(C.dgmatinv[t][m], C.w[m], a);
+    double *o = qh + (wc.c * NP + t * NS + wc.g) * V;
+#pragma unroll
+    for (int k = 0; k < V; k++)
+      o[k] = fma(a, r[k], q[k]);
+  }
 }
 
 // Picard predictor (dg1.cpp:58-114, dg2.cpp:102-171): q <- DG_U^-1 (W w +
-// dt R(q)) with the reference's initial guess q(t, s) = w(s), per-cell
-// stopping rule |q1 - q0| <= dg_tol (1 + |q0|) and iteration cap (none with
-// STIFF: every cell goes to the Newton pass).  The cell's node values pass
-// through shared memory.  status[c]: GPR_PRED_PICARD | iterations << 8 when
-// converged; a cell that does not converge within the cap, or whose
-// iterate turns NaN, gets the initial guess with a NaN marker in its first
-// entry (0x7ff8000000000bad) and GPR_PRED_FAILED | iterations << 8, and
-// k_predictor_stiff_n finishes it (the reference leaves such rows unwritten
+// dt R(q)) with the reference's initial guess q(t, s) = w(s) (its first iterate
+// from k_predictor_first_n), per-cell stopping rule |q1 - q0| <= dg_tol (1 +
+// |q0|), decided as in k_predictor_picard, and iteration cap (none with
+// STIFF: every cell goes to the Newton pass).  status[c]: GPR_PRED_PICARD |
+// iterations << 8 when converged; a cell that does not converge within the
+// cap, or whose iterate turns NaN, gets the initial guess with a NaN marker in
+// its first entry (0x7ff8000000000bad) and GPR_PRED_FAILED | iterations << 8,
+// and k_predictor_stiff_n finishes it (the reference leaves such rows unwritten
 // or calls its Newton-Krylov solver).
 template <class L, int NO, int ND>
-__global__ void __launch_bounds__(128) k_predictor_n(
+__global__ void __launch_bounds__(32 * NodeBlock<NO, ND>::NW) k_predictor_n(
     double *__restrict__ qh, const double *__restrict__ wh, long ncb,
     const uint8_t *__restrict__ mask, int32_t *__restrict__ status, double dt,
     const double *__restrict__ dt_dev, double idx, double idy, int stiff, DevPar P,
     ConstsN<NO> C) {
   constexpr int V = L::V;
-  using NB = NodeBlock<NO, ND>;
-  constexpr int NS = NB::NS, NP = NB::NP, CPB = NB::CPB;
-  __shared__ double sq[CPB][NP][V];
-  __shared__ int cflag[CPB];
+  constexpr int NS = NodeBlock<NO, ND>::NS, NP = NodeBlock<NO, ND>::NP;
+  constexpr int W = (1 + ND) * V;
+  __shared__ double sm[NodeBlock<NO, ND>::NW * WarpCells<NP>::CPW * NP * W];
   if (dt_dev)
     dt = *dt_dev;
-  const int lc = threadIdx.x / NP;  // cell within the block
-  const int g = threadIdx.x % NP;
-  const bool in_block = threadIdx.x < NB::THREADS;
-  const long c = (long)blockIdx.x * CPB + lc;
-  const bool valid = in_block && c < ncb;
+  const WarpCells<NP> wc;
+  const long c = wc.c;
+  const bool valid = wc.on && c < ncb;
   const bool active = valid && (mask == nullptr || mask[c]);
-  const int t = g / NS, sidx = g % NS;
+  const int g = wc.g, t = g / NS, sidx = g % NS;
   const int i = ND == 1 ? sidx : sidx / NO, j = ND == 1 ? 0 : sidx % NO;
   const long cc = valid ? c : 0;  // lanes without a cell read cell 0's data
-  double w[V], Ww[V], q[V], r[V], qn[V];
-  const double *wc = wh + (cc * NS + (in_block ? sidx : 0)) * V;
-  const double ws = ND == 1 ? C.w[i] : C.w[i] * C.w[j];
-  const double f = C.endv[0][t] * ws;
+  double *sq = wc.nodes(sm, W);
+  // the lanes of this lane's cell
+  const unsigned gmask = (NP >= 32 ? 0xffffffffu : ((1u << NP) - 1u)) << (wc.cell * NP);
+  double w[V], q[V], qn[V];
 #pragma unroll
   for (int k = 0; k < V; k++) {
-    w[k] = wc[k];
-    Ww[k] = f * w[k];
+    w[k] = wh[(cc * NS + sidx) * V + k];
     q[k] = w[k];
   }
   bool done = !active, nan_seen = false;
   int iters = 0;
-  const double wn = C.w[t] * ws;
-  double(*sqc)[V] = sq[in_block ? lc : 0];
+  const double sg = dt * C.w[t];
+  const float tolf = (float)C.dg_tol;
   const int maxit = stiff ? 0 : C.dg_it;
   for (int it = 0; it < maxit; it++) {
-    if (!__syncthreads_or(!done))
+    if (__all_sync(0xffffffffu, done))
       break;
-    picard_rhs_n<L, NO, ND>(q, Ww, r, sqc, in_block, g, t, i, j, wn, dt, idx, idy, P, C);
-    __syncthreads();
-    if (in_block) {
+    if (it == 0) {
+      const double *src = qh + (cc * NP + g) * V;
 #pragma unroll
       for (int k = 0; k < V; k++)
-        sq[lc][g][k] = r[k];
+        qn[k] = active ? src[k] : q[k];
+    } else {
+      dg_residual_n<L, NO, ND>(q, qn, sq, wc.on, g, t, i, j, sg, idx, idy, P, C);
+      dg_solve_n<V, NO, NS, W>(qn, w, sq, wc.on, g, t, sidx, C);
     }
-    if (in_block && g == 0)
-      cflag[lc] = 0;
-    __syncthreads();
-    // q_new(t, s) = sum_m DG_MATinv[t][m] r(m, s) / W_s
-    const double iw = 1.0 / ws;
+    bool big = false, open = false, hasnan = false;
 #pragma unroll
     for (int k = 0; k < V; k++) {
-      double a = 0.0;
-#pragma unroll
-      for (int m = 0; m < NO; m++)
-        a += C.dgmatinv[t][m] * (in_block ? sq[lc][m * NS + sidx][k] : 0.0);
-      qn[k] = a * iw;
+      const float df = f32_abs_hi(qn[k] - q[k]), qf = f32_abs_hi(q[k]);
+      const float th = fmaf(tolf, qf, tolf);
+      const bool ok = fmaxf(df, qf) < F32_TOP;
+      big = big || (ok && df > th * 1.00001f);
+      open = open || !ok || df > th * 0.99999f;
     }
-    bool big = false, hasnan = false;
+    unsigned bigm = __ballot_sync(0xffffffffu, wc.on && big) & gmask;
+    if (open && !bigm) {
 #pragma unroll
-    for (int k = 0; k < V; k++) {
-      if (fabs(qn[k] - q[k]) > C.dg_tol * (1.0 + fabs(q[k])))
-        big = true;
-      if (qn[k] != qn[k])
-        hasnan = true;
+      for (int k = 0; k < V; k++) {
+        if (fabs(qn[k] - q[k]) > C.dg_tol * (1.0 + fabs(q[k])))
+          big = true;
+        if (fp_abs_bits(qn[k]) > FP_INF_BITS)
+          hasnan = true;
+      }
     }
-    if (in_block && !done && (big || hasnan))
-      atomicOr(&cflag[lc], (big ? 1 : 0) | (hasnan ? 2 : 0));
-    __syncthreads();
+    bigm = __ballot_sync(0xffffffffu, wc.on && big) & gmask;
+    const unsigned nanm = __ballot_sync(0xffffffffu, wc.on && hasnan) & gmask;
     if (!done) {
-      const int fl = cflag[lc];
       iters = it + 1;
 #pragma unroll
       for (int k = 0; k < V; k++)
         q[k] = qn[k];
-      if (fl & 1) {
-        // not converged: iterate on
-      } else if (fl & 2) {
-        nan_seen = true;
+      if (!bigm) {
         done = true;
-      } else {
-        done = true;
-        double *out = qh + (c * NP + g) * V;
+        nan_seen = nanm != 0;
+        if (!nan_seen) {
+          double *out = qh + (c * NP + g) * V;
 #pragma unroll
-        for (int k = 0; k < V; k++)
-          out[k] = q[k];
-        if (status && g == 0)
-          status[c] = GPR_PRED_PICARD | (iters << 8);
+          for (int k = 0; k < V; k++)
+            out[k] = q[k];
+          if (status && g == 0)
+            status[c] = GPR_PRED_PICARD | (iters << 8);
+        }
       }
     }
   }
@@ -627,7 +697,8 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
   using SN = StiffN<L, NO, ND>;
   constexpr int NS = SN::NS, NP = SN::NP, NA = SN::NA, NJ = SN::NJ;
   static_assert(NP <= 32, "one cell per warp");
-  __shared__ double sq[NP][V];
+  constexpr int W = (1 + ND) * V;
+  __shared__ double sq[NP * W];
   __shared__ float sm[NS * SN::per_node];
   if (dt_dev)
     dt = *dt_dev;
@@ -636,9 +707,7 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
   const int g = in_block ? lane : 0;
   const int t = g / NS, sidx = g % NS;
   const int i = ND == 1 ? sidx : sidx / NO, j = ND == 1 ? 0 : sidx % NO;
-  const double ws = ND == 1 ? C.w[i] : C.w[i] * C.w[j];
-  const double f = C.endv[0][t] * ws;
-  const double wn = C.w[t] * ws;
+  const double f = C.endv[0][t];
   const double a_t = dt * C.w[t];
   float *Am = sm + sidx * SN::per_node;  // (9 NO) x (9 NO)
   float *Ab = Am + NA * NA;              // 9 NO
@@ -655,35 +724,30 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
     while (todo) {  // uniform over the block (one warp)
       const long c = base + __ffs(todo) - 1;
       todo &= todo - 1;
-      double Ww[V], q[V], r[V], delta[V];
+      double fw[V], q[V], r[V], delta[V];
       const double *wc = wh + (c * NS + sidx) * V;
 #pragma unroll
       for (int k = 0; k < V; k++) {
         const double w = wc[k];
-        Ww[k] = f * w;
+        fw[k] = f * w;
         q[k] = w;
       }
       bool ok = false;
       int iters = 0;
       for (int it = 0; it < C.stiff_it; it++) {
         __syncthreads();  // the previous iteration's reads of sq and sm are done
-        picard_rhs_n<L, NO, ND>(q, Ww, r, sq, in_block, g, t, i, j, wn, dt, idx, idy, P, C);
-        // residual r - W_s sum_m DG_MAT[t][m] q(m, s)
-        __syncthreads();
-        if (in_block) {
-#pragma unroll
-          for (int k = 0; k < V; k++)
-            sq[g][k] = q[k];
-        }
-        __syncthreads();
+        dg_residual_n<L, NO, ND>(q, r, sq, in_block, g, t, i, j, a_t, idx, idy, P, C);
+        // the fixed point's residual over W_s: r + ENDVALS[0][t] w - sum_m
+        // DG_MAT[t][m] q(m, s) (sq still holds q)
 #pragma unroll
         for (int k = 0; k < V; k++) {
-          double uq = 0.0;
+          double x = r[k] + fw[k];
 #pragma unroll
           for (int m = 0; m < NO; m++)
-            uq += C.dgmat[t][m] * sq[m * NS + sidx][k];
-          r[k] -= ws * uq;
+            x = fma(-C.dgmat[t][m], sq[(m * NS + sidx) * W + k], x);
+          r[k] = x;
         }
+        __syncthreads();
         if (in_block) {
           // this time node's rows of the two systems: the diagonal block
           // DG_MAT[t][t] I - dt W_t dS/dq, the others DG_MAT[t][t2] I
@@ -711,11 +775,11 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
           }
 #pragma unroll
           for (int a = 0; a < 9; a++)
-            Ab[t * 9 + a] = (float)(r[5 + a] / ws);
+            Ab[t * 9 + a] = (float)r[5 + a];
           if (L::THERMAL) {
 #pragma unroll
             for (int a = 0; a < 3; a++)
-              Jb[t * 3 + a] = (float)(r[14 + a] / ws);
+              Jb[t * 3 + a] = (float)r[14 + a];
           }
         }
         __syncthreads();
@@ -724,11 +788,11 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
           solved = smem_solve<NA>(Am, NA, Ab);
         else if (L::THERMAL && in_block && t == 1)
           solved = smem_solve<NJ>(Jm, NJ, Jb);
-        // the other variables: DG_MAT^-1 of the residual, / W_s
+        // the other variables: DG_MAT^-1 of the residual
         if (in_block) {
 #pragma unroll
           for (int k = 0; k < V; k++)
-            sq[g][k] = r[k];
+            sq[g * W + k] = r[k];
         }
         __syncthreads();
 #pragma unroll
@@ -736,8 +800,8 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
           double acc = 0.0;
 #pragma unroll
           for (int m = 0; m < NO; m++)
-            acc += C.dgmatinv[t][m] * sq[m * NS + sidx][k];
-          delta[k] = acc / ws;
+            acc += C.dgmatinv[t][m] * sq[(m * NS + sidx) * W + k];
+          delta[k] = acc;
         }
 #pragma unroll
         for (int a = 0; a < 9; a++)
@@ -812,13 +876,13 @@ GPR_D void interface_point_n(const double *ql, const double *qr, int d, const De
 // predictor cells (i, j) and (i + 1, j) (dir 0) or (i, j + 1) (dir 1), p = t
 // N + s over time node t and transverse node s.  fb[face][p][0][V] = k (b +
 // f) is subtracted from the left cell, fb[face][p][1][V] = k (b - f) from the
-// right one, k = W_t [W_s] dt / (2 dx_dir).  EIG: the Roe or Osher
+// right one, k = W_t [W_s] dt / (2 dx_dir), ih = 1 / dx_dir.  EIG: the Roe or Osher
 // dissipation (flux), one thread per face point as for Rusanov.
 template <class L, int NO, int ND, bool EIG = false>
 __global__ void __launch_bounds__(128) k_faces_n(
     double *__restrict__ fb, const double *__restrict__ qh, int nx, int ny, int dir,
-    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double dx,
-    double dy, DevPar P, ConstsN<NO> C, int flux = 0) {
+    const uint8_t *__restrict__ mask, double dt, const double *__restrict__ dt_dev, double ih,
+    DevPar P, ConstsN<NO> C, int flux = 0) {
   constexpr int V = L::V;
   constexpr int NQ = ND == 1 ? NO : NO * NO;  // points per face
   constexpr int NS = ND == 1 ? NO : NO * NO;
@@ -868,7 +932,7 @@ __global__ void __launch_bounds__(128) k_faces_n(
     qr[k] = e;
   }
   interface_point_n<L, NO, EIG>(ql, qr, dir, P, C, f, b, flux);
-  const double kk = dt * C.w[t] * (ND == 1 ? 1.0 : C.w[sq]) / (2.0 * (dir == 0 ? dx : dy));
+  const double kk = dt * C.w[t] * (ND == 1 ? 1.0 : C.w[sq]) * (0.5 * ih);
 #pragma unroll
   for (int k = 0; k < V; k++) {
     o[k] = kk * (b[k] + f[k]);
@@ -883,75 +947,76 @@ __global__ void __launch_bounds__(128) k_faces_n(
 // face c + 1 (left part); 2D: the x faces (ci + 1, cj + 1) and (ci, cj + 1),
 // the y faces (ci + 1, cj + 1) and (ci + 1, cj)), each summed over its points.
 template <class L, int NO, int ND>
-__global__ void __launch_bounds__(128) k_cells_n(
+__global__ void __launch_bounds__(32 * NodeBlock<NO, ND>::NW) k_cells_n(
     double *__restrict__ u, const double *__restrict__ qh, const double *__restrict__ fbx,
     const double *__restrict__ fby, int nx, int ny, const uint8_t *__restrict__ mask, double dt,
-    const double *__restrict__ dt_dev, double dx, double dy, DevPar P, ConstsN<NO> C) {
+    const double *__restrict__ dt_dev, double idx, double idy, DevPar P, ConstsN<NO> C) {
   constexpr int V = L::V;
-  using NB = NodeBlock<NO, ND>;
-  constexpr int NS = NB::NS, NP = NB::NP, CPB = NB::CPB;
+  constexpr int NS = NodeBlock<NO, ND>::NS, NP = NodeBlock<NO, ND>::NP;
   constexpr int NQ = NS;  // points per face
-  __shared__ double sq[CPB][NP][V];
+  __shared__ double sm[NodeBlock<NO, ND>::NW * WarpCells<NP>::CPW * NP * V];
   if (dt_dev)
     dt = *dt_dev;
-  const int lc = threadIdx.x / NP;
-  const int g = threadIdx.x % NP;
-  const bool in_block = threadIdx.x < NB::THREADS;
+  const WarpCells<NP> wc;
   const long ncell = ND == 1 ? nx : (long)nx * ny;
-  const long c = (long)blockIdx.x * CPB + lc;
-  const bool valid = in_block && c < ncell;
+  const long c = wc.c;
+  const bool valid = wc.on && c < ncell;
   const long cc = valid ? c : 0;  // lanes without a cell read cell 0's nodes
   const long ci = ND == 1 ? cc : cc / ny;
   const int cj = ND == 1 ? 0 : (int)(cc % ny);
   const long cb = ND == 1 ? ci + 1 : (ci + 1) * (ny + 2) + (cj + 1);
   const bool active = valid && (mask == nullptr || mask[cb]);
-  const int t = g / NS, sidx = g % NS;
+  const int g = wc.g, t = g / NS, sidx = g % NS;
   const int i = ND == 1 ? sidx : sidx / NO, j = ND == 1 ? 0 : sidx % NO;
-  const double idx = 1.0 / dx, idy = 1.0 / dy;
+  double *sq = wc.nodes(sm, V);
   double q[V], acc[V];
-  const double *qc = qh + (cb * NP + (in_block ? g : 0)) * V;
 #pragma unroll
   for (int k = 0; k < V; k++)
-    q[k] = qc[k];
-  if (in_block) {
+    q[k] = qh[(cb * NP + g) * V + k];
+  if (wc.on) {
 #pragma unroll
     for (int k = 0; k < V; k++)
-      sq[lc][g][k] = q[k];
+      sq[g * V + k] = q[k];
   }
-  __syncthreads();
+  __syncwarp();
   Prim<L::THERMAL> s;
   prim<L::THERMAL>(q, P, s);
   const double wn = dt * C.w[t] * C.w[i] * (ND == 1 ? 1.0 : C.w[j]);
   source<L::THERMAL, V>(q, s, P, acc, wn);
 #pragma unroll
-  for (int dir = 0; dir < ND; dir++) {
-    const int e = dir == 0 ? i : j;
-    const double h = dir == 0 ? idx : idy;
-    double dq[V];
+  for (int d = 0; d < ND; d++) {
+    const int e = d == 0 ? i : j;
+    const double h = wn * (d == 0 ? idx : idy);
+    double a[NO];
+    const double *line[NO];
 #pragma unroll
-    for (int k = 0; k < V; k++) {
-      double a = 0.0;
-#pragma unroll
-      for (int m = 0; m < NO; m++) {
-        const int node = ND == 1 ? t * NS + m
-                                 : (dir == 0 ? t * NS + m * NO + j : t * NS + i * NO + m);
-        a += C.derv[e][m] * (in_block ? sq[lc][node][k] : 0.0);
-      }
-      dq[k] = a * h * wn;
+    for (int m = 0; m < NO; m++) {
+      a[m] = h * C.derv[e][m];
+      line[m] = sq + (ND == 1 ? t * NS + m : (d == 0 ? t * NS + m * NO + j : t * NS + i * NO + m)) * V;
     }
-    double bd[V];
-    bdot<V, L::LSET>(s.v, dq, dir, bd);
+#pragma unroll
+    for (int k = 5; k < V; k++) {
+      const bool lset = k >= V - L::LSET;
+      if (!lset && (k >= 14 || (k - 5) % 3 == d))
+        continue;
+      double df = a[0] * line[0][k];
+#pragma unroll
+      for (int m = 1; m < NO; m++)
+        df = fma(a[m], line[m][k], df);
+      acc[k] = fma(-s.v[d], df, acc[k]);
+      if (!lset) {
+        const int col = (k - 5) % 3, dst = k - col + d;
+        acc[dst] = fma(s.v[col], df, acc[dst]);
+      }
+    }
+  }
+  __syncwarp();
+  if (wc.on) {
 #pragma unroll
     for (int k = 0; k < V; k++)
-      acc[k] -= bd[k];
+      sq[g * V + k] = acc[k];
   }
-  __syncthreads();
-  if (in_block) {
-#pragma unroll
-    for (int k = 0; k < V; k++)
-      sq[lc][g][k] = acc[k];
-  }
-  __syncthreads();
+  __syncwarp();
   if (!active)
     return;
   double *uc = u + c * V;
@@ -964,7 +1029,7 @@ __global__ void __launch_bounds__(128) k_cells_n(
       double x = 0.0;
 #pragma unroll
       for (int n = 0; n < NP; n++)
-        x += sq[lc][n][k];
+        x += sq[n * V + k];
       x += uc[k];
 #pragma unroll
       for (int p = 0; p < NQ; p++) {
@@ -982,7 +1047,7 @@ __global__ void __launch_bounds__(128) k_cells_n(
       double x = 0.0;
 #pragma unroll
       for (int n = 0; n < NP; n++)
-        x += sq[lc][n][k];
+        x += sq[n * V + k];
       x += uc[k];
 #pragma unroll
       for (int p = 0; p < NQ; p++) {
