@@ -91,30 +91,35 @@ template <class L> struct Adj {
     }
     DevPar P0{};
     double *mcell = tape ? tape + tl.o_mcell : nullptr;
-    k_b_cfl_max<L><<<blocks(b.nu, 256), 256, 0, st>>>(u, b.nu, mx, B, mcell);
+    // every launch shaped by spread(): a few hundred cells are some tens of
+    // warps, each a serial FP64 chain that runs best on an SM of its own
+    k_b_cfl_max<L><<<GPR_SPREAD(b.nu, 256), 0, st>>>(u, b.nu, mx, B, mcell);
     if (tape)
-      k_adj_argmax<<<blocks(b.nu, 256), 256, 0, st>>>(mcell, b.nu, mx, amax, B);
+      k_adj_argmax<<<GPR_SPREAD(b.nu, 256), 0, st>>>(mcell, b.nu, mx, amax, B);
     k_adj_clock_finalize<<<blocks(ninst, 128), 128, 0, st>>>(mx, B, dt_io, dt_mode, tclk, aux,
                                                              amax);
-    k_b_boundaries<V><<<blocks(b.nub * V, 256), 256, 0, st>>>(u, ub, b.nub, B);
-    k_b_weno<V><<<blocks(b.nb * V, 256), 256, 0, st>>>(wh, ub, b.nb, C, B);
+    k_b_boundaries<V><<<GPR_SPREAD(b.nub * V, 256), 0, st>>>(u, ub, b.nub, B);
+    k_b_weno<V><<<GPR_SPREAD(b.nb * V, 256), 0, st>>>(wh, ub, b.nb, C, B);
     // every iteration in the Picard kernel (no k_predictor_first): the
     // tightly converged forward the gradients and their finite-difference
     // checks difference keeps one arithmetic path
-    k_predictor_picard<L, 1, true><<<blocks(b.nb * NN * NN, 128), 128, 0, st>>>(
+    k_predictor_picard<L, 1, true><<<GPR_SPREAD(b.nb * NN * NN, 128), 0, st>>>(
         qh, wh, b.nb, nullptr, status, 0.0, nullptr, 1.0, 1.0, 0, P0, C, B, 0);
     int rc = launch_stiff<L, 1, true>(qh, wh, b.nb, nullptr, status, 0.0, nullptr, 1.0, 1.0, P0,
                                       C, st, B);
     if (rc)
       return rc;
-    k_faces1d<L, true><<<blocks(b.nf * NN, 128), 128, 0, st>>>(fb, qh, b.nf, nullptr, 0.0,
-                                                                nullptr, 1.0, 1, P0, C, B);
-    k_cells<L, 1, true><<<blocks(b.nu * NN * NN, 128), 128, 0, st>>>(
+    // two lanes to a quadrature point, each with one side's chain (400 cells: 37
+    // us with one lane to a point); one layout whatever the batch, so that an
+    // instance's result does not depend on its company
+    k_faces1d_split<L, true><<<GPR_SPREAD(b.nf * NN * 2, 128), 0, st>>>(
+        fb, qh, b.nf, nullptr, 0.0, nullptr, 1.0, 1, P0, C, B);
+    k_cells<L, 1, true><<<GPR_SPREAD(b.nu * NN * NN, 128), 0, st>>>(
         u, qh, fb, nullptr, b.nu, 1, nullptr, 0.0, nullptr, 1.0, 1.0, 1, 1, P0, C, B, FV_BOTH);
     if (tape && cudaMemcpyAsync(tape + tl.o_up, u, sizeof(double) * b.nu * V,
                                 cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return GPR_E_CUDA;
-    k_b_renorm<V><<<blocks(b.nu, 256), 256, 0, st>>>(u, b.nu, B);
+    k_b_renorm<V><<<GPR_SPREAD(b.nu, 256), 0, st>>>(u, b.nu, B);
     k_b_clock_advance<<<blocks(ninst, 128), 128, 0, st>>>(B, nullptr);
     return cuda_rc();
   }
@@ -136,8 +141,8 @@ template <class L> struct Adj {
            *thf = ascr + al.o_thf, *thp = ascr + al.o_thp, *dtf = ascr + al.o_dtf,
            *dtp = ascr + al.o_dtp, *mu = ascr + al.o_mu;
     int32_t *need = (int32_t *)(ascr + al.o_need);
-    k_adj_renorm<V><<<blocks(b.nu, 256), 256, 0, st>>>(ubar, up, b.nu, B);
-    k_adj_eig<L><<<blocks(b.nb * 4 + ninst, 128), 128, 0, st>>>(qh, b.nb, un, aux, EV, EIG, C,
+    k_adj_renorm<V><<<GPR_SPREAD(b.nu, 256), 0, st>>>(ubar, up, b.nu, B);
+    k_adj_eig<L><<<GPR_SPREAD(b.nb * 4 + ninst, 128), 0, st>>>(qh, b.nb, un, aux, EV, EIG, C,
                                                                   B);
     k_adj_fv<L><<<blocks(b.nb * 2, ADJ_FV_PAIRS), 4 * ADJ_FV_PAIRS, 0, st>>>(
         ubar, qh, EV, EIG, un, up, b.nb, qb, thf, dtf, C, B);
@@ -149,9 +154,9 @@ template <class L> struct Adj {
                              (int)dsmem) != cudaSuccess)
       return GPR_E_CUDA;
     k_adj_pred_dense<L><<<(unsigned)b.nb, 128, dsmem, st>>>(qh, qb, b.nb, need, mu, info, C, B);
-    k_adj_pred_post<L><<<blocks(b.nb * 4, 128), 128, 0, st>>>(qh, mu, b.nb, wb, thp, dtp, C, B);
-    k_adj_weno<V><<<blocks(b.nb * V, 256), 256, 0, st>>>(wb, un, b.nb, g, C, B);
-    k_adj_gather<V><<<blocks(b.nu * V, 256), 256, 0, st>>>(ubar, g, b.nu, B);
+    k_adj_pred_post<L><<<GPR_SPREAD(b.nb * 4, 128), 0, st>>>(qh, mu, b.nb, wb, thp, dtp, C, B);
+    k_adj_weno<V><<<GPR_SPREAD(b.nb * V, 256), 0, st>>>(wb, un, b.nb, g, C, B);
+    k_adj_gather<V><<<GPR_SPREAD(b.nu * V, 256), 0, st>>>(ubar, g, b.nu, B);
     k_adj_reduce<L><<<ninst, 128, 0, st>>>(ubar, thbar, tbar, thf, thp, dtf, dtp, un, aux, EVs,
                                            EIGs, frozen, B);
     return cuda_rc();

@@ -1300,17 +1300,18 @@ GPR_D void faces1d_split_body(double *__restrict__ fb, const double *__restrict_
   }
   bool active = valid && (mask == nullptr || (mask[fi] && mask[fi + 1])) && (time_dg || t == 0);
   int nt = time_dg ? NN : 1;
-  double ql[V], qr[V], f[V], b[V], dq[V];
-  const double *ql_ = qh + (fi * nt + (time_dg ? t : 0)) * NN * V;
-  const double *qr_ = qh + ((fi + 1) * nt + (time_dg ? t : 0)) * NN * V;
+  // each lane extrapolates its own side and takes the other from its partner
+  double qs[V], ql[V], f[V], b[V], dq[V];
+  const double *qs_ = qh + ((fi + side) * nt + (time_dg ? t : 0)) * NN * V;
+  const double e0 = C.endv[1 - side][0], e1 = C.endv[1 - side][1];
 #pragma unroll
   for (int k = 0; k < V; k++) {
-    ql[k] = C.endv[1][0] * ql_[k] + C.endv[1][1] * ql_[V + k];
-    qr[k] = C.endv[0][0] * qr_[k] + C.endv[0][1] * qr_[V + k];
-    dq[k] = qr[k] - ql[k];
+    qs[k] = e0 * qs_[k] + e1 * qs_[V + k];
+    const double o = __shfl_xor_sync(0xffffffffu, qs[k], 1);
+    ql[k] = side ? o : qs[k];
+    dq[k] = (side ? qs[k] : o) - ql[k];
   }
   const double kk = dt * idx * (time_dg ? 0.5 * GAUSS_W : 0.5);
-  const double *qs = side ? qr : ql;
   Prim<L::THERMAL> ps;
   prim<L::THERMAL>(qs, P, ps);
   const double lam = max_abs_eigs<L::THERMAL>(qs, ps, 0, P);

@@ -616,7 +616,7 @@ template <class L> struct Ops {
   // The stages of one batched step with the launch shapes sh.
   static void batch_cfl(double *u, unsigned long long *mx, const BatchLayout &b, const Batch &B,
                         int ninst, cudaStream_t st) {
-    k_b_cfl_max<L><<<blocks(b.nu, 256), 256, 0, st>>>(u, b.nu, mx, B);
+    k_b_cfl_max<L><<<GPR_SPREAD(b.nu, 256), 0, st>>>(u, b.nu, mx, B);
     k_b_clock_finalize<<<blocks(ninst, 128), 128, 0, st>>>(mx, B);
   }
   static void batch_weno(double *wh, const double *ub, const BatchLayout &b, const Batch &B,
@@ -686,7 +686,7 @@ template <class L> struct Ops {
         return rc;
       batch_faces(fb, qh, b, B, sh.faces_split, sh.faces, st);
       batch_cells(u, qh, fb, b, B, sh.cells, st);
-      k_b_renorm<V><<<blocks(b.nu, 256), 256, 0, st>>>(u, b.nu, B);
+      k_b_renorm<V><<<GPR_SPREAD(b.nu, 256), 0, st>>>(u, b.nu, B);
       k_b_clock_advance<<<blocks(ninst, 128), 128, 0, st>>>(B, updates);
     }
     return cuda_rc();

@@ -2049,13 +2049,17 @@ __global__ void __launch_bounds__(128) k_faces1d_osher(
   const bool on = valid && (mask == nullptr || (mask[fi] && mask[fi + 1]));
   const bool active = on && (time_dg || t == 0);
   const int nt = time_dg ? NN : 1, tt = time_dg ? t : 0;
-  const double *ql_ = qh + (fi * nt + tt) * NN * V, *qr_ = qh + ((fi + 1) * nt + tt) * NN * V;
-  double ql[V], qr[V], dq[V], f[V], b[V];
+  // each lane extrapolates its own side and takes the other from its partner
+  const double *qs_ = qh + ((fi + side) * nt + tt) * NN * V;
+  const double e0 = C.endv[1 - side][0], e1 = C.endv[1 - side][1];
+  double qs[V], ql[V], qr[V], dq[V], f[V], b[V];
   bool flat = true;
 #pragma unroll
   for (int k = 0; k < V; k++) {
-    ql[k] = C.endv[1][0] * ql_[k] + C.endv[1][1] * ql_[V + k];
-    qr[k] = C.endv[0][0] * qr_[k] + C.endv[0][1] * qr_[V + k];
+    qs[k] = e0 * qs_[k] + e1 * qs_[V + k];
+    const double o = __shfl_xor_sync(0xffffffffu, qs[k], 1);
+    ql[k] = side ? o : qs[k];
+    qr[k] = side ? qs[k] : o;
     dq[k] = ql[k] - qr[k];
     f[k] = 0.0;
     flat = flat && (__double_as_longlong(dq[k]) << 1) == 0;
@@ -2070,12 +2074,9 @@ __global__ void __launch_bounds__(128) k_faces1d_osher(
     ok = abs_apply_acoustic<L>(q, dq, GAUSS_W, P, f);
   }
   {
-    double qs[V];
 #pragma unroll
-    for (int k = 0; k < V; k++) {
-      qs[k] = side ? qr[k] : ql[k];
+    for (int k = 0; k < V; k++)
       dq[k] = -dq[k];
-    }
     Prim<L::THERMAL> s;
     prim<L::THERMAL>(qs, P, s);
     flux_add<L::THERMAL, V>(qs, s, 0, P, f);

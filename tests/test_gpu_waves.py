@@ -9,9 +9,15 @@ largest eigenvalue is determined to a few roundings: 1e-13.  Along y and z
 the reference's tensor is not symmetric (its pressure and density entries
 stay in row and column 0) and an eigenvalue moves by the rounding times
 about c0^2 / cs^2 and the inverse relative gap: 1e-11 for distortions up to
-1e-3, where the dominant root is real and separated.  The oracle's Osher
-dissipation carries its 17 x 17 eigenvectors' conditioning, about 1e3
-roundings at these scales: 1e-11 of the largest flux entry."""
+1e-3, where the dominant root is real and separated.  A 17 x 17
+eigen-decomposition carries its eigenvectors' conditioning, about 1e3
+roundings at these scales: 1e-11 of the largest flux entry.  Two are compared
+with, along x on states with the axes exchanged (the system is invariant), and
+each state is held to the nearer: the oracle's, and numpy's of the balanced
+system matrix.  Either can lose more where eigenvalues coincide (against 40
+digits: the oracle's 2e-11 in the fast smg flow and 1e-3 along z at an
+isotropic distortion, numpy's 7e-11 in a fluid at rest; the closed form
+stays within 1e-12)."""
 import numpy as np
 import pytest
 import torch
@@ -90,16 +96,16 @@ def _exchange(V, d):
 
 def _osher(O, ql, qr, MP):
     """D_OSH along x: two Gauss nodes of |M| (qL - qR), plus both fluxes, by
-    numpy's decomposition of the balanced system matrix; the oracle's where its
-    eigenvectors lose close to three digits (fluid at rest, slow heat wave)."""
+    numpy's decomposition of the balanced system matrix (None where it has no
+    eigenvector basis)."""
     f = O.flux(ql, 0, MP) + O.flux(qr, 0, MP)
     dq = ql - qr
     for x in (0.5 - 0.5 / np.sqrt(3), 0.5 + 0.5 / np.sqrt(3)):
         M, (D, _) = matrix_balance(O.system_matrix(qr + x * dq, 0, MP), permute=False,
                                    separate=True)
         lam, R = np.linalg.eig(M)
-        if np.linalg.cond(R) > 500.0:
-            return O.D(2, ql, qr, 0, MP)
+        if not np.linalg.cond(R) <= 1e6:
+            return None
         f = f + 0.5 * D * (R @ (np.abs(lam) * np.linalg.solve(R, dq / D + 0j))).real
     return f
 
@@ -120,10 +126,11 @@ def test_osher_closed_form(V, name, amp, jump, mach):
         got = G.solvers.fv.D_OSH(torch.tensor(QL, device=DEV), torch.tensor(QR, device=DEV), d,
                                  MP).cpu().numpy()
         ix = _exchange(V, d)
-        ref = np.array([_osher(O, QL[i, ix].copy(), QR[i, ix].copy(), MP)[ix]
-                        for i in range(len(QL))])
-        scale = np.max(np.abs(ref), axis=1, keepdims=True)
-        assert np.max(np.abs(got - ref) / scale) < 1e-11, d
+        for i in range(len(QL)):
+            ql, qr = QL[i, ix].copy(), QR[i, ix].copy()
+            refs = [r for r in (_osher(O, ql, qr, MP), O.D(2, ql, qr, 0, MP)) if r is not None]
+            err = min(np.max(np.abs(got[i, ix] - r)) / np.max(np.abs(r)) for r in refs)
+            assert err < 1e-11, (d, i, err)
 
 
 @pytest.mark.parametrize("flux", [1, 2])
