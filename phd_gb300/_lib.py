@@ -14,7 +14,8 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgpr_gb300.so")
 SOURCES = ["gpr_capi.cu", "gpr_adjoint.cu", "gpr_multi.cu", "gpr_order.cu"]
-HEADERS = ["gpr_fastmath.cuh", "gpr_device.cuh", "gpr_kernels.cuh", "gpr_consts.cuh", "gpr_ode.cuh",
+HEADERS = ["gpr_fastmath.cuh", "gpr_device.cuh", "gpr_jacobi.cuh", "gpr_kernels.cuh",
+           "gpr_consts.cuh", "gpr_ode.cuh",
            "gpr_host.cuh", "gpr_osher.cuh", "gpr_ops.cuh", "gpr_ops15.h", "gpr_multi.cuh",
            "gpr_adjoint.cuh", "gpr_order.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

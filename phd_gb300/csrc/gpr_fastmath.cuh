@@ -75,11 +75,11 @@ static __device__ __noinline__ double pow53_general(double x) {
   const double cb = cbrt(x);
   return x * cb * cb;
 }
-GPR_D double pow53(double x) {
+// The start y ~ |x|^(-1/3) and the step's correction: |x|^(-1/3) = y + y p.
+// The exponent of x is within 300 of 0.
+GPR_D double icbrt_start(double x, double &p) {
   const int hi = __double2hiint(x);
   const int ex = (hi >> 20) & 0x7ff;
-  if ((unsigned)(ex - 723) >= 600u)
-    return pow53_general(x);
   const int k = (ex - 1023 + 3000) / 3 - 1000;  // floor((ex - 1023) / 3)
   const int rem = ex - 1023 - 3 * k;
   const float m = __int_as_float(((127 + rem) << 23) | ((hi & 0xfffff) << 3) |
@@ -87,11 +87,18 @@ GPR_D double pow53(double x) {
   const float s = exp2f(-0.33333333f * __log2f(m));  // in (1/2, 1]
   const unsigned sb = __float_as_uint(s);
   const double y = __hiloint2double((int)((sb >> 3) + ((1023 - 127 - k) << 20)), (int)(sb << 29));
-  const double a = fabs(x);
-  const double u = a * (y * y);
+  const double u = fabs(x) * (y * y);
   const double e = fma(-u, y, 1.0);
-  const double p = e * fma(2.0 / 9.0, e, 1.0 / 3.0);
-  const double w = (x * a) * y;
+  p = e * fma(2.0 / 9.0, e, 1.0 / 3.0);
+  return y;
+}
+GPR_D double pow53(double x) {
+  const int ex = (__double2hiint(x) >> 20) & 0x7ff;
+  if ((unsigned)(ex - 723) >= 600u)
+    return pow53_general(x);
+  double p;
+  const double y = icbrt_start(x, p);
+  const double w = (x * fabs(x)) * y;
   return fma(w, p, w);
 }
 

@@ -3,7 +3,7 @@
 // system/relaxation/analytic.cpp:11-162 and solvers/split/ode.cpp:5-11.
 #pragma once
 
-#include "gpr_device.cuh"
+#include "gpr_jacobi.cuh"
 
 namespace gpr {
 
@@ -154,9 +154,10 @@ GPR_D double nondim_time(double r, double detA3, double m0, double u0, double dt
   return P.rho0 * P.b02 * (d4 * d2 * detA3) / (3. * P.mu) * dt;
 }
 
-// analyticSolver_distortion (analytic.cpp:71-128)
-GPR_D void ode_distortion(double *q, double dt, const DevPar &P) {
-  double *A = q + 5;
+// analyticSolver_distortion (analytic.cpp:71-128) by the singular value
+// decomposition, for the distortions that ode_distortion leaves (singular,
+// non-finite, or a determinant beyond 2^+-300).
+static __device__ __noinline__ void ode_distortion_general(double *A, double dt, const DevPar &P) {
   double U[3][3], s[3], Vm[3][3];
   svd3(A, U, s, Vm);
   double detA = s[0] * s[1] * s[2];
@@ -206,12 +207,117 @@ GPR_D void ode_distortion(double *q, double dt, const DevPar &P) {
                      U[i][2] * sc[2] * Vm[j][2];
 }
 
+// analyticSolver_distortion (analytic.cpp:71-128).  The step is one lane's
+// serial FP64 chain per cell (a dependent FP64 instruction takes 64 cycles
+// whatever the grid), so its length is its time:
+//  - A^T A = V diag(d) V^T by jacobi_sym (rotation tangents in FP32);
+//  - the new distortion U diag(s') V^T is A V diag(s' / s) V^T, so neither U nor
+//    the singular values are formed;
+//  - det^(1/3) and its powers from one inverse cube root, the relaxed
+//    exponentials e^(-6 tau), e^(-9 tau) from one e^(-3 tau).
+GPR_D void ode_distortion(double *q, double dt, const DevPar &P) {
+  double *A = q + 5;
+  double S[3][3], V[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = i; j < 3; j++)
+      S[i][j] = A[i] * A[j] + A[3 + i] * A[3 + j] + A[6 + i] * A[6 + j];
+  bool ok = jacobi_sym<3>(S, V);
+  const double det2 = S[0][0] * S[1][1] * S[2][2];
+  ok = ok && S[0][0] > 0.0 && S[1][1] > 0.0 && S[2][2] > 0.0 &&
+       (unsigned)(fp_exponent(det2) - 723) < 600u;
+  if (!ok) {
+    double Am[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      Am[k] = A[k];
+    ode_distortion_general(Am, dt, P);
+#pragma unroll
+    for (int k = 0; k < 9; k++)
+      A[k] = Am[k];
+    return;
+  }
+  const double detA = sqrt64(det2);
+  double p;
+  double y = icbrt_start(detA, p);
+  y = fma(y, p, y);  // det^(-1/3)
+  const double id23 = y * y, d13 = detA * id23;
+  const double s0 = S[0][0] * id23, s1 = S[1][1] * id23, s2 = S[2][2] * id23;
+  const double third = 1.0 / 3.0;
+  const double m0 = (s0 + s1 + s2) * third;
+  const double u0 =
+      ((s0 - s1) * (s0 - s1) + (s1 - s2) * (s1 - s2) + (s2 - s0) * (s2 - s0)) * third;
+  if (u0 < 1e-12)
+    return;
+  double e3;
+  if (P.flags & GPR_POWER_LAW)
+    e3 = exp(-3. * nondim_time(detA * P.rho0, d13, m0, u0, dt, P));
+  else  // tau = rho0 cs^2 det^(7/3) dt / (3 mu)
+    e3 = exp(-(P.rho0 * P.b02) * (detA * detA) * d13 * rcp64(P.mu) * dt);
+  const double e6 = e3 * e3, e9 = e6 * e3;
+  const double a = 3. * m0 - u0 * third - 3.;
+  const double b = 2. * m0 - u0 * third - 2.;
+  const double m = 1. + a * e6 - b * e9;
+  const double u = posd(6. * a * e6 - 9. * b * e9);
+  const double Dl = -2. * m * m * m + m * u + 2.;
+  const double arg1 = posd(6. * u * u * u - 81. * Dl * Dl);
+  double x1;
+  if (fabs(Dl) < 1e-12)
+    x1 = sqrt64(6. * u) * third * 0.86602540378443864676 + m;  // cos(pi/6)
+  else if (arg1 == 0.) {
+    const double tmp = cbrt(54. * Dl);
+    x1 = tmp * (1.0 / 6.0) + u / tmp + m;
+  } else {
+    const double th = atan(sqrt64(arg1) * rcp64(9. * Dl));
+    x1 = sqrt64(6. * u) * third * cos(th * third) + m;
+  }
+  const double tmp2 = 3. * m - x1;
+  const double arg2 = posd(x1 * tmp2 * tmp2 - 4.);
+  const double ix1 = rcp64(x1);
+  const double x2 = 0.5 * (sqrt64(arg2 * ix1) + tmp2);
+  const double x3 = ix1 * rcp64(x2);
+  // the largest goes with the largest singular value: both in the order of
+  // the eigenvalues S_ii
+  const double lo = fmin(fmin(x1, x2), x3), hi = fmax(fmax(x1, x2), x3);
+  const double mid = x1 + x2 + x3 - lo - hi;
+  const double sk[3] = {s0, s1, s2};
+  double f[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double d = S[k][k];
+    const int rank = (int)(d > S[(k + 1) % 3][(k + 1) % 3] ||
+                           (d == S[(k + 1) % 3][(k + 1) % 3] && k < (k + 1) % 3)) +
+                     (int)(d > S[(k + 2) % 3][(k + 2) % 3] ||
+                           (d == S[(k + 2) % 3][(k + 2) % 3] && k < (k + 2) % 3));
+    f[k] = sqrt64((rank == 2 ? hi : (rank == 1 ? mid : lo)) * rcp64(sk[k]));
+  }
+  // A V diag(f) V^T
+  double M[6];  // 00, 11, 22, 01, 02, 12
+#pragma unroll
+  for (int e = 0; e < 6; e++) {
+    const int i = e < 3 ? e : (e == 5 ? 1 : 0), j = e < 3 ? e : (e == 3 ? 1 : 2);
+    double x = 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      x = fma(V[i][k] * f[k], V[j][k], x);
+    M[e] = x;
+  }
+#pragma unroll
+  for (int i = 0; i < 3; i++) {
+    const double a0 = A[3 * i], a1 = A[3 * i + 1], a2 = A[3 * i + 2];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      A[3 * i + j] = a0 * sym3(M, 0, j) + a1 * sym3(M, 1, j) + a2 * sym3(M, 2, j);
+  }
+}
+
 // analyticSolver_thermal (analytic.cpp:130-150)
 template <bool TH>
 GPR_D void ode_thermal(double *q, double dt, const DevPar &P) {
   if (!TH)
     return;
-  double r = q[0], ir = 1.0 / r;
+  double r = q[0], ir = rcp64(r);
   double E = q[1] * ir;
   double v0 = q[2] * ir, v1 = q[3] * ir, v2 = q[4] * ir;
   const double *A = q + 5;
@@ -221,21 +327,21 @@ GPR_D void ode_thermal(double *q, double dt, const DevPar &P) {
   double G01 = A[0] * A[1] + A[3] * A[4] + A[6] * A[7];
   double G02 = A[0] * A[2] + A[3] * A[5] + A[6] * A[8];
   double G12 = A[1] * A[2] + A[4] * A[5] + A[7] * A[8];
-  double t = (G00 + G11 + G22) / 3.0;
+  double t = (G00 + G11 + G22) * (1.0 / 3.0);
   double dg = (G00 - t) * (G00 - t) + (G11 - t) * (G11 - t) + (G22 - t) * (G22 - t) +
               2.0 * (G01 * G01 + G02 * G02 + G12 * G12);
-  double Gm = eos_rho(r, ir, P).G;
-  double cs2 = P.beta == 0.0 ? P.b02 : P.b02 * pow(r * P.ir0, P.beta);
-  double C0 = (1.0 - P.beta / Gm) * cs2;
+  double C0 = P.b02;
+  if (P.has_beta)
+    C0 = (1.0 - P.beta / eos_rho(r, ir, P).G) * (P.b02 * pow(r * P.ir0, P.beta));
   double c1 = E - 0.25 * C0 * dg - 0.5 * (v0 * v0 + v1 * v1 + v2 * v2);
-  double c2 = P.calpha2 / 2.;
-  double k = 2 * P.calpha2 / (P.kappa * r * P.cv);
+  double c2 = P.hca2;
+  double k = 2 * P.ca2ik * ir * P.icv;
   c1 *= k;
   c2 *= k;
   double ea = exp(-c1 * dt / 2);
   double J2 = q[14] * q[14] + q[15] * q[15] + q[16] * q[16];
-  double den = 1 - c2 / c1 * (1 - ea * ea) * J2 * ir * ir;
-  double f = ea / sqrt(den);
+  double den = 1 - c2 * rcp64(c1) * (1 - ea * ea) * J2 * ir * ir;
+  double f = ea * rcp64(sqrt64(den));
   q[14] *= f;
   q[15] *= f;
   q[16] *= f;
