@@ -238,6 +238,11 @@ int gpr_contorted(const double *u, int64_t ncell, double contorted_tol, int32_t 
 int gpr_reset_contorted(double *u, int64_t ncell, double contorted_tol, const gpr_par *pars,
                         int nmat, int32_t *flag, int nvar, void *stream);
 
+/* The NaN test of the reference's loop (solvers/iterator.cpp:153-161) without a
+ * synchronisation: *flag (device double) = 1 if any of the n entries of u is a
+ * NaN; otherwise it is left as it is. */
+int gpr_any_nan(const double *u, int64_t n, double *flag, void *stream);
+
 /* One 1D ADER-WENO step that allocates nothing and takes no scratch.  It has
  * no counterpart in the reference.  It is for callers that cannot allocate
  * device memory (an application that owns the device through its own fixed

@@ -431,6 +431,14 @@ int gpr_iterate(double *u, const int32_t *nX, int ndim, const double *dX, const 
                             S(stream), flux, contorted_tol))
 }
 
+int gpr_any_nan(const double *u, int64_t n, double *flag, void *stream) {
+  if (!u || !flag || n < 1)
+    return GPR_E_ARG;
+  const long nb = (n + 255) / 256, most = 4L * sm_count();
+  k_any_nan<<<(unsigned)(nb < most ? nb : most), 256, 0, S(stream)>>>(u, n, flag);
+  return cuda_rc();
+}
+
 int gpr_contorted(const double *u, int64_t ncell, double contorted_tol, int32_t *flag, int nvar,
                   void *stream) {
   if (!u || !flag || ncell < 1)

@@ -5,6 +5,8 @@
 
 #include <stdio.h>
 
+#include <atomic>
+
 #include "gpr_kernels.cuh"
 
 namespace gpr {
@@ -155,16 +157,23 @@ int launch_stiff(double *qh, const double *wh, long ncb, const uint8_t *mask, in
   constexpr int NP = ND == 1 ? NN * NN : NN * NN * NN;
   constexpr int BS = 64;
   size_t smem = (size_t)(BS / NP) * StiffSmem<L, ND>::per_cell * sizeof(float);
-  // per device and cheap: set on every call
-  cudaFuncSetAttribute(k_predictor_stiff<L, ND, BATCH>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  int dev = 0, nsm = 152, per_sm = 1;
+  // the opt-in and the occupancy do not change: asked once per device (the
+  // queries cost more host time than the launch)
+  static std::atomic<int> blocks_per_sm[64];
+  int dev = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_predictor_stiff<L, ND, BATCH>, BS,
-                                                smem);
+  int per_sm = dev >= 0 && dev < 64 ? blocks_per_sm[dev].load() : 0;
+  if (!per_sm) {
+    cudaFuncSetAttribute(k_predictor_stiff<L, ND, BATCH>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_predictor_stiff<L, ND, BATCH>, BS,
+                                                  smem);
+    per_sm = per_sm > 0 ? per_sm : 1;
+    if (dev >= 0 && dev < 64)
+      blocks_per_sm[dev].store(per_sm);
+  }
   long need = (ncb * NP + BS - 1) / BS;
-  long grid = (long)nsm * (per_sm > 0 ? per_sm : 1);
+  long grid = (long)sm_count() * per_sm;
   if (grid > need)
     grid = need;
   k_predictor_stiff<L, ND, BATCH><<<(int)grid, BS, smem, st>>>(qh, wh, ncb, mask, status, dt,

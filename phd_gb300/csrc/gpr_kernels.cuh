@@ -1697,6 +1697,16 @@ static __global__ void k_clock_advance(double *__restrict__ clk,
     *mx = 0ull;
 }
 
+// *flag = 1 if any of the n entries is a NaN (integer tests on the bit patterns).
+static __global__ void k_any_nan(const double *__restrict__ u, long n, double *__restrict__ flag) {
+  bool found = false;
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n;
+       i += (long)gridDim.x * blockDim.x)
+    found = found || fp_abs_bits(u[i]) > FP_INF_BITS;
+  if (found)
+    *flag = 1.0;
+}
+
 // renorm_distortion (solvers/utils.cpp:6-23); skipped when the device clock
 // says the step did not run (dt == 0).
 template <int V>

@@ -261,8 +261,10 @@ class MultiIterator:
         self.arr, self.pp = _pars(MPs)
         self.scr = torch.empty(max(int(self.lib.gpr_iterate_multi_scratch_doubles(
             self.pn, self.nd, V)), 1), dtype=torch.float64, device=device)
-        self.clock = torch.tensor([0.0, 0.0, float(tf), float(cfl), 0.0], dtype=torch.float64,
-                                  device=device)
+        # the loop's clock, and after it the NaN flag of step(), read together
+        self.control = torch.tensor([0.0, 0.0, float(tf), float(cfl), 0.0, 0.0],
+                                    dtype=torch.float64, device=device)
+        self.clock = self.control[:5]
         self.status = torch.zeros(4, dtype=torch.int32, device=device)
         self.contorted_tol = float(contorted_tol)
 
@@ -276,6 +278,15 @@ class MultiIterator:
         return u
 
 
+    def step(self, u):
+        """One step; returns the host's copy of (t, dt, NaN found)."""
+        self.run(u, 1)
+        _lib.check(self.lib.gpr_any_nan(_dev(u, "u"), u.numel(), _dev(self.control[5:], "flag"),
+                                        _stream()), "any_nan")
+        c = self.control.tolist()
+        return c[0], c[1], c[5] != 0.0
+
+
 def iterate(u, tf, nX, dX, CFL, boundaryTypes, MPs, max_steps=None, contorted_tol=1.0,
             SPLIT=False, HALF_STEP=True, STIFF=False, FLUX=0):
     """GPRpy.solvers.iterator (solvers/iterator.cpp:85-170) with the ghost
@@ -287,19 +298,19 @@ def iterate(u, tf, nX, dX, CFL, boundaryTypes, MPs, max_steps=None, contorted_to
                        contorted_tol=contorted_tol, split=SPLIT, half_step=HALF_STEP,
                        stiff=STIFF, flux=FLUX)
     uf = u.view(-1)
+    uprev = torch.empty_like(uf)
     ret = [None] * 100
     push, count = 0, 0
     while True:
-        uprev = uf.clone()
-        it.run(uf, 1)
-        t, dt, _, _, cnt = it.clock.tolist()
+        uprev.copy_(uf)
+        t, dt, nan = it.step(uf)
         if dt == 0.0:
             break
         count += 1
         if t >= (push + 1) / 100.0 * tf:
             ret[push] = uf.clone()
             push += 1
-        if torch.isnan(uf).any():
+        if nan:
             ret[push] = uprev
             if push + 1 < 100:
                 ret[push + 1] = uf.clone()
