@@ -190,7 +190,7 @@ int fmm_mono_from(const Grid &g) { return fmm_rounds(g) - fmm_tiles_across(g) / 
 // Scratch of one fill (offsets in doubles, 256-byte aligned pieces).
 struct FillLayout {
   long o_d, o_phim, o_dphi, o_star, o_plan, o_fz, o_im0, o_im1, o_lastw, o_pidx, o_dep,
-      o_level, o_cnt, o_flags, o_tflag, o_lastg, o_par, o_d2, o_par2, o_list, o_qst, o_gs,
+      o_level, o_cnt, o_flags, o_tflag, o_lastg, o_par, o_d2, o_par2, o_map, o_gs,
       total;
 };
 
@@ -222,13 +222,12 @@ FillLayout fill_layout(const Grid &g) {
   L.o_tflag = cv.take(dbl((long)fmm_rounds(g) * fmm_tiles(g) * 4L));
   L.o_lastg = cv.take(dbl(n * 4));
   L.o_par = cv.take(dbl(n));
-  // the 2D global sweeps: second buffers, two work lists, list stamps,
-  // counters and the grid barrier
+  // the 2D global sweeps: second buffers, the two maps of waiting points and
+  // the grid barrier
   L.o_d2 = cv.take(n);
   L.o_par2 = cv.take(dbl(n));
-  L.o_list = cv.take(dbl(2 * n * 4));
-  L.o_qst = cv.take(dbl(n * 4));
-  L.o_gs = cv.take(dbl(16 * 4));
+  L.o_map = cv.take(dbl(2 * (n + 16)));
+  L.o_gs = cv.take(2);
   L.total = cv.o;
   return L;
 }
@@ -240,8 +239,8 @@ FillLayout fill_layout(const Grid &g) {
 int fmm_mono_sweeps(const Grid &g) { return 2 * (g.nx + g.ny) + 64; }
 int fmm_max_sweeps(const Grid &g) { return 3 * (g.nx + g.ny) + 128; }
 
-// Blocks of the cooperative k_fmm_global launch: one per SM (the lists
-// rarely hold more points than its threads; fewer blocks make the barrier
+// Blocks of the cooperative k_fmm_global launch: one per SM (a sweep's points
+// rarely fill more warps than its schedulers; fewer blocks make the barrier
 // cheaper).
 int fmm_global_blocks() {
   static int cached[64] = {0};
@@ -289,11 +288,10 @@ int redistance(const double *phi, long ps, double *u, const Grid &g, double *scr
     G.par[0] = par;
     G.par[1] = at<uint8_t>(scr, L.o_par2);
     G.fz = fz;
-    G.list[0] = at<int>(scr, L.o_list);
-    G.list[1] = G.list[0] + g.ncell;
-    G.qst = at<int>(scr, L.o_qst);
-    G.cnt = at<int>(scr, L.o_gs);
-    G.bar = (unsigned *)(G.cnt + 8);
+    const long stride = (g.ncell + 15) / 16 * 16;
+    G.map[0] = at<uint8_t>(scr, L.o_map);
+    G.map[1] = G.map[0] + stride;
+    G.bar = at<unsigned long long>(scr, L.o_gs);
     G.err = err;
     G.sweeps = sweeps;
     G.mono_from = fmm_mono_sweeps(g);
@@ -301,8 +299,8 @@ int redistance(const double *phi, long ps, double *u, const Grid &g, double *scr
     const int nb = fmm_global_blocks();
     if (nb <= 0)
       return GPR_E_CUDA;
-    cudaMemsetAsync(G.cnt, 0, 16 * sizeof(int), st);
-    cudaMemsetAsync(G.qst, 0xff, g.ncell * sizeof(int), st);
+    cudaMemsetAsync(G.bar, 0, 2 * sizeof(unsigned long long), st);
+    cudaMemsetAsync(G.map[0], 0, 2 * stride, st);
     cudaMemcpyAsync(G.d[1], d, g.ncell * sizeof(double), cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(G.par[1], par, g.ncell, cudaMemcpyDeviceToDevice, st);
     k_fmm_seed<<<blocks(g.ncell, 256), 256, 0, st>>>(g, G, clk);

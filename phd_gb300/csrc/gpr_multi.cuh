@@ -113,7 +113,8 @@ __global__ void k_fmm_init(const double *__restrict__ phi, long ps, double *__re
   }
   d[c] = x;
   fz[c] = (frozen ? 1 : 0) | pos;
-  par[c] = 0;
+  // (2D: the flags again in bits 4 and 5, so that a sweep reads one byte)
+  par[c] = g.nd == 2 ? ((frozen ? 1 : 0) | pos) << 4 : 0;
   if (frozen)
     atomicOr(anyfrozen, 1);
 }
@@ -145,6 +146,12 @@ inline FmmConst fmm_const(double dx, double dy) {
   return K;
 }
 
+// |x| compares as the integer of its bits (the order of |x| for finite
+// values and infinity), on the integer pipe.
+GPR_D unsigned long long fmm_key(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+
 // updatePointOrderOne + solveQuadratic (distance_marcher.cpp:5-28, 72-88)
 // for the entered axes (use): a = sum idx2, b = -sum 2 idx2 v, c = sum idx2
 // v^2 - 1, root (-b +- sqrt(b^2 - 4ac)) / 2 / a by the sign of phi, in FP64
@@ -171,13 +178,14 @@ GPR_D bool fmm_root(const double v[2], const bool use[2], const FmmConst &K, int
   const int ka = use[0] && use[1] ? 2 : (use[0] ? 0 : 1);
   c = sub(c, 1.0);
   const double det = __fma_rn(b, b, -mul(K.a4[ka], c));
-  if (!(det > 0.0))
+  // (comparisons on the bits where they are exact: the integer pipe)
+  if (__double_as_longlong(det) <= 0 || fmm_key(det) > 0x7ff0000000000000ull)
     return false;
   const double sq = __dsqrt_rn(det);
   const double num = mul(pos ? add(-b, sq) : sub(-b, sq), 0.5);
   const double q0 = mul(num, K.ra[ka]);
   x = __fma_rn(__fma_rn(-q0, K.a[ka], num), K.ra[ka], q0);
-  return x != 0.0;
+  return fmm_key(x) != 0ull;
 }
 
 // Update of one unfrozen point from its neighbours' current values
@@ -202,13 +210,6 @@ GPR_D bool fmm_root(const double v[2], const bool use[2], const FmmConst &K, int
 // whether the next neighbour enters and the decision is clear by 256 times
 // that bound, and evaluated exactly where it is the result or the decision
 // is close.  The result is the same as evaluating every root exactly.
-//
-// |x| compares as the integer of its bits (the order of |x| for finite
-// values and infinity), on the integer pipe.
-GPR_D unsigned long long fmm_key(double x) {
-  return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
-}
-
 GPR_D double fmm_update(const double nb[2][2], const bool band[2][2], const bool excl[2][2],
                         bool pos, int nd, double old, const FmmConst &K, int &mask) {
   const double INF = INFINITY;
@@ -294,6 +295,50 @@ GPR_D double fmm_update(const double nb[2][2], const bool band[2][2], const bool
       t = r;
   }
   return isinf(t) ? old : t;
+}
+
+// fmm_update in 2D, with one root for all lanes of a warp.  Away from the band
+// the entered set is decided from v +- h alone (above), so the smaller
+// neighbour enters, the other one enters or not, and the quadratic of the
+// final set is evaluated once; in fmm_update the one- and two-axis roots
+// are different branches, which a warp takes one after the other.  Band
+// neighbours, close decisions and quadratics without a real root take
+// fmm_update itself.  The value and the mask are fmm_update's bit for bit.
+GPR_D double fmm_update_2d(const double nb[2][2], const bool band[2][2], const bool excl[2][2],
+                           bool pos, double old, const FmmConst &K, int &mask) {
+  const unsigned long long KINF = 0x7ff0000000000000ull;
+  double v[2] = {INFINITY, INFINITY};
+  unsigned long long ck[2] = {KINF, KINF};
+  int cs[2] = {0, 0};
+#pragma unroll
+  for (int dim = 0; dim < 2; dim++)
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+      const unsigned long long kx = fmm_key(nb[dim][s]);
+      if (!excl[dim][s] && kx < ck[dim]) {
+        ck[dim] = kx;
+        v[dim] = nb[dim][s];
+        cs[dim] = s;
+      }
+    }
+  const bool second = ck[1] < ck[0], tie = ck[0] == ck[1];
+  const double va = second ? v[1] : v[0], h = second ? K.h[1] : K.h[0];
+  const double wb = fabs(second ? v[0] : v[1]), t = fabs(va + (pos ? h : -h));
+  // the bound in FP32, from high words (relative error below 2^-19, an
+  // overflow or NaN makes every comparison false)
+  const float wf = f32_abs_hi(va), hf = f32_abs_hi(h) * 1.00001f;
+  const float tm = 1.0001f * 256.0f * (float)DBL_EPSILON *
+                   (wf * (wf * f32_abs_hi(second ? K.ih[1] : K.ih[0])) + wf + hf);
+  const bool both = tie || fmm_key(wb) < fmm_key(t);
+  const bool use[2] = {both || !second, both || second};
+  bool easy = !(band[0][0] || band[0][1] || band[1][0] || band[1][1]);
+  easy = easy && (tie || (f32_abs_hi(t) > tm && f32_abs_hi(wb - t) > tm));
+  double x;
+  easy = fmm_root(v, use, K, 2, pos, x) && easy && fmm_key(x) < KINF;
+  if (!easy)
+    return fmm_update(nb, band, excl, pos, 2, old, K, mask);
+  mask = (use[0] ? 1 << cs[0] : 0) | (use[1] ? 4 << cs[1] : 0);
+  return x;
 }
 
 // The four neighbours of shared-memory point m (x neighbours m -+ o0, y
@@ -534,23 +579,37 @@ __global__ void __launch_bounds__(FmmThreads<ND>::value, ND == 2 ? 16 : 2)
 // exchange halos only between launches, so information crosses a tile per
 // round and each tile re-sweeps its points until its halo settles (33-91
 // updates per cell on the 800 x 400 bubble).  Here every sweep sees the
-// previous sweep's values everywhere: a sweep updates only the points whose
-// neighbours changed in the previous sweep (a work list), the front moves a
-// cell per sweep, and the number of sweeps is the depth of the marcher's
-// dependency chain (~1.4 x the largest distance in cells).  Each sweep is
-// one FP64 update per listed point (one lane each) and one barrier, so a
-// sweep costs about one update's FP64 chain (on GB300 a warp's FP64
-// instruction holds its partition's FP64 unit ~64 cycles) plus the barrier.
+// previous sweep's values everywhere: a sweep updates only the points that
+// changed, or whose neighbours changed, in the previous sweep, the front
+// moves a cell per sweep, and the number of sweeps is the depth of the
+// marcher's dependency chain (~1.3 x the largest distance in cells: 680
+// sweeps of 14400 points, a ring ~25 cells wide, on that bubble).
+//
+// What bounds it is a sweep's latency, not its work (3 warps of points per
+// SM): the waiting points are marked in a byte map, a plain store that
+// nobody waits for; each block reads the map of its own cells (dealt out in
+// segments of 8, so that a front's ring falls on all SMs alike), gathers
+// the marked ones into a list in shared memory and updates them, a lane
+// each; then the barrier.  Of a sweep's 13000 cycles (6.7 us, 4.5 ms for the
+// bubble) the map and the list take 2500, the update 5000 (43 FP64
+// instructions at 64 cycles a warp) and the barrier 5500, whose release
+// waits for the sweep's stores.  Before, lists of points in global memory
+// with a stamp per point cost 5500 cycles for the dependent atomics that
+// dedupe and append, and entries dealt out by the block left 96 SMs idle: 11
+// us a sweep.  Also measured: stamping only the changed point and reading
+// the map around each segment, fewer stores and seven loads for one (8.2
+// us); whole parts of the grid in shared memory, exchanging frames every 4
+// sweeps, where the ring falls on few of them (25 us).
 //
 // Jacobi with two buffers: sweep s reads d[s % 2] / par[s % 2] and writes
-// d[(s + 1) % 2] / par[(s + 1) % 2] for its listed points; a point that
-// changes lists itself for the next sweep as well as its unfrozen
-// neighbours, which copies its new value into the other buffer, so after
-// sweep s the written buffer holds every point's latest value.  The fixed
-// point, and so the result, is that of the tiled form: the sweeps end when
-// no point changes, whatever the order of the work.  From sweep mono_from
-// on only smaller |d| is taken (termination, as the tiled form's last
-// rounds); a list still non-empty after max_sweeps sets err bit 0.
+// d[(s + 1) % 2] / par[(s + 1) % 2] for its marked points; a point that
+// changes marks itself for the next sweep as well as its neighbours, which
+// copies its new value into the other buffer, so after sweep s the written
+// buffer holds every point's latest value.  The fixed point, and so the
+// result, is that of the tiled form: the sweeps end when no point changes,
+// whatever the order of the work.  From sweep mono_from on only smaller |d|
+// is taken (termination, as the tiled form's last rounds); a change still
+// found in sweep max_sweeps - 1 sets err bit 0.
 //
 // The blocks wait for one another at the barrier, so the kernel is launched
 // cooperatively (all blocks resident); each wait is bounded (~1 s), after
@@ -559,23 +618,16 @@ struct FmmGlobal {
   double *d[2];
   uint8_t *par[2];
   const uint8_t *fz;
-  int *list[2];
-  int *qst;           // the sweep a point is listed for (dedupes the lists)
-  int *cnt;           // cnt[3]: list lengths, rotating
-  unsigned *bar;      // bar + 2: the barrier's two 64-bit words
+  uint8_t *map[2];          // a byte per cell: waits for sweep s (map[s % 2])
+  unsigned long long *bar;  // the barrier's two words
   int *err;
-  int *sweeps;        // optional: receives the sweeps taken
+  int *sweeps;  // optional: receives the sweeps taken
   int mono_from, max_sweeps;
 };
 
-// GPU-scope acquire / release accesses (PTX memory model, sm_70 and later).
-GPR_D unsigned long long fmm_add_acq_rel64(unsigned long long *p, unsigned long long v) {
-  unsigned long long old;
-  asm volatile("atom.acq_rel.gpu.global.add.u64 %0, [%1], %2;"
-               : "=l"(old)
-               : "l"(p), "l"(v)
-               : "memory");
-  return old;
+// GPU-scope release / acquire accesses (PTX memory model, sm_70 and later).
+GPR_D void fmm_add_release64(unsigned long long *p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" : : "l"(p), "l"(v) : "memory");
 }
 GPR_D unsigned long long fmm_ld_acquire(const unsigned long long *p) {
   unsigned long long v;
@@ -583,178 +635,195 @@ GPR_D unsigned long long fmm_ld_acquire(const unsigned long long *p) {
   return v;
 }
 
-// Grid barrier at the end of sweep s, which also sums the sweep's list
-// appends: the 64-bit word words[s % 2] counts the blocks' arrivals (bits
-// 40..63) and the entries they appended (bits 0..39) over the sweeps of that
-// parity.  Each block arrives once (one thread, an acquire-release add of
-// 2^40 + its appends, after the block barrier, which orders the block's
-// writes before it) and waits with acquire loads until all blocks have
-// arrived for this sweep: nblocks (s / 2 + 1) arrivals.  Two words, so that
-// a block already at the next sweep's barrier cannot be counted here.  The
-// next list's length is the sum's growth since the previous sweep of the
-// same parity (prev[2], kept by the block).  The wait gives up after ~1 s
-// (err bit 2).  Returns the length, or -1 after a timeout.
-GPR_D int fmm_grid_sync(unsigned long long *words, unsigned nblocks, int s, int appended,
+// Grid barrier at the end of sweep s, which also sums what the blocks report
+// (changed: 1 if any of the block's points did): the 64-bit word words[s % 2]
+// counts the arrivals (bits 40..63) and the reports (bits 0..39) over the
+// sweeps of that parity.  Each block arrives once (one thread, a release add
+// after the block barrier, which orders the block's writes before it) and
+// waits with acquire loads until all blocks have arrived for this sweep:
+// nblocks (s / 2 + 1) arrivals.  Two words, so that a block already at the
+// next sweep's barrier cannot be counted here.  The sweep's sum is the
+// word's growth since the previous sweep of the same parity (prev[2], kept
+// by the block).  The wait gives up after ~1 s (err bit 2).  Returns the
+// sum, or -1 after a timeout.
+GPR_D int fmm_grid_sync(unsigned long long *words, unsigned nblocks, int s, int changed,
                         unsigned long long prev[2], int *err) {
   __shared__ int shn;
   constexpr unsigned long long ARR = 1ull << 40, CNT = ARR - 1;
-  __syncthreads();
+  // the block barrier is the caller's (it also makes `changed`)
   if (threadIdx.x == 0) {
     const int k = s & 1;
     unsigned long long *w = words + k;
     const unsigned long long target = (unsigned long long)nblocks * (unsigned)(s / 2 + 1);
-    unsigned long long v = fmm_add_acq_rel64(w, ARR + (unsigned)appended) + ARR + (unsigned)appended;
+    fmm_add_release64(w, ARR + (unsigned)changed);
+    unsigned long long v = fmm_ld_acquire(w);
     const long long t0 = clock64();
-    shn = 0;
+    int n = 0;
     while ((v >> 40) < target) {
       if (clock64() - t0 > 2000000000LL) {  // ~1 s at 2 GHz
         atomicOr(err, 4);
-        shn = -1;
+        n = -1;
         break;
       }
       v = fmm_ld_acquire(w);
     }
-    if (shn == 0) {
-      shn = (int)((v & CNT) - prev[k]);
-      prev[k] = v & CNT;
+    if (n == 0) {
+      n = (int)((v & CNT) - (k ? prev[1] : prev[0]));
+      (k ? prev[1] : prev[0]) = v & CNT;
     }
+    shn = n;
   }
   __syncthreads();
   return shn;
 }
 
-// Lists the candidates cand[k] with want[k] for sweep s, each point once per
-// sweep (stamps in qst): the stamps' atomics are issued back to back, and a
-// warp reserves its list entries with one atomic.
-template <int K>
-GPR_D void fmm_enqueue(const bool (&want)[K], const int (&cand)[K], int s, const FmmGlobal &G,
-                       int *appended = nullptr) {
-  bool mine[K];
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    mine[k] = want[k] ? atomicMax(G.qst + cand[k], s) < s : false;
-  int nk = 0;
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    nk += mine[k];
-  const int lane = threadIdx.x & 31;
-  int incl = nk;  // inclusive warp scan
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o)
-      incl += y;
-  }
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
-  if (total == 0)
-    return;
-  int base = 0;
-  if (lane == 31) {
-    base = atomicAdd(G.cnt + s % 3, total);
-    if (appended)
-      atomicAdd(appended, total);  // the block's appends (shared memory)
-  }
-  base = __shfl_sync(0xffffffffu, base, 31);
-  int pos = base + incl - nk;
-  int *lst = G.list[s & 1];
-#pragma unroll
-  for (int k = 0; k < K; k++)
-    if (mine[k])
-      lst[pos++] = cand[k];
-}
-
-// The first list: unfrozen points next to the frozen band.
+// The first map: unfrozen points next to the frozen band.
 __global__ void k_fmm_seed(Grid g, FmmGlobal G, const double *__restrict__ clk) {
   if (clk && clk[0] >= clk[2])
     return;
   const long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  bool want[1] = {false};
-  if (c < g.ncell && !(G.fz[c] & 1)) {
-    const int i = c / g.ny, j = c % g.ny;
-    want[0] = (i > 0 && (G.fz[c - g.ny] & 1)) || (i < g.nx - 1 && (G.fz[c + g.ny] & 1)) ||
-              (j > 0 && (G.fz[c - 1] & 1)) || (j < g.ny - 1 && (G.fz[c + 1] & 1));
-  }
-  const int cand[1] = {(int)(c < g.ncell ? c : 0)};
-  fmm_enqueue<1>(want, cand, 0, G);
+  if (c >= g.ncell || (G.fz[c] & 1))
+    return;
+  const int i = c / g.ny, j = c % g.ny;
+  if ((i > 0 && (G.fz[c - g.ny] & 1)) || (i < g.nx - 1 && (G.fz[c + g.ny] & 1)) ||
+      (j > 0 && (G.fz[c - 1] & 1)) || (j < g.ny - 1 && (G.fz[c + 1] & 1)))
+    G.map[0][c] = 1;
 }
 
-__global__ void __launch_bounds__(256) k_fmm_global(Grid g, FmmConst K, FmmGlobal G,
-                                                     const double *__restrict__ clk) {
+constexpr int FMM_G_THREADS = 256, FMM_G_SEGS = 2;  // segments per thread and pass
+
+__global__ void __launch_bounds__(FMM_G_THREADS) k_fmm_global(Grid g, FmmConst K, FmmGlobal G,
+                                                              const double *__restrict__ clk) {
   if (clk && clk[0] >= clk[2])
     return;
-  const unsigned nb = gridDim.x;
-  const long nthr = (long)gridDim.x * blockDim.x;
-  const long gid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  __shared__ int appended;
-  if (threadIdx.x == 0)
-    appended = 0;
+  constexpr int NT = FMM_G_THREADS, U = FMM_G_SEGS;
+  __shared__ int list[NT * U * 8], nlist;
+  const int tid = threadIdx.x, lane = tid & 31, nb = gridDim.x;
+  const int nseg = (int)((g.ncell + 7) / 8), ngroup = (nseg + nb - 1) / nb;
+  // Segment of this block in group k of nb consecutive ones: the blocks take
+  // them in turn, shifted by 61 from group to group (152 = 8 x 19), since a
+  // grid whose rows are whole groups would give a column to one block.
+  auto segment = [&](int k) {
+    const int at = ((int)blockIdx.x + nb - (int)((61L * k) % nb)) % nb;
+    return k < ngroup ? k * nb + at : nseg;
+  };
+  int mine[U];
+#pragma unroll
+  for (int u = 0; u < U; u++)
+    mine[u] = segment(u * NT + tid);
+  if (tid == 0)
+    nlist = 0;
+  __syncthreads();
   unsigned long long prev[2] = {0ull, 0ull};  // used by thread 0
-  int s = 0;
-  int n = __ldcg(G.cnt);  // the first list (k_fmm_seed)
-  for (; s < G.max_sweeps; s++) {
-    if (n <= 0)
-      break;
-    if (gid == 0)
-      G.cnt[(s + 2) % 3] = 0;  // the list count of sweep s - 1, no longer read
+  int s = 0, n = 1;
+  for (; s < G.max_sweeps && n > 0; s++) {
     const double *src = G.d[s & 1];
     double *dst = G.d[(s + 1) & 1];
     const uint8_t *psrc = G.par[s & 1];
     uint8_t *pdst = G.par[(s + 1) & 1];
-    const int *lst = G.list[s & 1];
+    uint8_t *map = G.map[s & 1], *next = G.map[(s + 1) & 1];
     const bool mono = s >= G.mono_from;
-    // whole warps take list entries, so that the enqueues can aggregate
-    const long nround = (n + 31) / 32 * 32;
-    for (long q = gid; q < nround; q += nthr) {
-      const bool live = q < n;
-      const int c = live ? __ldcg(lst + q) : 0;
-      const int i = c / g.ny, j = c % g.ny;
-      bool chg = false;
-      if (live) {
+    bool any = false;
+    for (int k0 = 0; k0 < ngroup; k0 += NT * U) {
+      uint2 w[U], fr[U];
+      int seg[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        seg[u] = k0 ? segment(k0 + u * NT + tid) : mine[u];
+        const bool in = seg[u] < nseg;
+        // (the map's and fz's last segment ends within their padding)
+        w[u] = in ? __ldcg((const uint2 *)map + seg[u]) : make_uint2(0u, 0u);
+        fr[u] = in ? *((const uint2 *)G.fz + seg[u]) : make_uint2(0u, 0u);
+      }
+      unsigned bits = 0;  // 8 u + b: cell b of segment u
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (w[u].x | w[u].y)
+          __stcg((uint2 *)map + seg[u], make_uint2(0u, 0u));
+        // bytes 0 or 1, frozen points left out; the four bytes' bits together
+        const unsigned lo = w[u].x & ~fr[u].x & 0x01010101u, hi = w[u].y & ~fr[u].y & 0x01010101u;
+        bits |= (((lo * 0x01020408u) >> 24) | ((hi * 0x01020408u) >> 24) << 4) << (8 * u);
+      }
+      int incl = __popc(bits);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        incl += lane >= o ? y : 0;
+      }
+      int pos = 0;
+      if (lane == 31 && incl)
+        pos = atomicAdd(&nlist, incl);
+      pos = __shfl_sync(0xffffffffu, pos, 31) + incl - __popc(bits);
+      while (bits) {
+        const int b = __ffs(bits) - 1;
+        bits &= bits - 1;
+        int sg = seg[0];
+#pragma unroll
+        for (int u = 1; u < U; u++)
+          sg = (b >> 3) == u ? seg[u] : sg;
+        list[pos++] = sg * 8 + (b & 7);
+      }
+      __syncthreads();
+      const int nl = nlist;
+      for (int q = tid; q < nl; q += NT) {
+        const int c = list[q];
+        const int i = c / g.ny, j = c - i * g.ny;
         double nb4[2][2];
         bool bd[2][2], ex[2][2];
-        const long cn[2][2] = {{c - g.ny, c + g.ny}, {c - 1, c + 1}};
+        const int cn[2][2] = {{c - g.ny, c + g.ny}, {c - 1, c + 1}};
         const bool in[2][2] = {{i > 0, i < g.nx - 1}, {j > 0, j < g.ny - 1}};
         // a neighbour that recorded this point as entered (its bit for the
         // opposite side) is not a candidate: bits 2 dim + side
         const int xb[2][2] = {{1, 0}, {3, 2}};
+#pragma unroll
         for (int dim = 0; dim < 2; dim++)
+#pragma unroll
           for (int sd = 0; sd < 2; sd++) {
             const bool ok = in[dim][sd];
-            const long m = ok ? cn[dim][sd] : c;
-            nb4[dim][sd] = ok ? __ldcg(src + m) : INFINITY;
-            bd[dim][sd] = ok && (G.fz[m] & 1);
-            ex[dim][sd] = ok && ((__ldcg(psrc + m) >> xb[dim][sd]) & 1);
+            const int m = ok ? cn[dim][sd] : c;
+            const double x = __ldcg(src + m);
+            const uint8_t pm = __ldcg(psrc + m);
+            nb4[dim][sd] = ok ? x : INFINITY;
+            bd[dim][sd] = ok && (pm & 16);
+            ex[dim][sd] = ok && ((pm >> xb[dim][sd]) & 1);
           }
         const double old = __ldcg(src + c);
         const uint8_t pold = __ldcg(psrc + c);
         int msk;
-        const double nv = fmm_update(nb4, bd, ex, (G.fz[c] & 2) != 0, 2, old, K, msk);
-        chg = mono ? fabs(nv) < fabs(old) : (nv != old || (uint8_t)msk != pold);
+        const double nv = fmm_update_2d(nb4, bd, ex, (pold & 32) != 0, old, K, msk);
+        const bool chg = mono ? fmm_key(nv) < fmm_key(old)
+                              : (__double_as_longlong(nv) != __double_as_longlong(old) ||
+                                 msk != (pold & 15));
         __stcg(dst + c, chg ? nv : old);
-        __stcg(pdst + c, chg ? (uint8_t)msk : pold);
-      }
-      // list the point itself and its unfrozen neighbours for sweep s + 1
-      const int cand[5] = {c, i > 0 ? c - g.ny : c, i < g.nx - 1 ? c + g.ny : c,
-                           j > 0 ? c - 1 : c, j < g.ny - 1 ? c + 1 : c};
-      bool want[5] = {chg, chg && i > 0, chg && i < g.nx - 1, chg && j > 0, chg && j < g.ny - 1};
+        __stcg(pdst + c, chg ? (uint8_t)(msk | (pold & 48)) : pold);
+        if (chg) {  // the point itself and its neighbours wait for sweep s + 1
+          any = true;
+          __stcg(next + c, (uint8_t)1);
 #pragma unroll
-      for (int k = 1; k < 5; k++)
-        want[k] = want[k] && !(G.fz[cand[k]] & 1);
-      fmm_enqueue<5>(want, cand, s + 1, G, &appended);
+          for (int dim = 0; dim < 2; dim++)
+#pragma unroll
+            for (int sd = 0; sd < 2; sd++)
+              if (in[dim][sd])
+                __stcg(next + cn[dim][sd], (uint8_t)1);
+        }
+      }
+      if (k0 + NT * U < ngroup) {  // the list again, for the next pass
+        __syncthreads();
+        if (tid == 0)
+          nlist = 0;
+        __syncthreads();
+      }
     }
-    __syncthreads();
-    const int app = appended;
-    __syncthreads();
-    if (threadIdx.x == 0)
-      appended = 0;
-    n = fmm_grid_sync((unsigned long long *)(G.bar + 2), nb, s, app, prev, G.err);
+    const int changed = __syncthreads_or(any);
+    if (tid == 0)
+      nlist = 0;
+    n = fmm_grid_sync(G.bar, (unsigned)nb, s, changed ? 1 : 0, prev, G.err);
     if (n < 0)
       return;
   }
-  if (gid == 0 && s >= G.max_sweeps && n != 0)
-    atomicOr(G.err, 1);  // not converged within the sweep budget
-  if (gid == 0) {
-    G.cnt[3] = s;  // the sweeps taken
+  if (blockIdx.x == 0 && tid == 0) {
+    if (n != 0)
+      atomicOr(G.err, 1);  // not converged within the sweep budget
     if (G.sweeps)
       *G.sweeps = s;
   }
