@@ -341,7 +341,7 @@ int boundary_fill(double *grid, const double *phim, const double *dphi, const in
                                                      cnt + 1, pidx, lastw, err, clk);
   k_plan_deps<<<kPlanGrid, 128, 0, st>>>(plan, cnt + 1, pidx, lastw, dep, clk);
   k_plan_levels<<<kPlanGrid, 128, 0, st>>>(cnt + 1, dep, level, cnt + 2, clk);
-  k_star_level0<V15><<<kPlanGrid, 64, 0, st>>>(plan, cnt + 1, dep, level, grid, star, P0, P1,
+  k_star_level0<V15><<<kPlanGrid, 32, 0, st>>>(plan, cnt + 1, dep, level, grid, star, P0, P1,
                                                mat, dt, dt_dev, g.nd, clk);
   k_star_levels<V15><<<1, 64, 0, st>>>(plan, cnt + 1, dep, level, cnt + 2, grid, star, P0,
                                        P1, mat, dt, dt_dev, g.nd, clk);
@@ -489,7 +489,7 @@ int gpr_left_star_state(const double *QL, const double *QR, const double *n, dou
     return GPR_E_UNSUPPORTED;
   if (count == 0)
     return GPR_OK;
-  k_star_pointwise<V15><<<blocks(count, 64), 64, 0, S(stream)>>>(
+  k_star_pointwise<V15><<<blocks(2 * count, 64), 64, 0, S(stream)>>>(
       QL, QR, n, out, count, ndim, dt, make_devpar(*parL), make_devpar(*parR));
   return cuda_rc();
 }

@@ -990,52 +990,54 @@ GPR_D void rotate(double *Q, const double R[3][3]) {
 }
 
 // Gaussian elimination with partial pivoting: A X = B in place (A n x n,
-// B n x m, row-major).  Returns false on a zero pivot.
+// B n x m, row-major).  Returns false on a zero pivot.  Rows are exchanged
+// one comparison at a time, so that every index is a constant (arrays in
+// registers), and each pivot is inverted once.
 template <int n, int m> GPR_D bool gauss(double *A, double *B) {
+  double ip[n];
+#pragma unroll
   for (int c = 0; c < n; c++) {
-    int p = c;
-    for (int r = c + 1; r < n; r++)
-      if (fabs(A[r * n + c]) > fabs(A[p * n + c]))
-        p = r;
-    if (A[p * n + c] == 0.0)
-      return false;
-    if (p != c) {
-      for (int j = 0; j < n; j++) {
-        double t = A[c * n + j];
-        A[c * n + j] = A[p * n + j];
-        A[p * n + j] = t;
+#pragma unroll
+    for (int r = c + 1; r < n; r++) {
+      const bool sw = fp_abs_bits(A[r * n + c]) > fp_abs_bits(A[c * n + c]);
+#pragma unroll
+      for (int j = c; j < n; j++) {
+        const double t = A[c * n + j], u = A[r * n + j];
+        A[c * n + j] = sw ? u : t;
+        A[r * n + j] = sw ? t : u;
       }
+#pragma unroll
       for (int j = 0; j < m; j++) {
-        double t = B[c * m + j];
-        B[c * m + j] = B[p * m + j];
-        B[p * m + j] = t;
+        const double t = B[c * m + j], u = B[r * m + j];
+        B[c * m + j] = sw ? u : t;
+        B[r * m + j] = sw ? t : u;
       }
     }
+    if (A[c * n + c] == 0.0)
+      return false;
+    ip[c] = rcp64(A[c * n + c]);
+#pragma unroll
     for (int r = c + 1; r < n; r++) {
-      double f = A[r * n + c] / A[c * n + c];
-      for (int j = c; j < n; j++)
-        A[r * n + j] -= f * A[c * n + j];
+      const double f = -A[r * n + c] * ip[c];
+#pragma unroll
+      for (int j = c + 1; j < n; j++)
+        A[r * n + j] = fma(f, A[c * n + j], A[r * n + j]);
+#pragma unroll
       for (int j = 0; j < m; j++)
-        B[r * m + j] -= f * B[c * m + j];
+        B[r * m + j] = fma(f, B[c * m + j], B[r * m + j]);
     }
   }
+#pragma unroll
   for (int c = n - 1; c >= 0; c--)
+#pragma unroll
     for (int j = 0; j < m; j++) {
-      double s = B[c * m + j];
+      double t = B[c * m + j];
+#pragma unroll
       for (int k = c + 1; k < n; k++)
-        s -= A[c * n + k] * B[k * m + j];
-      B[c * m + j] = s / A[c * n + c];
+        t = fma(-A[c * n + k], B[k * m + j], t);
+      B[c * m + j] = t * ip[c];
     }
   return true;
-}
-
-GPR_D bool inv3(const double *M, double *out) {
-  double A[9];
-  for (int k = 0; k < 9; k++) {
-    A[k] = M[k];
-    out[k] = (k % 4) == 0 ? 1.0 : 0.0;
-  }
-  return gauss<3, 3>(A, out);
 }
 
 // Eigenvalues of a real 3 x 3 matrix from its characteristic polynomial
@@ -1045,7 +1047,7 @@ GPR_D bool inv3(const double *M, double *out) {
 // reference's Q diag(Re(lambda)^(-1/2)) Q^(-1) with Q = Re(eigenvectors)
 // (riemann.cpp:136-141) is NaN or singular there and its star state falls
 // back to the input state.
-GPR_D bool eig3_real_positive(const double *M) {
+static __device__ __noinline__ bool eig3_real_positive(const double *M) {
   double p1 = M[0] + M[4] + M[8];
   double p2 = M[0] * M[4] - M[1] * M[3] + M[0] * M[8] - M[2] * M[6] + M[4] * M[8] -
               M[5] * M[7];
@@ -1079,33 +1081,73 @@ GPR_D bool eig3_real_positive(const double *M) {
   return lo > 0.0;
 }
 
-// Inverse principal square root by the Denman-Beavers iteration
-// (Y -> M^(1/2), Z -> M^(-1/2)); the reference forms the same matrix
-// function from an eigen-decomposition (riemann.cpp:136-141).
+// Whether the eigenvalues of M are real and positive, as eig3_real_positive
+// decides.  With disc <= 0 the roots are real, and positive exactly when the
+// coefficients p1, p2 and p3 are; a complex pair's imaginary part is at most
+// sqrt(3 disc) / -a, which settles the rounding-level pairs of a nearly
+// isotropic state; anything else takes eig3_real_positive (roots and
+// angles).
+GPR_D bool spectrum_positive(const double *M) {
+  const double m1 = M[4] * M[8] - M[5] * M[7], m2 = M[0] * M[8] - M[2] * M[6],
+               m3 = M[0] * M[4] - M[1] * M[3];
+  const double p1 = M[0] + M[4] + M[8], p2 = m1 + m2 + m3;
+  const double p3 = M[0] * m1 - M[1] * (M[3] * M[8] - M[5] * M[6]) +
+                    M[2] * (M[3] * M[7] - M[4] * M[6]);
+  const double a = p2 - p1 * p1 * (1.0 / 3.0);
+  const double b = p1 * fma(-2.0 / 27.0 * p1, p1, p2 * (1.0 / 3.0)) - p3;
+  const double disc = fma(b * b, 0.25, a * a * a * (1.0 / 27.0));
+  const double lim = 0.9e-6 / 3.0 * p1 * a;
+  bool ok = p1 > 0.0 && p2 > 0.0 && p3 > 1e-10 * p1 * p1 * p1;
+  ok = ok && (disc <= 0.0 || (a < 0.0 && 3.0 * disc < lim * lim));
+  return ok || eig3_real_positive(M);
+}
+
+GPR_D bool inv3(const double *M, double *out) {
+  double A[9];
+  for (int k = 0; k < 9; k++) {
+    A[k] = M[k];
+    out[k] = (k % 4) == 0 ? 1.0 : 0.0;
+  }
+  return gauss<3, 3>(A, out);
+}
+
+// Inverse principal square root of a matrix with positive eigenvalues by the
+// Denman-Beavers iteration (Y -> M^(1/2), Z -> M^(-1/2)), on M over the mean
+// of its eigenvalues; the reference forms the same matrix function from an
+// eigen-decomposition (riemann.cpp:136-141).  An update below 3e-9 leaves an
+// error below its square, so the iteration ends with it: 5 iterations for
+// eigenvalues 1 : 1 : 3 (9 unscaled and run to a standstill), with the same
+// errors against 64-bit mantissas (mean 2e-16).  The closed form by the
+// theorem of Cayley and Hamilton takes an eighth of the operations and
+// loses a digit.
 GPR_D bool inv_sqrt3(const double *M, double *Zout) {
   double Y[9], Z[9], Yi[9], Zi[9];
+  const double sc = 3.0 * rcp64(M[0] + M[4] + M[8]);
+#pragma unroll
   for (int k = 0; k < 9; k++) {
-    Y[k] = M[k];
-    Z[k] = (k % 4) == 0 ? 1.0 : 0.0;
+    Y[k] = M[k] * sc;
+    Z[k] = Zi[k] = (k % 4) == 0 ? 1.0 : 0.0;
   }
-  int extra = 0;
+#pragma unroll 1
   for (int it = 0; it < 100; it++) {
-    if (!inv3(Y, Yi) || !inv3(Z, Zi))
+    if (!inv3(Y, Yi) || (it > 0 && !inv3(Z, Zi)))
       return false;
-    double dmax = 0.0, ymax = 0.0;
+    float dmax = 0.0f, ymax = 0.0f;
+#pragma unroll
     for (int k = 0; k < 9; k++) {
-      double y = 0.5 * (Y[k] + Zi[k]);
-      double z = 0.5 * (Z[k] + Yi[k]);
-      dmax = fmax(dmax, fabs(y - Y[k]));
-      ymax = fmax(ymax, fabs(y));
-      Y[k] = y;
-      Z[k] = z;
+      const double e = 0.5 * (Zi[k] - Y[k]);
+      Y[k] += e;
+      Z[k] = 0.5 * (Z[k] + Yi[k]);
+      dmax = fmaxf(dmax, f32_abs_hi(e));
+      ymax = fmaxf(ymax, f32_abs_hi(Y[k]));
     }
-    if (dmax <= 1e-13 * ymax && ++extra == 2)
+    if (!(dmax > 3e-9f * ymax))
       break;
   }
+  const double f = sqrt64(sc);
+#pragma unroll
   for (int k = 0; k < 9; k++)
-    Zout[k] = Z[k];
+    Zout[k] = Z[k] * f;
   return true;
 }
 
@@ -1122,133 +1164,93 @@ GPR_D void Sigma0(const double *Q, const Prim<false> &s, double *S) {
 GPR_D void dsigma0(const double *Q, const Prim<false> &s, const DevPar &P, double *sr,
                    double *Pi1) {
   double r = s.r;
-  double dcs2 = P.beta / r * s.cs2;
   sigma_col<false>(Q, s, 0, sr);
-  double f = 1.0 / r + dcs2 / s.cs2;
+  double f = (1.0 + P.beta) * s.ir;  // 1 / rho + (d cs2 / d rho) / cs2
   for (int i = 0; i < 3; i++)
     sr[i] *= f;
   const double *A = Q + 5;
-  double G[9], ret[9];
+  const double G0[3] = {s.G[0], s.G[3], s.G[4]}, w = -r * s.cs2;
   for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++)
-      G[3 * i + j] = A[i] * A[j] + A[3 + i] * A[3 + j] + A[6 + i] * A[6 + j];
-  for (int k = 0; k < 9; k++)
-    ret[k] = s.AdG[k];
-  for (int i = 0; i < 3; i++)
-    ret[3 * i] *= 2.0;
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++)
-      ret[3 * i + j] += 1.0 / 3.0 * A[3 * i] * G[j];
-  for (int k = 0; k < 9; k++)
-    ret[k] += G[0] * A[k];
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++)
-      Pi1[3 * i + j] = -r * s.cs2 * ret[3 * j + i];
+    for (int j = 0; j < 3; j++) {
+      double ret = (j == 0 ? 2.0 : 1.0) * s.AdG[3 * i + j];
+      ret = fma(1.0 / 3.0 * A[3 * i], G0[j], ret);
+      Pi1[3 * j + i] = w * fma(s.G[0], A[3 * i + j], ret);
+    }
 }
 
-// c_0 (waves/speeds.cpp:8-18).
-GPR_D double c0_of(const Prim<false> &s, const DevPar &P) {
-  double r = s.r, G = s.e.G, dG = s.e.dG;
-  double dedrho = s.e.der - (s.e.dpr * r * G + (G + r * dG) * (s.p - s.e.pr)) /
-                                ((r * G) * (r * G));
-  double dcs2 = P.beta / r * s.cs2;
-  double dC0 = (1.0 - P.beta / G) * dcs2 + P.beta / (G * G) * dG * s.cs2;
-  double dEdr = dedrho + dC0 / 4.0 * s.devGsq;
-  double dedp = 1.0 / (r * G);
-  return sqrt((s.p / (r * r) - dEdr) / dedp);
+// c_0^2 (waves/speeds.cpp:8-18).
+GPR_D double c0sq_of(const Prim<false> &s, const DevPar &P) {
+  double r = s.r, G = s.e.G, dG = s.e.dG, rG = r * G, irG = s.irG;
+  double dedrho = s.e.der - (s.e.dpr * rG + (G + r * dG) * (s.p - s.e.pr)) * (irG * irG);
+  double iG = r * irG;
+  double dcs2 = P.beta * s.ir * s.cs2;
+  double dC0 = (1.0 - P.beta * iG) * dcs2 + P.beta * (iG * iG) * dG * s.cs2;
+  double dEdr = dedrho + dC0 * 0.25 * s.devGsq;
+  return (s.p * (s.ir * s.ir) - dEdr) * rG;
 }
 
 // The first three columns of riemann_constraints (riemann.cpp:79-154) for
 // the non-thermal system; rows 0-4 are X, rows 11-13 -sgn Y0 Xi1 X, the rest
 // zero (the other columns multiply zero coefficients in star_stepper).
 // Rx is [5][3], Ry is [3][3].
-GPR_D bool constraints(const double *Q, double sgn, const DevPar &P, double *Rx, double *Ry) {
-  Prim<false> s;
-  prim<false>(Q, P, s);
-  double r = s.r;
+//
+// X solves the reference's 5 x 5 system: with y = its rows 2-4 (the
+// distortion's first column), the two lower rows say (rho, p) = BA y, BA =
+// (rho, 0, 0; sigma0 - rho sigma_r + rho c0^2 e0) A^-1, whatever regular
+// matrix the reference multiplies them by, and the upper ones become (-Pi1 -
+// sigma_r BA0 + e0 BA1) y = I: one 3 x 3 inverse, singular where the
+// reference's 2 x 2 factor Z or Pi1 is.
+GPR_D bool constraints(const double *Q, const Prim<false> &s, double sgn, const DevPar &P,
+                       double *Rx, double *Ry) {
+  const double r = s.r, ir = s.ir;
   const double *A = Q + 5;
-  double sr[3], Pi1[9], Pi1i[9], Ai[9], sg[3];
+  double sr[3], Pi1[9], sg[3];
   dsigma0(Q, s, P, sr, Pi1);
   sigma_col<false>(Q, s, 0, sg);
-  if (!inv3(A, Ai) || !inv3(Pi1, Pi1i))
-    return false;
-  double tmp[25];
-  for (int k = 0; k < 25; k++)
-    tmp[k] = 0.0;
+  const double x1[3] = {fma(r, c0sq_of(s, P), fma(-r, sr[0], sg[0])), fma(-r, sr[1], sg[1]),
+                        fma(-r, sr[2], sg[2])};
+  double At[9], BA[6];  // BA^T = A^-T (rho e0, x1)
   for (int i = 0; i < 3; i++) {
-    tmp[5 * i] = -sr[i];
     for (int j = 0; j < 3; j++)
-      tmp[5 * i + 2 + j] = -Pi1[3 * i + j];
+      At[3 * i + j] = A[3 * j + i];
+    BA[2 * i] = i == 0 ? r : 0.0;
+    BA[2 * i + 1] = x1[i];
   }
-  tmp[1] = 1.0;
-  double c0 = c0_of(s, P);
-  double B[6] = {r, 0.0, 0.0, 0.0, 0.0, 0.0};
-  for (int j = 0; j < 3; j++)
-    B[3 + j] = sg[j] - r * sr[j];
-  B[3] += r * c0 * c0;
-  double C[6];
-  for (int i = 0; i < 3; i++) {
-    C[2 * i] = -(Pi1i[3 * i] * sr[0] + Pi1i[3 * i + 1] * sr[1] + Pi1i[3 * i + 2] * sr[2]);
-    C[2 * i + 1] = Pi1i[3 * i];
-  }
-  double BA[6];
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 3; j++)
-      BA[3 * i + j] = B[3 * i] * Ai[j] + B[3 * i + 1] * Ai[3 + j] + B[3 * i + 2] * Ai[6 + j];
-  double Z[4];
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 2; j++)
-      Z[2 * i + j] = (i == j ? 1.0 : 0.0) -
-                     (BA[3 * i] * C[j] + BA[3 * i + 1] * C[2 + j] + BA[3 * i + 2] * C[4 + j]);
-  double dz = Z[0] * Z[3] - Z[1] * Z[2];
-  if (dz == 0.0)
+  if (!gauss<3, 2>(At, BA))
     return false;
-  double Zi[4] = {Z[3] / dz, -Z[1] / dz, -Z[2] / dz, Z[0] / dz};
-  for (int i = 0; i < 2; i++)
-    for (int j = 0; j < 5; j++) {
-      double w0 = j == 0 ? 1.0 : (j == 1 ? 0.0 : -BA[j - 2]);
-      double w1 = j == 0 ? 0.0 : (j == 1 ? 1.0 : -BA[3 + j - 2]);
-      tmp[5 * (3 + i) + j] = Zi[2 * i] * w0 + Zi[2 * i + 1] * w1;
-    }
-  for (int i = 0; i < 5; i++)
-    for (int j = 0; j < 3; j++)
-      Rx[3 * i + j] = i == j ? 1.0 : 0.0;
-  if (!gauss<5, 3>(tmp, Rx))
-    return false;
-  // Xi1 (3 x 5) and Xi2 (5 x 3) of system/eig.cpp:8-53 along x
-  double X1[15], X2[15], Xi[9], Y0[9];
-  for (int k = 0; k < 15; k++)
-    X1[k] = X2[k] = 0.0;
-  X1[1] = 1.0 / r;
-  for (int i = 0; i < 3; i++) {
-    X1[5 * i] = -1.0 / r * sr[i];
-    for (int j = 0; j < 3; j++)
-      X1[5 * i + 2 + j] = -1.0 / r * Pi1[3 * i + j];
-  }
-  X2[0] = r;
-  X2[3] = r * c0 * c0;
-  for (int j = 0; j < 3; j++)
-    X2[3 + j] += sg[j] - r * sr[j];
-  for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++)
-      X2[3 * (2 + i) + j] = A[3 * i + j];
+  double N[9], y[9];
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) {
-      double t = 0.0;
-      for (int k = 0; k < 5; k++)
-        t += X1[5 * i + k] * X2[3 * k + j];
-      Xi[3 * i + j] = t;
+      N[3 * i + j] = fma(-sr[i], BA[2 * j], -Pi1[3 * i + j]);
+      if (i == 0)
+        N[j] += BA[2 * j + 1];
+      y[3 * i + j] = i == j ? 1.0 : 0.0;
     }
-  if (!eig3_real_positive(Xi) || !inv_sqrt3(Xi, Y0))
+  if (!gauss<3, 3>(N, y))
     return false;
-  double X1X[9];
+  for (int j = 0; j < 3; j++) {
+    for (int i = 0; i < 2; i++)
+      Rx[3 * i + j] = BA[i] * y[j] + BA[2 + i] * y[3 + j] + BA[4 + i] * y[6 + j];
+    for (int i = 0; i < 3; i++)
+      Rx[3 * (2 + i) + j] = y[3 * i + j];
+  }
+  // Xi1 Xi2 and Xi1 X of system/eig.cpp:8-53 along x, without Xi1's and Xi2's
+  // zeros: Xi1 = (-sigma_r, e0, -Pi1) / rho
+  double Xi[9], Y0[9], X1X[9];
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++) {
-      double t = 0.0;
-      for (int k = 0; k < 5; k++)
-        t += X1[5 * i + k] * Rx[3 * k + j];
-      X1X[3 * i + j] = t;
+      double t = Pi1[3 * i] * A[j] + Pi1[3 * i + 1] * A[3 + j] + Pi1[3 * i + 2] * A[6 + j];
+      double u = Pi1[3 * i] * y[j] + Pi1[3 * i + 1] * y[3 + j] + Pi1[3 * i + 2] * y[6 + j];
+      u = fma(sr[i], Rx[j], u);
+      if (i == 0) {
+        t -= x1[j];
+        u -= Rx[3 + j];
+      }
+      Xi[3 * i + j] = j == 0 ? fma(-ir, t, -sr[i]) : -ir * t;
+      X1X[3 * i + j] = -ir * u;
     }
+  if (!spectrum_positive(Xi) || !inv_sqrt3(Xi, Y0))
+    return false;
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++)
       Ry[3 * i + j] = -sgn * (Y0[3 * i] * X1X[j] + Y0[3 * i + 1] * X1X[3 + j] +
@@ -1259,10 +1261,8 @@ GPR_D bool constraints(const double *Q, double sgn, const DevPar &P, double *Rx,
 // Cvec_to_Pvec + P += R c + Pvec_to_Cvec (functions/vectors.cpp:85-154,
 // riemann.cpp:191-200) for the non-thermal layout
 // P = [rho, p, A(:,0), A(:,1), A(:,2), v, phi].
-GPR_D void apply_correction(double *Q, const double *Rx, const double *Ry, const double *cc,
-                            const DevPar &P) {
-  Prim<false> s;
-  prim<false>(Q, P, s);
+GPR_D void apply_correction(double *Q, const Prim<false> &s, const double *Rx,
+                            const double *Ry, const double *cc, const DevPar &P) {
   double Pv[14];
   Pv[0] = Q[0];
   Pv[1] = s.p;
@@ -1288,131 +1288,132 @@ GPR_D void apply_correction(double *Q, const double *Rx, const double *Ry, const
   Q[3] = r * v1;
   Q[4] = r * v2;
   // total_energy (energy/eos.cpp:43-47)
-  double ir = 1.0 / r;
+  const double ir = rcp64(r);
   EosRho e = eos_rho(r, ir, P);
-  double cs2 = P.beta == 0.0 ? P.b02 : P.b02 * pow(r * P.ir0, P.beta);
-  double C0 = (1.0 - P.beta / e.G) * cs2;
+  double C0q = P.b02q;  // C_0 / 4, as prim() forms it
+  if (P.has_beta) {
+    const double cs2 = P.b02 * pow(r * P.ir0, P.beta);
+    C0q = 0.25 * ((P.EOS == 1 ? (1.0 - P.beta / e.G) : P.C0f) * cs2);
+  }
   double G00 = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
   double G11 = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
   double G22 = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
   double G01 = A[0] * A[3] + A[1] * A[4] + A[2] * A[5];
   double G02 = A[0] * A[6] + A[1] * A[7] + A[2] * A[8];
   double G12 = A[3] * A[6] + A[4] * A[7] + A[5] * A[8];
-  double t = (G00 + G11 + G22) / 3.0;
+  double t = (G00 + G11 + G22) * (1.0 / 3.0);
   double dg = (G00 - t) * (G00 - t) + (G11 - t) * (G11 - t) + (G22 - t) * (G22 - t) +
               2.0 * (G01 * G01 + G02 * G02 + G12 * G12);
-  double E = e.er + (p - e.pr) / (r * e.G) + 0.5 * (v0 * v0 + v1 * v1 + v2 * v2) +
-             C0 / 4.0 * dg;
+  const double irG = P.EOS == 1 ? P.iG : ir * P.iG;
+  double E = e.er + (p - e.pr) * irG + 0.5 * (v0 * v0 + v1 * v1 + v2 * v2) + C0q * dg;
   Q[1] = r * E;
-}
-
-constexpr double STAR_TOL = 1e-8;  // options.h:22
-
-// check_star_convergence (riemann.cpp:26-77), slip conditions.
-GPR_D bool star_converged(const double *QL, const double *QR, const DevPar &PL,
-                          const DevPar &PR) {
-  Prim<false> sl;
-  prim<false>(QL, PL, sl);
-  double SL[3];
-  Sigma0(QL, sl, SL);
-  if (PR.EOS > -1) {
-    Prim<false> sr;
-    prim<false>(QR, PR, sr);
-    double SR[3];
-    Sigma0(QR, sr, SR);
-    double r0 = fmin(PL.rho0, PR.rho0), b02 = fmin(PL.b02, PR.b02);
-    return fabs(SL[0] - SR[0]) / (b02 * r0) < STAR_TOL &&
-           fabs(QL[2] / QL[0] - QR[2] / QR[0]) / sqrt(b02) < STAR_TOL;
-  }
-  double mx = fmax(fabs(SL[0]), fmax(fabs(SL[1]), fabs(SL[2])));
-  return mx / (PL.b02 * PL.rho0) < STAR_TOL;
-}
-
-// star_stepper (riemann.cpp:156-201) with slip_bcs (conditions.cpp:31-64).
-GPR_D bool star_step(double *QL, double *QR, const DevPar &PL, const DevPar &PR) {
-  double RLx[15], RLy[9], cL[3];
-  if (!constraints(QL, 1.0, PL, RLx, RLy))
-    return false;
-  Prim<false> sl;
-  prim<false>(QL, PL, sl);
-  double xL[3];
-  Sigma0(QL, sl, xL);
-  if (PR.EOS > -1) {
-    double RRx[15], RRy[9], xR[3], cR[3];
-    if (!constraints(QR, -1.0, PR, RRx, RRy))
-      return false;
-    Prim<false> sr;
-    prim<false>(QR, PR, sr);
-    Sigma0(QR, sr, xR);
-    double yL = QL[2] / QL[0], yR = QR[2] / QR[0];
-    // row 11 of the constraint matrices (the normal velocity)
-    double dL = RLy[0] * xL[0] + RLy[1] * xL[1] + RLy[2] * xL[2];
-    double dR = RRy[0] * xR[0] + RRy[1] * xR[1] + RRy[2] * xR[2];
-    double x0 = (yR - yL + dL - dR) / (RLy[0] - RRy[0]);
-    double xs[3] = {x0, 0.0, 0.0};
-    for (int i = 0; i < 3; i++) {
-      cL[i] = xs[i] - xL[i];
-      cR[i] = xs[i] - xR[i];
-    }
-    apply_correction(QR, RRx, RRy, cR, PR);
-  } else {
-    for (int i = 0; i < 3; i++)
-      cL[i] = -xL[i];
-    for (int k = 0; k < 14; k++)
-      QR[k] = 0.0;
-  }
-  apply_correction(QL, RLx, RLy, cL, PL);
-  return true;
 }
 
 // left_star_state (riemann.cpp:203-233): the left star state of the
 // interface Riemann problem between QL (material PL) and QR (material PR)
-// along the unit normal n: at most ten linearised steps, each after a half
-// step dt/2 of the stiff relaxation; the input is returned if a NaN appears.
-// The level set entry (index 14) is carried through unchanged.
-GPR_D void left_star_state(const double *QL0, const double *QR0, const DevPar &PL,
-                           const DevPar &PR, double dt, const double n[2], int nd,
-                           double *out) {
-  double QL[15], QR[15], R[3][3];
-  for (int k = 0; k < 15; k++) {
-    QL[k] = QL0[k];
-    QR[k] = QR0[k];
-  }
-  rotation(n, nd, R);
-  rotate(QL, R);
-  rotate(QR, R);
-  bool nan = false;
-  for (int count = 0; count < 10 && !star_converged(QL, QR, PL, PR); count++) {
-    // ode_stepper_analytic (relaxation/analytic.cpp:152-161), no heat flux
-    QL[2] += PL.dp0 * dt / 2;
-    QL[3] += PL.dp1 * dt / 2;
-    QL[4] += PL.dp2 * dt / 2;
-    ode_distortion(QL, dt / 2, PL);
-    if (PR.EOS > -1) {
-      QR[2] += PR.dp0 * dt / 2;
-      QR[3] += PR.dp1 * dt / 2;
-      QR[4] += PR.dp2 * dt / 2;
-      ode_distortion(QR, dt / 2, PR);
-    }
-    if (!star_step(QL, QR, PL, PR)) {
-      nan = true;
-      break;
-    }
-  }
+// along the unit normal n: at most ten linearised steps (star_stepper,
+// riemann.cpp:156-201, slip_bcs, conditions.cpp:31-64), each after a half
+// step dt/2 of the stiff relaxation, until check_star_convergence
+// (riemann.cpp:26-77) holds; the input is returned if a NaN appears.  The
+// level set entry (index 14) is carried through unchanged.
+//
+// Two neighbouring lanes work on one problem, the even one on the left
+// state and the odd one on the right (each lane's Q0, P its own; EOS, rho0
+// and b02 of the other side's material): the sides meet in one normal
+// velocity and stress per step.  An interface of the 800 x 400 bubble has
+// ~1000 problems, a few warps for 608 schedulers, so a launch lasts as long
+// as one problem's chain of FP64 instructions (64 cycles each): 1.2 ms with
+// one lane per problem, eliminations with a division per entry, two more of
+// them and a matrix root of 18 inverses per side and step; 0.27 ms now.  Every lane of the
+// warp calls it (live: the pair has a problem); the even lane writes out.
+constexpr double STAR_TOL = 1e-8;  // options.h:22
+GPR_D void left_star_pair(const double *Q0, const DevPar &P, int oEOS, double orho0, double ob02,
+                          double dt, const double n[2], int nd, bool live, double *out) {
+  const bool right = threadIdx.x & 1;
+  const bool two = (right ? P.EOS : oEOS) > -1;  // the right side is a material
+  const bool work = live && (two || !right);
+  const double r0 = fmin(P.rho0, orho0), b02 = fmin(P.b02, ob02);
+  double Q[15], R[3][3];
   for (int k = 0; k < 15; k++)
-    nan = nan || isnan(QL[k]);
-  if (nan) {
+    Q[k] = work ? Q0[k] : 0.0;
+  rotation(n, nd, R);
+  rotate(Q, R);
+  bool open = live, bad = false;
+  for (int count = 0; count < 10; count++) {
+    double S[3] = {0.0, 0.0, 0.0}, y = 0.0;
+    if (open && work) {
+      Prim<false> s;
+      prim<false>(Q, P, s);
+      Sigma0(Q, s, S);
+      y = s.v[0];
+    }
+    const double So = __shfl_xor_sync(0xffffffffu, S[0], 1);
+    const double yo = __shfl_xor_sync(0xffffffffu, y, 1);
+    bool conv;
+    if (two)
+      conv = fabs(S[0] - So) < STAR_TOL * (b02 * r0) && fabs(y - yo) < STAR_TOL * sqrt64(b02);
+    else
+      conv = fmax(fabs(S[0]), fmax(fabs(S[1]), fabs(S[2]))) < STAR_TOL * (P.b02 * P.rho0);
+    // (the left lane decides: with one material only it has the stress)
+    conv = (__ballot_sync(0xffffffffu, conv) >> (threadIdx.x & 30u)) & 1u;
+    open = open && !conv;
+    if (!__any_sync(0xffffffffu, open))
+      break;
+    const bool step = open && work;
+    double Rx[15], Ry[9], x[3] = {0.0, 0.0, 0.0}, d = 0.0, Ry0 = 0.0;
+    bool ok = true;
+    Prim<false> s;
+    y = 0.0;
+    if (step) {
+      // ode_stepper_analytic (relaxation/analytic.cpp:152-161), no heat flux
+      Q[2] += P.dp0 * dt * 0.5;
+      Q[3] += P.dp1 * dt * 0.5;
+      Q[4] += P.dp2 * dt * 0.5;
+      ode_distortion(Q, dt * 0.5, P);
+      prim<false>(Q, P, s);
+      ok = constraints(Q, s, right ? -1.0 : 1.0, P, Rx, Ry);
+      Sigma0(Q, s, x);
+      y = s.v[0];
+      // row 11 of the constraint matrices (the normal velocity)
+      if (ok) {
+        d = Ry[0] * x[0] + Ry[1] * x[1] + Ry[2] * x[2];
+        Ry0 = Ry[0];
+      }
+    }
+    const double yq = __shfl_xor_sync(0xffffffffu, y, 1);
+    const double dq = __shfl_xor_sync(0xffffffffu, d, 1);
+    const double Rq = __shfl_xor_sync(0xffffffffu, Ry0, 1);
+    const bool okq = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
+    if (open && !(ok && okq)) {
+      bad = true;
+      open = false;
+    }
+    if (open && work) {
+      double cc[3] = {-x[0], -x[1], -x[2]};
+      if (two) {
+        // (yR - yL + dL - dR) / (RL - RR), the same number from either side
+        const double num = right ? (y - yq) + (dq - d) : (yq - y) + (d - dq);
+        cc[0] = num / (right ? Rq - Ry0 : Ry0 - Rq) - x[0];
+      }
+      apply_correction(Q, s, Rx, Ry, cc, P);
+    }
+  }
+  if (right || !live)
+    return;
+  for (int k = 0; k < 15; k++)
+    bad = bad || isnan(Q[k]);
+  if (bad) {
     for (int k = 0; k < 15; k++)
-      out[k] = QL0[k];
+      out[k] = Q0[k];
     return;
   }
   double RT[3][3];
   for (int i = 0; i < 3; i++)
     for (int j = 0; j < 3; j++)
       RT[i][j] = R[j][i];
-  rotate(QL, RT);
+  rotate(Q, RT);
   for (int k = 0; k < 15; k++)
-    out[k] = QL[k];
+    out[k] = Q[k];
 }
 
 // ===========================================================================
@@ -1623,41 +1624,47 @@ __global__ void k_plan_levels(const int *__restrict__ nplan, const int32_t *__re
   }
 }
 
+// The star state of plan entry k, by two lanes (left_star_pair): every lane of
+// the warp calls it, live where the pair has an entry.
 template <int V>
-GPR_D void solve_plan(int k, const BPlan *plan, const int32_t *dep, const double *grid,
-                      double *star, const DevPar &P0, const DevPar &P1, int mat, double dt,
-                      int nd) {
+GPR_D void solve_plan(int k, bool live, const BPlan *plan, const int32_t *dep,
+                      const double *grid, double *star, const DevPar &P0, const DevPar &P1,
+                      int mat, double dt, int nd) {
   static_assert(V == 15, "the ghost fill is for the viscous one-level-set layout");
-  const BPlan &b = plan[k];
-  double QL[V], QR[V], out[V];
-  for (int v = 0; v < V; v++)
-    QL[v] = grid[(long)b.ql * V + v];
-  int dk = dep[k];
-  for (int v = 0; v < V; v++)
-    QR[v] = dk >= 0 && v < V - 1 ? star[(long)dk * V + v] : grid[(long)b.R * V + v];
-  const DevPar &PL = mat == 0 ? P0 : P1;
-  const DevPar &PR = b.miR == 0 ? P0 : P1;
-  left_star_state(QL, QR, PL, PR, dt, b.n, nd, out);
-  for (int v = 0; v < V; v++)
-    star[(long)k * V + v] = out[v];
+  const BPlan &b = plan[live ? k : 0];
+  const bool right = threadIdx.x & 1;
+  const int miR = live ? b.miR : 0, dk = live ? dep[k] : -1;
+  const DevPar &P = (right ? miR : mat) == 0 ? P0 : P1;
+  const DevPar &O = (right ? mat : miR) == 0 ? P0 : P1;
+  double Q[V], n[2] = {1.0, 0.0};
+  if (live) {
+    const double *src = grid + (long)(right ? b.R : b.ql) * V;
+    for (int v = 0; v < V; v++)
+      Q[v] = right && dk >= 0 && v < V - 1 ? star[(long)dk * V + v] : src[v];
+    n[0] = b.n[0];
+    n[1] = b.n[1];
+  }
+  left_star_pair(Q, P, O.EOS, O.rho0, O.b02, dt, n, nd, live, star + (long)(live ? k : 0) * V);
 }
 
 // Star states of the plan entries on level 0 (all independent).
 template <int V>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(32)
     k_star_level0(const BPlan *__restrict__ plan, const int *__restrict__ nplan,
                   const int32_t *__restrict__ dep, const int32_t *__restrict__ level,
-                  const double *__restrict__ grid, double *__restrict__ star, DevPar P0,
-                  DevPar P1, int mat, double dt, const double *__restrict__ dt_dev, int nd,
-                  const double *__restrict__ clk) {
+                  const double *grid, double *star, DevPar P0, DevPar P1, int mat, double dt,
+                  const double *__restrict__ dt_dev, int nd, const double *__restrict__ clk) {
   if (clk && clk[0] >= clk[2])
     return;
   if (dt_dev)
     dt = *dt_dev;
-  int B = *nplan;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < B; k += gridDim.x * blockDim.x)
-    if (level[k] == 0)
-      solve_plan<V>(k, plan, dep, grid, star, P0, P1, mat, dt, nd);
+  const int B = *nplan;
+  for (int k0 = blockIdx.x * 16; k0 < B; k0 += gridDim.x * 16) {
+    const int k = k0 + (int)(threadIdx.x >> 1);
+    const bool live = k < B && level[k] == 0;
+    if (__any_sync(0xffffffffu, live))
+      solve_plan<V>(k, live, plan, dep, grid, star, P0, P1, mat, dt, nd);
+  }
 }
 
 // Deeper levels, in order, in one block (rare: only where a boundary cell's
@@ -1666,18 +1673,21 @@ template <int V>
 __global__ void __launch_bounds__(64)
     k_star_levels(const BPlan *__restrict__ plan, const int *__restrict__ nplan,
                   const int32_t *__restrict__ dep, const int32_t *__restrict__ level,
-                  const int *__restrict__ maxlevel, const double *__restrict__ grid,
-                  double *__restrict__ star, DevPar P0, DevPar P1, int mat, double dt,
-                  const double *__restrict__ dt_dev, int nd, const double *__restrict__ clk) {
+                  const int *__restrict__ maxlevel, const double *grid, double *star, DevPar P0,
+                  DevPar P1, int mat, double dt, const double *__restrict__ dt_dev, int nd,
+                  const double *__restrict__ clk) {
   if (clk && clk[0] >= clk[2])
     return;
   if (dt_dev)
     dt = *dt_dev;
-  int B = *nplan, ML = *maxlevel;
+  const int B = *nplan, ML = *maxlevel;
   for (int L = 1; L <= ML; L++) {
-    for (int k = threadIdx.x; k < B; k += blockDim.x)
-      if (level[k] == L)
-        solve_plan<V>(k, plan, dep, grid, star, P0, P1, mat, dt, nd);
+    for (int k0 = 0; k0 < B; k0 += 32) {
+      const int k = k0 + (int)(threadIdx.x >> 1);
+      const bool live = k < B && level[k] == L;
+      if (__any_sync(0xffffffffu, live))
+        solve_plan<V>(k, live, plan, dep, grid, star, P0, P1, mat, dt, nd);
+    }
     __syncthreads();
   }
 }
@@ -1911,14 +1921,16 @@ __global__ void k_renorm_multi(double *__restrict__ u, long ncell, double r00, d
 
 // Pointwise left_star_state for tests and the system.multi binding.
 template <int V>
-__global__ void k_star_pointwise(const double *__restrict__ QL, const double *__restrict__ QR,
-                                 const double *__restrict__ nrm, double *__restrict__ out,
+__global__ void k_star_pointwise(const double *QL, const double *QR,
+                                 const double *__restrict__ nrm, double *out,
                                  long count, int nd, double dt, DevPar PL, DevPar PR) {
-  long k = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (k >= count)
-    return;
-  double n[2] = {nrm[k * nd], nd == 2 ? nrm[k * nd + 1] : 0.0};
-  left_star_state(QL + k * V, QR + k * V, PL, PR, dt, n, nd, out + k * V);
+  const long k = blockIdx.x * (long)(blockDim.x / 2) + (threadIdx.x >> 1);
+  const bool live = k < count, right = threadIdx.x & 1;
+  const long kk = live ? k : 0;
+  double n[2] = {nrm[kk * nd], nd == 2 ? nrm[kk * nd + 1] : 0.0};
+  const DevPar &P = right ? PR : PL, &O = right ? PL : PR;
+  left_star_pair((right ? QR : QL) + kk * V, P, O.EOS, O.rho0, O.b02, dt, n, nd, live,
+                 out + kk * V);
 }
 
 }  // namespace multi
