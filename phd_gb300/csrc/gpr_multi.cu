@@ -670,7 +670,7 @@ static int iterate_multi(double *u, const int32_t *nX, int ndim, const double *d
           return rc;
         continue;
       }
-      if ((rc = Ops<L15>::weno(wh, ub, nX, ndim, tmp, st)))
+      if ((rc = Ops<L15>::weno(wh, ub, nX, ndim, tmp, st, maskb)))
         return rc;
       if ((rc = Ops<L15>::predictor(qh, wh, 0.0, dt_dev, dX, ndim, nX, stiff, P[m], maskb, pst,
                                     st, tmp)))

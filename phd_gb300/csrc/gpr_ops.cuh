@@ -179,8 +179,9 @@ template <class L> struct Ops {
     return (long)(nX[0] + 2) * (nX[1] + 2 * NN) * NN * V;
   }
 
+  // mask (2D, optional): only these predictor cells are reconstructed
   static int weno(double *wh, const double *ub, const int32_t *nX, int nd, double *scratch,
-                  cudaStream_t st) {
+                  cudaStream_t st, const uint8_t *mask = nullptr) {
     const Consts &C = consts();
     if (nd == 1) {
       int ncb = nX[0] + 2;
@@ -192,7 +193,7 @@ template <class L> struct Ops {
     int nxp = nX[0] + 2, nyp = nX[1] + 2;
     const int tj = weno2d_tile(nyp);
     const long nblk = (long)nxp * ((nyp + tj - 1) / tj);
-    k_weno2d<V><<<(unsigned)nblk, WENO2_THREADS, 0, st>>>(wh, ub, nxp, nyp, tj, C);
+    k_weno2d<V><<<(unsigned)nblk, WENO2_THREADS, 0, st>>>(wh, ub, nxp, nyp, tj, C, mask);
     return cuda_rc();
   }
 
@@ -482,7 +483,7 @@ template <class L> struct Ops {
       int rc = boundaries(u, ub, nX, nd, bcs, st);
       if (rc)
         return rc;
-      rc = weno(wh, ub, nX, nd, tmp, st);
+      rc = weno(wh, ub, nX, nd, tmp, st, mask);
       if (rc)
         return rc;
       // tmp (the FV face buffers, used after the predictor) holds the
@@ -549,7 +550,7 @@ template <class L> struct Ops {
     // the half steps on u and ub in one launch
     k_ode<L><<<GPR_SPREAD(ncell + nub, 128), 0, st>>>(u, ncell, dt / 2, dt_dev, 0.5, P, ub,
                                                        nub);
-    int rc = weno(wh, ub, nX, nd, tmp, st);
+    int rc = weno(wh, ub, nX, nd, tmp, st, mask);
     if (rc)
       return rc;
     if (half_step && (rc = midstep(wh, dt, dt_dev, dX, nd, nX, P, mask, st)))
