@@ -491,14 +491,14 @@ GPR_D void shfl_vec(const double *src, double *dst, int lanemask) {
 // and the quotient goes into the coefficient (sign by the lane's end).
 // hx, hy: 1 / (dx (x1 - x0)), 1 / (dy (x1 - x0)).  The spatial partners are the
 // lanes g ^ XB (x) and g ^ YB (y) in every lane layout that calls it.
+// s receives q's primitive variables.
 template <class L, int ND, bool SOURCE = true>
 GPR_D void dg_residual(const double *q, double *r, double sg, int i, int j, double hx, double hy,
-                       const DevPar &P) {
+                       const DevPar &P, Prim<L::THERMAL> &s) {
   constexpr int V = L::V;
   // lane bit layout: 1D g = 2t + i ; 2D g = 4t + 2i + j
   constexpr int XB = ND == 1 ? 1 : 2;  // flips i
   constexpr int YB = 1;                // flips j (2D)
-  Prim<L::THERMAL> s;
   prim<L::THERMAL>(q, P, s);
   if (SOURCE) {
     source<L::THERMAL, V>(q, s, P, r, sg);
@@ -532,6 +532,13 @@ GPR_D void dg_residual(const double *q, double *r, double sg, int i, int j, doub
       if (flux_support<L::THERMAL>(k, d))
         r[k] = fma(-c, __shfl_xor_sync(0xffffffffu, F[k], lm) - F[k], r[k]);
   }
+}
+
+template <class L, int ND, bool SOURCE = true>
+GPR_D void dg_residual(const double *q, double *r, double sg, int i, int j, double hx, double hy,
+                       const DevPar &P) {
+  Prim<L::THERMAL> s;
+  dg_residual<L, ND, SOURCE>(q, r, sg, i, j, hx, hy, P, s);
 }
 
 // The Picard map at this node, q_new(t, s) = sum_m DG_MATinv[t][m] (ENDVALS[0][m]
@@ -899,7 +906,7 @@ GPR_D void stiff_jacobian_rows(const double *q, const Prim<TH> &s, const DevPar 
   double dA = det3(A);
   int newtonian = !(P.flags & (GPR_SOLID | GPR_POWER_LAW | GPR_BINGHAM));
   double th = theta1inv<TH>(q, s, P);
-  double id = 1.0 / dA;
+  double id = rcp64(dA);
   double Ai[9];  // A^-1
   Ai[0] = (A[4] * A[8] - A[5] * A[7]) * id;
   Ai[1] = (A[2] * A[7] - A[1] * A[8]) * id;
@@ -1042,6 +1049,7 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
   const unsigned gmask = ((NP == 32) ? 0xffffffffu : ((1u << NP) - 1u)) << (lane & ~(NP - 1u));
   const double f = C.endv[0][t];
   const double M0 = C.dgmat[t][t], M1 = C.dgmat[t][1 - t];
+  const float tolf = (float)C.stiff_tol;
   const long cells_per_block = blockDim.x / NP;
   // persistent: blocks stride over the cells; the loop bound is uniform in
   // the block so every lane takes part in the warp-level exchanges
@@ -1075,7 +1083,8 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
     for (int it = 0; it < C.stiff_it; it++) {
       if (__all_sync(0xffffffffu, done))
         break;
-      dg_residual<L, ND>(q, r, a_t, i, j, hx, hy, P);
+      Prim<L::THERMAL> st;
+      dg_residual<L, ND>(q, r, a_t, i, j, hx, hy, P, st);
       // the fixed point's residual over W_s: r + ENDVALS[0][t] w - sum_m
       // DG_MAT[t][m] q(m)
       shfl_vec<V>(q, other, TB);
@@ -1083,8 +1092,6 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
       for (int k = 0; k < V; k++)
         r[k] += fma(-M1, other[k], fma(-M0, q[k], fw[k]));
       if (!done) {
-        Prim<L::THERMAL> st;
-        prim<L::THERMAL>(q, P, st);
         // this time node's diagonal block A_t = M_tt I - a_t dS/dA of the
         // 18 x 18 Newton matrix (the off-diagonal blocks are M_t,1-t I) and
         // its right-hand side
@@ -1196,18 +1203,32 @@ __global__ void __launch_bounds__(64) k_predictor_stiff(
         }
       }
       __syncwarp();
-      bool big = false, bad = !solved;
+      // |delta| > stiff_tol (1 + |qn|), in FP32 from the high words wherever the
+      // sides differ by more than 1e-5, as the Picard pass's test
+      bool big = false, open = false, bad = !solved;
 #pragma unroll
       for (int k = 0; k < V; k++) {
-        double qn = q[k] + delta[k];
-        if (fabs(delta[k]) > C.stiff_tol * (1.0 + fabs(qn)))
-          big = true;
-        if (qn != qn)
-          bad = true;
+        const double qn = q[k] + delta[k];
+        const float df = f32_abs_hi(delta[k]), qf = f32_abs_hi(qn);
+        const float th = fmaf(tolf, qf, tolf);
+        const bool in = fmaxf(df, qf) < F32_TOP;
+        big = big || (in && df > th * 1.00001f);
+        open = open || !in || df > th * 0.99999f;
         if (!done)
           q[k] = qn;
       }
       unsigned bigm = __ballot_sync(0xffffffffu, big) & gmask;
+      if (open) {
+#pragma unroll
+        for (int k = 0; k < V; k++) {
+          const double qn = done ? q[k] + delta[k] : q[k];
+          if (!bigm && fabs(delta[k]) > C.stiff_tol * (1.0 + fabs(qn)))
+            big = true;
+          if (fp_abs_bits(qn) > FP_INF_BITS)
+            bad = true;
+        }
+      }
+      bigm = __ballot_sync(0xffffffffu, big) & gmask;
       unsigned badm = __ballot_sync(0xffffffffu, bad) & gmask;
       if (!done) {
         iters = it + 1;
