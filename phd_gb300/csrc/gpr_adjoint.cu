@@ -99,7 +99,7 @@ template <class L> struct Adj {
     k_adj_clock_finalize<<<blocks(ninst, 128), 128, 0, st>>>(mx, B, dt_io, dt_mode, tclk, aux,
                                                              amax);
     k_b_boundaries<V><<<GPR_SPREAD(b.nub * V, 256), 0, st>>>(u, ub, b.nub, B);
-    k_b_weno<V><<<GPR_SPREAD(b.nb * V, 256), 0, st>>>(wh, ub, b.nb, C, B);
+    k_b_weno<V><<<GPR_SPREAD(b.nb * V, 256), 0, st>>>(wh, ub, b.nb, B);
     // every iteration in the Picard kernel (no k_predictor_first): the
     // tightly converged forward the gradients and their finite-difference
     // checks difference keeps one arithmetic path

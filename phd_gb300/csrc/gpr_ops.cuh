@@ -182,10 +182,9 @@ template <class L> struct Ops {
   // mask (2D, optional): only these predictor cells are reconstructed
   static int weno(double *wh, const double *ub, const int32_t *nX, int nd, double *scratch,
                   cudaStream_t st, const uint8_t *mask = nullptr) {
-    const Consts &C = consts();
     if (nd == 1) {
       int ncb = nX[0] + 2;
-      k_weno1d<V><<<GPR_SPREAD((long)ncb * V, 256), 0, st>>>(wh, ub, ncb, C);
+      k_weno1d<V><<<GPR_SPREAD((long)ncb * V, 256), 0, st>>>(wh, ub, ncb);
       return cuda_rc();
     }
     // both sweeps in one launch through shared memory (k_weno2d); the
@@ -193,7 +192,7 @@ template <class L> struct Ops {
     int nxp = nX[0] + 2, nyp = nX[1] + 2;
     const int tj = weno2d_tile(nyp);
     const long nblk = (long)nxp * ((nyp + tj - 1) / tj);
-    k_weno2d<V><<<(unsigned)nblk, WENO2_THREADS, 0, st>>>(wh, ub, nxp, nyp, tj, C, mask);
+    k_weno2d<V><<<(unsigned)nblk, WENO2_THREADS, 0, st>>>(wh, ub, nxp, nyp, tj, mask);
     return cuda_rc();
   }
 
@@ -622,7 +621,7 @@ template <class L> struct Ops {
   }
   static void batch_weno(double *wh, const double *ub, const BatchLayout &b, const Batch &B,
                          int bs, cudaStream_t st) {
-    k_b_weno<V><<<blocks(b.nb * V, bs), bs, 0, st>>>(wh, ub, b.nb, consts(), B);
+    k_b_weno<V><<<blocks(b.nb * V, bs), bs, 0, st>>>(wh, ub, b.nb, B);
   }
   static void batch_picard_pair(double *qh, const double *wh, int32_t *status,
                                 const BatchLayout &b, const Batch &B, int bs_first,
