@@ -108,23 +108,24 @@ __global__ void k_fill_interior(const double *__restrict__ u, double *__restrict
 // copied from u, ghost cells by the boundary rule from their source cell of u
 // (the values k_fill_interior + k_ghosts give), one thread per (cell, var).
 template <int V>
-__global__ void k_boundaries1d(const double *__restrict__ u, double *__restrict__ ub, int nx,
-                               int bcl, int bcr) {
-  long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (idx >= (long)(nx + 2 * NN) * V)
-    return;
-  const int k = idx % V, p = idx / V;
-  if (p >= NN && p < nx + NN) {
-    ub[idx] = u[(long)(p - NN) * V + k];
-    return;
-  }
+GPR_D double ub_value1d(const double *__restrict__ u, int p, int k, int nx, int bcl, int bcr) {
+  if (p >= NN && p < nx + NN)
+    return u[(long)(p - NN) * V + k];
   const int side = p >= nx + NN;
   const int i = side ? p - nx - NN : p;
   int code = side ? bcr : bcl;
   const int si = bc_src_index(code, side, i, nx);
   if (code == GPR_BC_PERIODIC)
     code = GPR_BC_TRANSMISSIVE;  // plain copy
-  ub[idx] = bc_value<V>(code, 0, k, u + (long)si * V);
+  return bc_value<V>(code, 0, k, u + (long)si * V);
+}
+template <int V>
+__global__ void k_boundaries1d(const double *__restrict__ u, double *__restrict__ ub, int nx,
+                               int bcl, int bcr) {
+  long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (idx >= (long)(nx + 2 * NN) * V)
+    return;
+  ub[idx] = ub_value1d<V>(u, (int)(idx / V), (int)(idx % V), nx, bcl, bcr);
 }
 
 // Ghost rows along one axis.  For axis 0: lines are columns j (interior rows
@@ -181,9 +182,8 @@ __global__ void k_ghosts(double *__restrict__ ub, int nx, int ny, int nd, int ax
 // subtraction, which loses less on nearly constant data than those products.
 // 512 x 512: k_weno2d 1.10 to 0.51 ms.
 constexpr double WENO_X = 0.28867513459481288225;  // x_1 - 1/2 = 1 / (2 sqrt 3)
-GPR_D void weno_point(const double *__restrict__ d0, long sd, double *__restrict__ out,
-                      long so, int ind, int nx, int gap) {
-  const double a = d0[0], b = d0[sd], c = d0[2 * sd];
+GPR_D void weno_line(double a, double b, double c, double *__restrict__ out, long so, int ind,
+                     int nx, int gap) {
   const double dL = b - a, dR = c - b;
   double tL = fma(dL, dL, WENO_EPS), tR = fma(dR, dR, WENO_EPS);
   tL *= tL;
@@ -203,6 +203,10 @@ GPR_D void weno_point(const double *__restrict__ d0, long sd, double *__restrict
   out[0] = fma(-WENO_X, s, b);
   out[so] = fma(WENO_X, s, b);
 }
+GPR_D void weno_point(const double *__restrict__ d0, long sd, double *__restrict__ out,
+                      long so, int ind, int nx, int gap) {
+  weno_line(d0[0], d0[sd], d0[2 * sd], out, so, ind, nx, gap);
+}
 
 // 1D: wh[i][a][k] for i in 0..nx+1 from ub rows i..i+2 (weno.cpp:75-81, 146)
 template <int V>
@@ -213,6 +217,19 @@ __global__ void k_weno1d(double *__restrict__ wh, const double *__restrict__ ub,
   int k = idx % V;
   int i = idx / V;
   weno_point(ub + (long)i * V + k, V, wh + (long)i * NN * V + k, V, i, ncb, 0);
+}
+
+// The same straight from u, for steps that need the extended grid for nothing
+// else (one launch of ~3 us less).
+template <int V>
+__global__ void k_weno1d_u(double *__restrict__ wh, const double *__restrict__ u, int nx, int bcl,
+                           int bcr) {
+  const long idx = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (idx >= (long)(nx + 2) * V)
+    return;
+  const int k = idx % V, i = idx / V;
+  weno_line(ub_value1d<V>(u, i, k, nx, bcl, bcr), ub_value1d<V>(u, i + 1, k, nx, bcl, bcr),
+            ub_value1d<V>(u, i + 2, k, nx, bcl, bcr), wh + (long)i * NN * V + k, V, i, nx + 2, 0);
 }
 
 // 2D, both sweeps in one launch, staged in shared memory: a block takes
@@ -1686,14 +1703,46 @@ __global__ void __launch_bounds__(128) k_fv1d(
 }
 
 // ---------------------------------------------------------------------------
+// Device clock of the device-resident time loop: [t, dt, tf, cfl, count].
+// clock_dt reads t/count and writes dt from the CFL maximum (0 once t >= tf);
+// clock_step adds dt to t and counts the step.
+GPR_D void clock_dt(unsigned long long mx, double *__restrict__ clk) {
+  double t = clk[0], tf = clk[2], cfl = clk[3];
+  long count = (long)clk[4];
+  double dt = 0.0;
+  if (t < tf) {
+    double MAX = __longlong_as_double((long long)mx);
+    dt = cfl / MAX;
+    if (count <= 5)
+      dt *= 0.2;
+    if (t + dt > tf)
+      dt = tf - t;
+  }
+  clk[1] = dt;
+}
+GPR_D void clock_step(double *__restrict__ clk) {
+  if (clk[1] > 0.0) {
+    clk[0] += clk[1];
+    clk[4] += 1.0;
+  }
+}
+static __global__ void k_clock_finalize(const unsigned long long *__restrict__ mx,
+                                        double *__restrict__ clk) {
+  clock_dt(*mx, clk);
+}
+static __global__ void k_clock_advance(double *__restrict__ clk) { clock_step(clk); }
+
 // CFL time step (solvers/iterator.cpp:54-83): per-cell sum_d mae/dx_d,
 // block max, atomicMax on the bit pattern (non-negative doubles order as
 // unsigned integers); NaN cells are skipped as std::max skips them.
+// With clk the last block to finish (out[1]: the step's contortion flag, cleared
+// here, and the blocks' counter) sets the clock's dt, which saves a launch of
+// one thread (3.6 us in the 200-cell tube's step of 180).
 template <class L>
 __global__ void __launch_bounds__(256) k_cfl_max(const double *__restrict__ u, long ncell,
                                                  int nd, double idx, double idy,
                                                  unsigned long long *__restrict__ out,
-                                                 DevPar P) {
+                                                 DevPar P, double *__restrict__ clk = nullptr) {
   constexpr int V = L::V;
   long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
   double m = 0.0;
@@ -1722,6 +1771,15 @@ __global__ void __launch_bounds__(256) k_cfl_max(const double *__restrict__ u, l
     for (int w = 0; w < (int)(blockDim.x >> 5); w++)
       b = fmax(b, sm[w]);
     atomicMax(out, (unsigned long long)__double_as_longlong(b));
+    if (clk) {
+      int *flag = (int *)(out + 1), *count = flag + 1;
+      __threadfence();
+      if (atomicAdd(count, 1) == (int)gridDim.x - 1) {
+        __threadfence();
+        *flag = *count = 0;
+        clock_dt(atomicMax(out, 0ull), clk);
+      }
+    }
   }
 }
 
@@ -1734,40 +1792,6 @@ static __global__ void k_cfl_finalize(const unsigned long long *__restrict__ mx,
   if (t + dt > tf)
     dt = tf - t;
   *dt_out = dt;
-}
-
-// Device clock of the device-resident time loop: [t, dt, tf, cfl, count].
-// The CFL finalize reads t/count and writes dt (0 once t >= tf); the advance
-// kernel adds dt to t and counts the step.
-// flag (optional): the step's contortion flag, cleared here for the
-// contortion check later in the same step.
-static __global__ void k_clock_finalize(const unsigned long long *__restrict__ mx,
-                                        double *__restrict__ clk, int *__restrict__ flag = nullptr) {
-  if (flag)
-    *flag = 0;
-  double t = clk[0], tf = clk[2], cfl = clk[3];
-  long count = (long)clk[4];
-  double dt = 0.0;
-  if (t < tf) {
-    double MAX = __longlong_as_double((long long)*mx);
-    dt = cfl / MAX;
-    if (count <= 5)
-      dt *= 0.2;
-    if (t + dt > tf)
-      dt = tf - t;
-  }
-  clk[1] = dt;
-}
-
-// mx (optional): the CFL maximum, cleared here for the next step's k_cfl_max.
-static __global__ void k_clock_advance(double *__restrict__ clk,
-                                       unsigned long long *__restrict__ mx = nullptr) {
-  if (clk[1] > 0.0) {
-    clk[0] += clk[1];
-    clk[4] += 1.0;
-  }
-  if (mx)
-    *mx = 0ull;
 }
 
 // *flag = 1 if any of the n entries is a NaN (integer tests on the bit patterns).

@@ -113,12 +113,19 @@ __global__ void k_contorted(const double *__restrict__ u, long ncell, double tol
 // reset_distortion (solvers/utils.cpp:44-64) when *flag is set: every cell
 // of a non-vacuum material loses its distortion energy rho E_2A and gets
 // A = (rho / rho0)^(1/3) I.  The material is 0, or that of the level set
-// (functions/vectors.cpp:24-31) with one.
+// (functions/vectors.cpp:24-31) with one.  With clk (the step's clock, dt_dev
+// its dt) the first thread also ends the step: it advances t and the count,
+// which no thread here reads, and clears the CFL maximum mx.
 template <class L>
 __global__ void k_reset_distortion(double *__restrict__ u, long ncell,
                                    const int *__restrict__ flag, DevPar P0, DevPar P1,
-                                   const double *__restrict__ dt_dev) {
+                                   const double *__restrict__ dt_dev, double *clk = nullptr,
+                                   unsigned long long *mx = nullptr) {
   constexpr int V = L::V;
+  if (clk && blockIdx.x == 0 && threadIdx.x == 0) {
+    clock_step(clk);
+    *mx = 0ull;
+  }
   if (!*flag || (dt_dev && *dt_dev == 0.0))
     return;
   long c = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -479,12 +486,13 @@ template <class L> struct Ops {
       cudaMemsetAsync(mx, 0, 2 * sizeof(unsigned long long), st);
     for (int s = 0; s < nsteps; s++) {
       step_head(u, ncell, nd, dX, P, mx, clk, st);
-      int rc = boundaries(u, ub, nX, nd, bcs, st);
-      if (rc)
+      int rc = 0;
+      if (nd == 1) {
+        k_weno1d_u<V><<<GPR_SPREAD((nX[0] + 2L) * V, 256), 0, st>>>(wh, u, nX[0], bcs[0], bcs[1]);
+      } else if ((rc = boundaries(u, ub, nX, nd, bcs, st)) ||
+                 (rc = weno(wh, ub, nX, nd, tmp, st, mask))) {
         return rc;
-      rc = weno(wh, ub, nX, nd, tmp, st, mask);
-      if (rc)
-        return rc;
+      }
       // tmp (the FV face buffers, used after the predictor) holds the
       // predictor's deferred cells meanwhile
       rc = predictor(qh, wh, 0.0, dt_dev, dX, nd, nX, 0, P, mask, status, st, tmp);
@@ -499,15 +507,14 @@ template <class L> struct Ops {
   }
 
   // The clock kernels of a device-resident step around its stages:
-  // head = CFL maximum -> dt (and the contortion flag mx[1] cleared); tail =
-  // renorm + contortion test -> reset -> clock advance (and the CFL maximum
+  // head = CFL maximum -> dt (and the contortion flag in mx[1] cleared); tail =
+  // renorm + contortion test -> reset, clock advance (and the CFL maximum
   // mx[0] cleared for the next step).  mx[0..1] must be zero before the
   // first step.
   static void step_head(const double *u, long ncell, int nd, const double *dX, const DevPar &P,
                         unsigned long long *mx, double *clk, cudaStream_t st) {
     k_cfl_max<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, nd, 1.0 / dX[0],
-                                                      nd == 2 ? 1.0 / dX[1] : 0.0, mx, P);
-    k_clock_finalize<<<1, 1, 0, st>>>(mx, clk, (int *)(mx + 1));
+                                                      nd == 2 ? 1.0 / dX[1] : 0.0, mx, P, clk);
   }
   static void step_tail(double *u, long ncell, const DevPar &P, double tol,
                         unsigned long long *mx, double *clk, cudaStream_t st) {
@@ -515,8 +522,8 @@ template <class L> struct Ops {
     int *flag = (int *)(mx + 1);
     k_renorm_contorted<V><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, P.rho0, tol, flag,
                                                                dt_dev);
-    k_reset_distortion<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, flag, P, P, dt_dev);
-    k_clock_advance<<<1, 1, 0, st>>>(clk, mx);
+    k_reset_distortion<L><<<GPR_SPREAD(ncell, 256), 0, st>>>(u, ncell, flag, P, P, dt_dev, clk,
+                                                               mx);
   }
 
   // ---- split scheme (steppers.cpp:50-66, split/homogeneous.cpp) -------------
