@@ -58,18 +58,18 @@ TRAFFIC = {
 }
 
 OPS = {
-    "predictor_per_cell_iter": 4904.0,    # per predictor cell and Picard iteration
-    "face_quadrature_point": 1427.0,      # D_RUS + Bint + extrapolation, per point
-    "cells_per_cell": 2293.0,             # volume term (both time nodes), per cell
-    "weno_point": 48.0,                   # per (cell, variable, sweep)
-    "cfl_per_cell": 848.0,                # per cell (two max_abs_eigs)
+    "predictor_per_cell_iter": 4080.0,    # per predictor cell and Picard iteration
+    "face_quadrature_point": 834.0,      # D_RUS + Bint + extrapolation, per point
+    "cells_per_cell": 2093.0,             # volume term (both time nodes), per cell
+    "weno_point": 22.0,                   # per (cell, variable, sweep)
+    "cfl_per_cell": 360.0,                # per cell (two max_abs_eigs)
 }
 # the same for the 1D kernels (the batched form)
 OPS_1D = {
-    "predictor_per_cell_iter": 1840.0,    # per predictor cell and Picard iteration
-    "face_point": 1423.0,                 # per (face, time node)
-    "cells_per_cell": 963.0,              # volume term, per cell
-    "weno_per_cell": 816.0,               # per predictor cell (17 points)
+    "predictor_per_cell_iter": 1524.0,    # per predictor cell and Picard iteration
+    "face_point": 828.0,                 # per (face, time node)
+    "cells_per_cell": 895.0,              # volume term, per cell
+    "weno_per_cell": 374.0,               # per predictor cell (17 points)
 }
 
 
@@ -696,11 +696,11 @@ def run_gb300(args):
             "tgv_third_order": third,
             "shock_bubble": bubble,
             "adjoint": adjoint,
-            # kernels of one 2D gpr_iterate step: k_cfl_max, k_clock_finalize,
-            # k_fill_interior, k_ghosts x2, k_weno2d, k_predictor_first,
-            # k_predictor_picard, k_predictor_stiff, k_cells, k_faces2d x4,
-            # k_renorm, k_contorted, k_reset_distortion, k_clock_advance
-            "gpu_launches": 18 * args.steps,
+            # kernels of one 2D gpr_iterate step: k_cfl_max, k_fill_interior,
+            # k_ghosts x2, k_weno2d, k_predictor_first, k_predictor_picard x2,
+            # k_predictor_stiff, k_cells, k_faces2d x4, k_renorm_contorted,
+            # k_reset_distortion
+            "gpu_launches": 16 * args.steps,
             "clocks": cs.summary()}
     if peak_err:
         line["roofline"]["peak_error"] = peak_err
@@ -985,9 +985,10 @@ def tgv_n3_bench(torch, n=512, steps=10, warmup=8, cfl=0.4, cpu=True, profile_st
                        "picard_iteration_histogram": np.bincount(iters[pic]).tolist()
                        if pic.any() else []},
          # per step: k_cfl_max, k_clock_finalize, k_boundaries_n, k_weno2d_x_n,
-         # k_weno2d_y_n, k_predictor_n, k_predictor_stiff_n, k_faces_n x2,
-         # k_cells_n, k_renorm, k_contorted, k_reset_distortion, k_clock_advance
-         "gpu_launches": 14 * steps}
+         # k_weno2d_y_n, k_predictor_first_n, k_predictor_n, k_predictor_stiff_n,
+         # k_faces_n x2, k_cells_n, k_renorm, k_contorted, k_reset_distortion,
+         # k_clock_advance
+         "gpu_launches": 15 * steps}
     if cpu:
         from oracle import Oracle
         O = Oracle(N=N)

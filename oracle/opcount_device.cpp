@@ -205,32 +205,35 @@ int main(int argc, char **argv) {
   }
   auto per = [&](Tally t) { return (double)t.flops() / nst; };
   double Fp = per(tp), Ff = per(tf), Fs = per(ts), Fb = per(tb), Fm = per(tm);
-  // Bint path node: rho, 1/rho, 3 v (3 fma + 3 mul), bdot, accumulate over
-  // the 9 rows where B x can be nonzero (9 fma)
-  double Fbint_node = 1 + 1 + 3 * 2 + 3 + Fb + 9 * 2;
+  // what a kernel does not use of prim() is not evaluated in it: A devG (9 x 5)
+  // outside the source term, devG A^T A (6 x 5) where no flux or wave speed is
+  // formed, its last entry (5) where there is no flux along z
+  const double AdG = 45, S6 = 30, S1 = 5;
+  // path_product: per node the weighted reciprocal density (fma, reciprocal,
+  // mul) and 3 velocities (2 fma each); one bdot
+  double Fbint = 2 * (4 + 3 * 4) + Fb;
   // face quadrature point (k_faces2d): 2 extrapolations (17 x 3 each), 2 prim,
-  // 2 max_abs_eigs, dissipation 17 x (sub, mul), 2 fluxes, dq (17 sub),
-  // 2 Bint nodes, weighting (kk b, kk f: 34 mul), reduce-scatter over the 4
-  // lanes (20 + 10 add per lane) and the 5 kept pairs' sums and differences
-  double Fface = 2 * 17 * 3 + 2 * Fp + 2 * Fm + 17 * 2 + 2 * Ff + 17 + 2 * Fbint_node + 34 +
-                 30 + 10;
-  // predictor node and Picard iteration (dg_rhs_node + dg_solve_node +
-  // stopping rule): prim, source (node weight in its factors), 2 x
-  // (derivative of the 6 entries bdot reads 6 x 3, bdot, 9 sub), 2 fluxes,
-  // 2 x DG_DER term on the 11 entries of the flux's support (2 fma each),
-  // r dt + Ww 17 x 2, DG_MAT^-1 17 x 3, |qn - q| > tol (1 + |q|) 17 x 3
-  double Fpred_node = Fp + Fs + 2 * (6 * 3 + Fb + 9) + 2 * Ff + 2 * 11 * 4 + 17 * 2 + 17 * 3 +
-                      17 * 3;
-  // volume node (k_cells): prim, source (weight in its factors), 2 x
-  // (derivative 6 x 3, bdot, 9 sub), reduce-scatter over the 8 lanes
-  // (12 + 6 + 3 add per lane); cell adds 17 x 5
-  double Fcell_node = Fp + Fs + 2 * (6 * 3 + Fb + 9) + 21;
+  // 2 max_abs_eigs, dissipation 17 x (sub, mul), 2 fluxes, dq (17 sub), Bint,
+  // reduce-scatter over the 4 lanes (20 + 10 add per lane), the 5 kept pairs'
+  // sums and differences and their fma onto the cells (10 + 20)
+  double Fface = 2 * 17 * 3 + 2 * (Fp - AdG) + 2 * Fm + 17 * 2 + 2 * Ff + 17 + Fbint + 30 + 30;
+  // residual along one direction (dg_residual): scaled coefficient and
+  // velocity (1 + 3), the 6 entries B reads (difference and 2 fma, 6 x 5), the
+  // flux, its difference and fma on the 11 entries of its support (11 x 3)
+  double Fdir = 4 + 30 + Ff + 33;
+  // predictor node and Picard iteration: prim, source (weight in its factors),
+  // the directions, q = w + DG_MAT^-1 r (2 fma, 17 x 4), the differences of the
+  // stopping test (17; the comparisons are FP32)
+  double Fpred_node = Fp - S1 + Fs + 2 * Fdir + 17 * 4 + 17;
+  // volume node (k_cells): prim, source, 2 x (1 + 3 + 30), reduce-scatter over
+  // the 8 lanes (12 + 6 + 3 add per lane); cell adds 17 x 5
+  double Fcell_node = Fp - S6 + Fs + 2 * 34 + 21;
   double Fcell = 8 * Fcell_node + 17 * 5;
-  // WENO point (weno_point): 4 coefficients 4 x 3, 2 indicators 2 x 9 + eps,
-  // 2 x 3 squarings, tL + tR and its reciprocal, 2 blends (2 mul, add, mul)
-  double Fweno = 12 + 2 * 10 + 6 + 2 + 8;
+  // WENO point (weno_line): 2 slopes, 2 squares + eps (fma), 2 x 3 squarings,
+  // sum, reciprocal, blended slope (mul, fma, mul), 2 node values (fma)
+  double Fweno = 2 + 4 + 6 + 2 + 4 + 4;
   double Fweno_cell = 2 * Fweno * V * 2;  // x sweep (per ub column cell) + y sweep, ~2 per node
-  double Fcfl = Fp + 2 * Fm + 3;
+  double Fcfl = Fp - AdG + 2 * Fm + 3;
   printf("# FP64 operation counts of the device formulation (gpr_device.cuh compiled\n");
   printf("# for the host with a counting scalar), TGV tile %dx%d with the 512^2 cell size\n", n, n);
   printf("prim                       %8.1f\n", Fp);
@@ -245,21 +248,20 @@ int main(int argc, char **argv) {
   printf("weno_point                 %8.1f\n", Fweno);
   printf("cfl_per_cell               %8.1f\n", Fcfl);
   printf("mean_picard_iterations     %8.3f\n", (double)iters / ncb);
-  // 1D kernels (the batched form and 1D grids), same per-state costs:
-  // face point per (face, time node) of k_faces1d: as the 2D point with a
-  // 2-lane reduce-scatter of the 17 (b, f) pairs (18 adds) and the 9 kept
-  // pairs' sums and differences (18); predictor node: one derivative, one
-  // flux and one DG_DER term; volume node: one derivative, a 4-lane
+  // 1D kernels (the batched form and 1D grids), same per-state costs (of
+  // devG A^T A the flux along x uses one column, 3 entries): face point per
+  // (face, time node) with a 2-lane reduce-scatter of the 17 (b, f) pairs (18
+  // adds), the 9 kept pairs' sums and differences (18) and weights (18);
+  // predictor node: one direction; volume node: one direction, a 4-lane
   // reduce-scatter (10 + 5 adds), cell adds 17 x 3; WENO: 17 points per
   // predictor cell; CFL: one wave speed.
-  double Fface1 = 2 * 17 * 3 + 2 * Fp + 2 * Fm + 17 * 2 + 2 * Ff + 17 + 2 * Fbint_node + 34 +
-                  18 + 18;
-  double Fpred_node1 = Fp + Fs + (6 * 3 + Fb + 9) + Ff + 11 * 4 + 17 * 2 + 17 * 3 + 17 * 3;
-  double Fcell1 = 4 * (Fp + Fs + (6 * 3 + Fb + 9) + 15) + 17 * 3;
+  double Fface1 = 2 * 17 * 3 + 2 * (Fp - AdG) + 2 * Fm + 17 * 2 + 2 * Ff + 17 + Fbint + 18 + 36;
+  double Fpred_node1 = Fp - 3 * S1 + Fs + Fdir + 17 * 4 + 17;
+  double Fcell1 = 4 * (Fp - S6 + Fs + 34 + 15) + 17 * 3;
   printf("face_point_1d              %8.1f\n", Fface1);
   printf("predictor_cell_iteration_1d %7.1f\n", 4 * Fpred_node1);
   printf("cells_per_cell_1d          %8.1f\n", Fcell1);
   printf("weno_per_cell_1d           %8.1f\n", Fweno * V);
-  printf("cfl_per_cell_1d            %8.1f\n", Fp + Fm + 2);
+  printf("cfl_per_cell_1d            %8.1f\n", Fp - AdG + Fm + 2);
   return 0;
 }
