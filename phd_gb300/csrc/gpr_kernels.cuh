@@ -464,6 +464,7 @@ constexpr double PICARD_DIVERGE = 1e3;
 // iteration cap, that hands the cell over (log2)
 constexpr int PICARD_WINDOW0 = 4;
 constexpr float PICARD_HOPELESS = 13.2877f;  // 1e4
+constexpr int PICARD_RATE_CAP = 50;  // the caps up to which the rate is extrapolated
 GPR_D unsigned long long fp_abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
 }
@@ -689,9 +690,13 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
   // iterations instead of 46.  The test lies at 1e4 and not lower for that gap
   // of two decades; the windows begin at iteration 4 since with earlier
   // or shorter ones the transient's growth is taken for the rate (windows of
-  // two: converging cells predicted at 1e8).  A step of a 256 x 256 vortex at
-  // CFL 0.8 went from 19.8 to 8.5 ms, one of 512 x 512 at CFL 0.4, where every
-  // cell converges, stayed at 16.3 ms (r is taken from iteration 4 on only).
+  // two: converging cells predicted at 1e8).  The rule is applied up to the
+  // reference's cap of 50, where it was measured: a rate taken from eight
+  // iterations says nothing about the 300 of the differentiated forward,
+  // where cells converge to 1e-13 after as many as 290.  A step of a 256 x
+  // 256 vortex at CFL 0.8 went from 19.8 to 8.5 ms, one of 512 x 512 at CFL
+  // 0.4, where every cell converges, stayed at 16.3 ms (r is taken from
+  // iteration 4 on only).
   const bool resume = R.in != nullptr && valid;
   const int it0 = resume ? R.it[c] : 0;
   float dmin = resume ? (float)R.dmin[c] : F32_TOP;
@@ -699,7 +704,8 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
   float wa = 0.0f, wb = 0.0f;  // the last window's maximum and this one's
   for (int kq = 0;; kq++) {
     const int it = it0 + kq;
-    const bool late = R.in != nullptr || kq >= PICARD_WINDOW0;  // the same over the warp
+    // the same over the warp
+    const bool late = (R.in != nullptr || kq >= PICARD_WINDOW0) && maxit <= PICARD_RATE_CAP;
     if (!done && it >= maxit) {
       failed = true;
       done = true;
