@@ -1198,16 +1198,22 @@ GPR_D double c0sq_of(const Prim<false> &s, const DevPar &P) {
 // distortion's first column), the two lower rows say (rho, p) = BA y, BA =
 // (rho, 0, 0; sigma0 - rho sigma_r + rho c0^2 e0) A^-1, whatever regular
 // matrix the reference multiplies them by, and the upper ones become (-Pi1 -
-// sigma_r BA0 + e0 BA1) y = I: one 3 x 3 inverse, singular where the
-// reference's 2 x 2 factor Z or Pi1 is.
+// sigma_r BA0 + e0 BA1) y = I: one 3 x 3 inverse, whose determinant is that of
+// Pi1 times that of the reference's 2 x 2 factor Z.
 GPR_D bool constraints(const double *Q, const Prim<false> &s, double sgn, const DevPar &P,
                        double *Rx, double *Ry) {
   const double r = s.r, ir = s.ir;
   const double *A = Q + 5;
+  const double c02 = c0sq_of(s, P);
+  // the reference takes the root (waves/speeds.cpp:17): a negative square, or a
+  // NaN, makes its whole step NaN, although the shear part may keep the
+  // spectrum of Xi real and positive
+  if (!(c02 >= 0.0))
+    return false;
   double sr[3], Pi1[9], sg[3];
   dsigma0(Q, s, P, sr, Pi1);
   sigma_col<false>(Q, s, 0, sg);
-  const double x1[3] = {fma(r, c0sq_of(s, P), fma(-r, sr[0], sg[0])), fma(-r, sr[1], sg[1]),
+  const double x1[3] = {fma(r, c02, fma(-r, sr[0], sg[0])), fma(-r, sr[1], sg[1]),
                         fma(-r, sr[2], sg[2])};
   double At[9], BA[6];  // BA^T = A^-T (rho e0, x1)
   for (int i = 0; i < 3; i++) {
