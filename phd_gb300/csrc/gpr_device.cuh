@@ -746,6 +746,8 @@ GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
     if (y > 0.0f && y <= 1.0f)
       x = fmin((double)y * (1.0 + 4e-6), 1.0) * Rs;
   }
+  // without a real root above the other roots' real parts the steps wander
+  bool found = false;
   for (int it = 0; it < 16; it++) {
     double p = 1.0, dp = 0.0, d2p = 0.0;
     const double cf[4] = {-c1, c2, -c3, c4};
@@ -755,7 +757,8 @@ GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
       dp = fma(dp, x, p);
       p = fma(p, x, cf[k]);
     }
-    if (p == 0.0)
+    found = p == 0.0;
+    if (found)
       break;
     double ip = 1.0 / p;
     double G = dp * ip;
@@ -763,11 +766,12 @@ GPR_D bool max_eig_laguerre(const double (&X)[m][m], double &lam) {
     double disc = fmax((m - 1) * fma((double)m, H, -(G * G)), 0.0);
     double a = m / (G + copysign(sqrt(disc), G));
     x -= a;
-    if (!(fabs(a) > 1e-5 * fabs(x)))  // cubic convergence: the error is now ~|a|^3
+    found = fabs(a) <= 1e-5 * fabs(x);  // cubic convergence: the error is now ~|a|^3
+    if (found)
       break;
   }
   lam = x;
-  if (!(x > 0.0) || !(x <= R * (1.0 + 1e-9)))
+  if (!found || !(x > 0.0) || !(x <= R * (1.0 + 1e-9)))
     return false;
   // deflate and certify: all other roots strictly inside |z| < (1-1e-9) lam
   double l = x * (1.0 - 1e-9);
