@@ -588,18 +588,26 @@ __global__ void __launch_bounds__(FmmThreads<ND>::value, ND == 2 ? 16 : 2)
 // What bounds it is a sweep's latency, not its work (3 warps of points per
 // SM): the waiting points are marked in a byte map, a plain store that
 // nobody waits for; each block reads the map of its own cells (dealt out in
-// segments of 8, so that a front's ring falls on all SMs alike), gathers
-// the marked ones into a list in shared memory and updates them, a lane
-// each; then the barrier.  Of a sweep's 13000 cycles (6.7 us, 4.5 ms for the
-// bubble) the map and the list take 2500, the update 5000 (43 FP64
-// instructions at 64 cycles a warp) and the barrier 5500, whose release
-// waits for the sweep's stores.  Before, lists of points in global memory
-// with a stamp per point cost 5500 cycles for the dependent atomics that
-// dedupe and append, and entries dealt out by the block left 96 SMs idle: 11
-// us a sweep.  Also measured: stamping only the changed point and reading
-// the map around each segment, fewer stores and seven loads for one (8.2
-// us); whole parts of the grid in shared memory, exchanging frames every 4
-// sweeps, where the ring falls on few of them (25 us).
+// segments of 8, so that a front's ring falls on all SMs alike) in passes of
+// 4096 cells, two passes' words in flight beside the one it works on, gathers
+// the marked ones into a list in shared memory and, when all passes are read or
+// the list could not take another, updates them, a lane each; then the
+// barrier.  On the evolved 800 x 400 bubble, one pass, a sweep of 13000 cycles
+// (6.7 us) spends 2500 on the map and the list, 5000 on the update (43 FP64
+// instructions at 64 cycles a warp) and 5500 on the barrier, whose release
+// waits for the sweep's stores.
+//
+// Lists of points in global memory with a stamp per point, the other form, cost
+// 5500 cycles a sweep for the dependent atomics that dedupe and append, but read
+// no cell that does not wait.  Microseconds a sweep, this form and that: a circle
+// on 800 x 400 5.3 and 11.0, 1600 x 800 10.1 and 19.0, 3200 x 1600 28 and 50,
+// 4096^2 118 and 212; a front along a strip, where the fewest points wait for
+// the cells, 64 x 65536 9.8 and 11.3, 512 x 8192 15.9 and 19.7.  An update in
+// each pass would cost 22 and 31 on those two.  Also measured at 800 x 400:
+// stamping only the changed point and reading the map around each segment,
+// fewer stores and seven loads for one (8.2 us); whole parts of the grid in
+// shared memory, exchanging frames every 4 sweeps, where the ring falls on few
+// of them (25 us).
 //
 // Jacobi with two buffers: sweep s reads d[s % 2] / par[s % 2] and writes
 // d[(s + 1) % 2] / par[(s + 1) % 2] for its marked points; a point that
@@ -691,26 +699,25 @@ __global__ void k_fmm_seed(Grid g, FmmGlobal G, const double *__restrict__ clk) 
 }
 
 constexpr int FMM_G_THREADS = 256, FMM_G_SEGS = 2;  // segments per thread and pass
+constexpr int FMM_G_PASS = FMM_G_THREADS * FMM_G_SEGS * 8;  // cells a pass may list
 
 __global__ void __launch_bounds__(FMM_G_THREADS) k_fmm_global(Grid g, FmmConst K, FmmGlobal G,
                                                               const double *__restrict__ clk) {
   if (clk && clk[0] >= clk[2])
     return;
   constexpr int NT = FMM_G_THREADS, U = FMM_G_SEGS;
-  __shared__ int list[NT * U * 8], nlist;
+  __shared__ int list[2 * FMM_G_PASS], nlist;
   const int tid = threadIdx.x, lane = tid & 31, nb = gridDim.x;
   const int nseg = (int)((g.ncell + 7) / 8), ngroup = (nseg + nb - 1) / nb;
   // Segment of this block in group k of nb consecutive ones: the blocks take
   // them in turn, shifted by 61 from group to group (152 = 8 x 19), since a
-  // grid whose rows are whole groups would give a column to one block.
-  auto segment = [&](int k) {
-    const int at = ((int)blockIdx.x + nb - (int)((61L * k) % nb)) % nb;
-    return k < ngroup ? k * nb + at : nseg;
-  };
-  int mine[U];
+  // grid whose rows are whole groups would give a column to one block.  A
+  // thread's groups lie NT * U apart, so its place in them moves by `hop`.
+  const int hop = (int)((61L * NT * U) % nb);
+  int place0[U];
 #pragma unroll
   for (int u = 0; u < U; u++)
-    mine[u] = segment(u * NT + tid);
+    place0[u] = ((int)blockIdx.x + nb - (int)((61L * (u * NT + tid)) % nb)) % nb;
   if (tid == 0)
     nlist = 0;
   __syncthreads();
@@ -724,45 +731,75 @@ __global__ void __launch_bounds__(FMM_G_THREADS) k_fmm_global(Grid g, FmmConst K
     uint8_t *map = G.map[s & 1], *next = G.map[(s + 1) & 1];
     const bool mono = s >= G.mono_from;
     bool any = false;
-    for (int k0 = 0; k0 < ngroup; k0 += NT * U) {
-      uint2 w[U], fr[U];
-      int seg[U];
+    // the words of this pass and the next two (loads in flight meanwhile)
+    uint2 w[3][U];
+    int seg[3][U], place[U];
+    auto fetch = [&](int slot, int k0) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        seg[u] = k0 ? segment(k0 + u * NT + tid) : mine[u];
-        const bool in = seg[u] < nseg;
-        // (the map's and fz's last segment ends within their padding)
-        w[u] = in ? __ldcg((const uint2 *)map + seg[u]) : make_uint2(0u, 0u);
-        fr[u] = in ? *((const uint2 *)G.fz + seg[u]) : make_uint2(0u, 0u);
+        const int k = k0 + u * NT + tid;
+        seg[slot][u] = k * nb + place[u];
+        // (the map's last segment ends within its padding)
+        w[slot][u] = k < ngroup && seg[slot][u] < nseg
+                         ? __ldcg((const uint2 *)map + seg[slot][u])
+                         : make_uint2(0u, 0u);
+        place[u] -= hop;
+        place[u] += place[u] < 0 ? nb : 0;
       }
+    };
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      place[u] = place0[u];
+    fetch(0, 0);
+    if (NT * U < ngroup)
+      fetch(1, NT * U);
+    for (int k0 = 0; k0 < ngroup; k0 += NT * U) {
+      const bool more = k0 + NT * U < ngroup;
+      if (k0 + 2 * NT * U < ngroup)
+        fetch(2, k0 + 2 * NT * U);
       unsigned bits = 0;  // 8 u + b: cell b of segment u
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        if (w[u].x | w[u].y)
-          __stcg((uint2 *)map + seg[u], make_uint2(0u, 0u));
-        // bytes 0 or 1, frozen points left out; the four bytes' bits together
-        const unsigned lo = w[u].x & ~fr[u].x & 0x01010101u, hi = w[u].y & ~fr[u].y & 0x01010101u;
+        if (w[0][u].x | w[0][u].y)
+          __stcg((uint2 *)map + seg[0][u], make_uint2(0u, 0u));
+        // bytes 0 or 1, the four bytes' bits together
+        const unsigned lo = w[0][u].x, hi = w[0][u].y;
         bits |= (((lo * 0x01020408u) >> 24) | ((hi * 0x01020408u) >> 24) << 4) << (8 * u);
       }
-      int incl = __popc(bits);
+      int end = 0;  // entries listed so far, as this warp knows
+      if (__any_sync(0xffffffffu, bits != 0u)) {
+        int incl = __popc(bits);
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        incl += lane >= o ? y : 0;
-      }
-      int pos = 0;
-      if (lane == 31 && incl)
-        pos = atomicAdd(&nlist, incl);
-      pos = __shfl_sync(0xffffffffu, pos, 31) + incl - __popc(bits);
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        int sg = seg[0];
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          incl += lane >= o ? y : 0;
+        }
+        int pos = 0;
+        if (lane == 31)
+          pos = atomicAdd(&nlist, incl);
+        pos = __shfl_sync(0xffffffffu, pos, 31) + incl;
+        end = pos;
+        pos -= __popc(bits);
+        while (bits) {
+          const int b = __ffs(bits) - 1;
+          bits &= bits - 1;
+          int sg = seg[0][0];
 #pragma unroll
-        for (int u = 1; u < U; u++)
-          sg = (b >> 3) == u ? seg[u] : sg;
-        list[pos++] = sg * 8 + (b & 7);
+          for (int u = 1; u < U; u++)
+            sg = (b >> 3) == u ? seg[0][u] : sg;
+          list[pos++] = sg * 8 + (b & 7);
+        }
       }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        w[0][u] = w[1][u];
+        seg[0][u] = seg[1][u];
+        w[1][u] = w[2][u];
+        seg[1][u] = seg[2][u];
+      }
+      // updates wait until the list could not take another pass
+      if (more && !__syncthreads_or(end > FMM_G_PASS))
+        continue;
       __syncthreads();
       const int nl = nlist;
       for (int q = tid; q < nl; q += NT) {
@@ -803,11 +840,11 @@ __global__ void __launch_bounds__(FMM_G_THREADS) k_fmm_global(Grid g, FmmConst K
           for (int dim = 0; dim < 2; dim++)
 #pragma unroll
             for (int sd = 0; sd < 2; sd++)
-              if (in[dim][sd])
+              if (in[dim][sd] && !bd[dim][sd])  // (frozen ones never)
                 __stcg(next + cn[dim][sd], (uint8_t)1);
         }
       }
-      if (k0 + NT * U < ngroup) {  // the list again, for the next pass
+      if (more) {  // the list again, for the next passes
         __syncthreads();
         if (tid == 0)
           nlist = 0;
