@@ -279,10 +279,8 @@ template <class L> struct Ops {
   static long fv_scratch(const int32_t *nX, int nd) {
     if (nd == 1)
       return (long)(nX[0] + 1) * 2 * V;
-    // x and y face sums, then the per-point terms of both directions (Roe,
-    // k_faces2d_eigp)
-    const long nf = (long)(nX[0] + 1) * (nX[1] + 1);
-    return 2L * nf * 2 * V + 2L * nf * NN * NN * 2 * V;
+    // x and y face sums (Roe, k_faces2d_eigp)
+    return 2L * (nX[0] + 1) * (nX[1] + 1) * 2 * V;
   }
 
   // parts: FV_BOTH (fv_launcher), FV_CENTERS (centers1/2: the volume term,
@@ -340,8 +338,8 @@ template <class L> struct Ops {
     // direction to scratch, then the cell pass applies the volume
     // and face terms
     long nf = (long)(nx + 1) * (ny + 1);
-    double *fbx = scratch, *fby = scratch + nf * 2 * V, *pp = scratch + 2 * nf * 2 * V;
-    faces2d_eig(fbx, pp, qh, nx, ny, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
+    double *fbx = scratch, *fby = scratch + nf * 2 * V;
+    faces2d_eig(fbx, qh, nx, ny, mask, dt, dt_dev, dX, time_dg, flux, P, C, st);
     k_cells<L, 2><<<blocks(nc, 128), 128, 0, st>>>(u, qh, fbx, fby, nx, ny, mask, dt, dt_dev,
                                                     hx, hy, sources, time_dg, P, C, Batch{},
                                                     parts);
@@ -367,8 +365,7 @@ template <class L> struct Ops {
     int ny = nX[1];
     long nf = (long)(nx + 1) * (ny + 1);
     if (flux != GPR_FLUX_RUSANOV && !osher_closed(flux, P)) {
-      double *pp = fb + 2 * nf * 2 * V;
-      faces2d_eig(fb, pp, qh, nx, ny, mask, dt, nullptr, dX, time_dg, flux, P, C, st);
+      faces2d_eig(fb, qh, nx, ny, mask, dt, nullptr, dX, time_dg, flux, P, C, st);
       return cuda_rc();
     }
     launch_faces2d(fb, qh, nx, ny, 0, -1, mask, dt, nullptr, 1.0 / dX[0], time_dg, flux, P, C,
@@ -419,16 +416,13 @@ template <class L> struct Ops {
   }
 
   // Roe faces of a 2D grid (k_faces2d_eigp): one thread per quadrature point
-  // of both directions into pp (2 x nf x 4 x 2V doubles), then the face sums
-  // into fb (2 x nf x 2V).
-  static void faces2d_eig(double *fb, double *pp, const double *qh, int nx, int ny,
-                          const uint8_t *mask, double dt, const double *dt_dev, const double *dX,
-                          int time_dg, int flux, const DevPar &P, const Consts &C,
-                          cudaStream_t st) {
+  // of both directions, the face sums into fb (2 x nf x 2V).
+  static void faces2d_eig(double *fb, const double *qh, int nx, int ny, const uint8_t *mask,
+                          double dt, const double *dt_dev, const double *dX, int time_dg,
+                          int flux, const DevPar &P, const Consts &C, cudaStream_t st) {
     long nf = (long)(nx + 1) * (ny + 1);
     k_faces2d_eigp<L><<<dim3(blocks(nf * NN * NN, 64), 2), 64, 0, st>>>(
-        pp, qh, nx, ny, mask, dt, dt_dev, dX[0], dX[1], time_dg, flux, P, C);
-    k_faces2d_eigsum<V><<<blocks(2 * nf * 2 * V, 256), 256, 0, st>>>(fb, pp, 2 * nf);
+        fb, qh, nx, ny, mask, dt, dt_dev, dX[0], dX[1], time_dg, flux, P, C);
   }
 
   static int timestep(const double *u, long ncell, const double *dX, int nd, double cfl,
