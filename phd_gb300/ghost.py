@@ -281,9 +281,12 @@ class MultiIterator:
     def step(self, u):
         """One step; returns the host's copy of (t, dt, NaN found)."""
         self.run(u, 1)
-        _lib.check(self.lib.gpr_any_nan(_dev(u, "u"), u.numel(), _dev(self.control[5:], "flag"),
-                                        _stream()), "any_nan")
+        flag = self.control[5:]
+        _lib.check(self.lib.gpr_any_nan(_dev(u, "u"), u.numel(), _dev(flag, "flag"), _stream()),
+                   "any_nan")
         c = self.control.tolist()
+        if c[5] != 0.0:  # gpr_any_nan sets it only
+            flag.zero_()
         return c[0], c[1], c[5] != 0.0
 
 
