@@ -457,14 +457,15 @@ GPR_D void face2_cells(double *u, int i, int j, int nx, int ny, int dir, int V, 
 // FP_INF_BITS are NaNs.
 constexpr unsigned long long FP_INF_BITS = 0x7ff0000000000000ULL;
 // growth of a cell's largest Picard update over its smallest that hands the
-// cell to the Newton pass (k_predictor_picard)
-constexpr double PICARD_DIVERGE = 1e3;
+// cell to the Newton pass (k_predictor_picard): in general, and in a Newtonian
+// fluid up to the caps below
+constexpr float PICARD_DIVERGE = 1e3f, PICARD_GROWN = 31.6f;
 // first iteration of the windows over which the rate of a cell's updates is
 // taken, and the largest update over its threshold, extrapolated to the
-// iteration cap, that hands the cell over (log2)
+// iteration cap in two windows running, that hands the cell over (log2)
 constexpr int PICARD_WINDOW0 = 4;
-constexpr float PICARD_HOPELESS = 13.2877f;  // 1e4
-constexpr int PICARD_RATE_CAP = 50;  // the caps up to which the rate is extrapolated
+constexpr float PICARD_HOPELESS = 16.6096f;  // 1e5
+constexpr int PICARD_RATE_CAP = 50;  // the caps up to which both were measured
 GPR_D unsigned long long fp_abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
 }
@@ -672,36 +673,43 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
   // Divergence detection: a cell whose largest update has grown DIVERGE
   // times above the smallest it reached is diverging and goes to the
   // stiff-source Newton pass at once instead of spending the rest of the
-  // iteration cap.  Measured with the oracle's Picard iteration over
-  // 2D TGV states at CFL 0.4 .. 1.0, stiff 1D tubes and the batched
-  // instances: cells that converge (some only after ~40 iterations) grow by
-  // at most 4.3x before converging, cells that fail grow past 1e3 within
-  // 4 .. 25 iterations and saturate near O(1) updates (without this test
-  // they run the whole cap of 50).  So every cell the reference's Picard
-  // iteration converges still converges by Picard.
-  // Most of those that fail grow slower than that, or settle into O(1)
-  // oscillations.  They are told by their rate: r, the largest update over its
-  // threshold, in windows of four iterations (their maxima b after a); a
-  // cell whose r, continued at the rate (b / a) per window, still stands
-  // above 1e4 at the cap goes to the Newton pass now.  Over 1.3 M cells
-  // (vortices of viscosity 0.05 .. 0.5 at CFL 0.3 .. 1.0, tubes of 1e-5 .. 1e-2,
-  // batched instances; 650 k of them converge) no cell that converges is ever
-  // predicted above 92, and the failing ones at CFL 0.8 stop after 22
-  // iterations instead of 46.  The test lies at 1e4 and not lower for that gap
-  // of two decades; the windows begin at iteration 4 since with earlier
-  // or shorter ones the transient's growth is taken for the rate (windows of
-  // two: converging cells predicted at 1e8).  The rule is applied up to the
-  // reference's cap of 50, where it was measured: a rate taken from eight
-  // iterations says nothing about the 300 of the differentiated forward,
-  // where cells converge to 1e-13 after as many as 290.  A step of a 256 x
-  // 256 vortex at CFL 0.8 went from 19.8 to 8.5 ms, one of 512 x 512 at CFL
-  // 0.4, where every cell converges, stayed at 16.3 ms (r is taken from
-  // iteration 4 on only).
+  // iteration cap; in a Newtonian fluid, whose iteration map is smooth, GROWN
+  // times.  Measured with the oracle's iteration over 32 M cells (every
+  // equation of state; Newtonian, power-law and Bingham fluids, elastoplastic
+  // solids; V = 14, 15 and 17; tubes, 2D flows and batched instances, CFL 0.2 ..
+  // 1), 20 M of them converging: a converging cell's updates grow by at most 10
+  // times on the way, in a Newtonian fluid (8 M) 4 times, and no further in a
+  // search that perturbs such cells towards larger growth.  Cells that fail
+  // pass 32 times within 6 .. 20 iterations, 1e3 within 8 .. 25, or settle into
+  // O(1) oscillations.
+  // Those oscillations are told by their rate, in Newtonian fluids: r, the
+  // largest update over its threshold, in windows of four iterations (their
+  // maxima b after a); a cell whose r, continued at the rate (b / a) per window,
+  // stands above 1e5 at the cap from two windows running goes to the Newton
+  // pass too.  Converging cells: at most 10^1.6 in that measurement, 10^4.2 in
+  // that search.  (One window tells too little: 10^3.2 and 10^7.4.  Nor does
+  // the rate tell anything where the relaxation has a yield point or a steep
+  // power: the iteration can leave a plateau from one update to the next, and
+  // converging Bingham cells are predicted at 10^9 from one window and 10^7
+  // from two.)  The windows begin at iteration 4 since with earlier or shorter
+  // ones the transient's growth is taken for the rate.
+  // Both are applied up to the reference's cap of 50, where they were measured:
+  // eight iterations say nothing about the 300 of the differentiated forward,
+  // where cells converge to 1e-13 after as many as 290.
+  // The failing cells of a 256 x 256 vortex of viscosity 0.02 at CFL 0.8 stop
+  // after 12 iterations, with the growth of 1e3 alone after 22, those of random
+  // Newtonian flows after 11 instead of 17: 19.8 to 8.1 ms a step of that
+  // vortex; one of 512 x 512, viscosity 0.01, at CFL 0.4, where every cell
+  // converges, stays at 16.1 ms (r is taken from iteration 4 on only).
+  const bool rated =
+      maxit <= PICARD_RATE_CAP && !(P.flags & (GPR_SOLID | GPR_POWER_LAW | GPR_BINGHAM));
+  const float grown = rated ? PICARD_GROWN : PICARD_DIVERGE;
   const bool resume = R.in != nullptr && valid;
   const int it0 = resume ? R.it[c] : 0;
   float dmin = resume ? (float)R.dmin[c] : F32_TOP;
   bool failed = false, deferred = false;
   float wa = 0.0f, wb = 0.0f;  // the last window's maximum and this one's
+  bool hopeless = false;       // the last window's verdict
   for (int kq = 0;; kq++) {
     const int it = it0 + kq;
     // the same over the warp
@@ -772,7 +780,7 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
 #pragma unroll
     for (int o = 1; o < NP; o <<= 1)
       dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-    if (!done && bigm && it >= 3 && dmax > (float)PICARD_DIVERGE * dmin) {
+    if (!done && bigm && it >= 3 && dmax > grown * dmin) {
       nan_seen = true;  // hand over to the Newton pass
       done = true;
       iters = it + 1;
@@ -785,12 +793,14 @@ __global__ void __launch_bounds__(128) k_predictor_picard(
         wb = fmaxf(wb, rmax);
         if ((it - PICARD_WINDOW0) % 4 == 3) {
           const float lb = __log2f(wb);
-          if (!done && bigm && it >= PICARD_WINDOW0 + 7 &&
-              lb + 0.25f * (float)(maxit - 1 - it) * (lb - __log2f(wa)) > PICARD_HOPELESS) {
+          const float lp = lb + 0.25f * (float)(maxit - 1 - it) * (lb - __log2f(wa));
+          const bool above = it >= PICARD_WINDOW0 + 7 && lp > PICARD_HOPELESS;
+          if (!done && bigm && rated && above && hopeless) {
             nan_seen = true;  // hand over to the Newton pass
             done = true;
             iters = it + 1;
           }
+          hopeless = above;
           wa = wb;
           wb = 0.0f;
         }
