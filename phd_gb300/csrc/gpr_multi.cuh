@@ -1152,11 +1152,11 @@ GPR_D bool inv3(const double *M, double *out) {
 // Denman-Beavers iteration (Y -> M^(1/2), Z -> M^(-1/2)), on M over the mean
 // of its eigenvalues; the reference forms the same matrix function from an
 // eigen-decomposition (riemann.cpp:136-141).  An update below 3e-9 leaves an
-// error below its square, so the iteration ends with it: 5 iterations for
-// eigenvalues 1 : 1 : 3 (9 unscaled and run to a standstill), with the same
-// errors against 64-bit mantissas (mean 2e-16).  The closed form by the
-// theorem of Cayley and Hamilton takes an eighth of the operations and
-// loses a digit.
+// error of about its square, times the root of the eigenvalues' ratio, so the
+// iteration ends with it: 5 iterations for eigenvalues 1 : 1 : 3 (9 unscaled
+// and run to a standstill), with the same errors against 64-bit mantissas on
+// ratios from 3 (mean 2e-16) to 1e8.  The closed form by the theorem of Cayley
+// and Hamilton takes an eighth of the operations and loses a digit.
 GPR_D bool inv_sqrt3(const double *M, double *Zout) {
   double Y[9], Z[9], Yi[9], Zi[9];
   const double sc = 3.0 * rcp64(M[0] + M[4] + M[8]);

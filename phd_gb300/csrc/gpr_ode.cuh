@@ -156,7 +156,8 @@ GPR_D double nondim_time(double r, double detA3, double m0, double u0, double dt
 
 // analyticSolver_distortion (analytic.cpp:71-128) by the singular value
 // decomposition, for the distortions that ode_distortion leaves (singular,
-// non-finite, or a determinant beyond 2^+-300).
+// non-finite, a determinant beyond 2^+-150, or one whose Jacobi iteration does
+// not converge).
 static __device__ __noinline__ void ode_distortion_general(double *A, double dt, const DevPar &P) {
   double U[3][3], s[3], Vm[3][3];
   svd3(A, U, s, Vm);

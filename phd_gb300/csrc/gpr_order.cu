@@ -115,8 +115,9 @@ template <class L, int NO> struct OpsN {
     return (unsigned)(grid < windows ? grid : windows);
   }
   // Face terms of direction dir: Rusanov, or the Roe / Osher eigen
-  // dissipation at one thread per face point in 64-thread blocks (its 17 x 17
-  // matrices live in local memory, as in the N = 2 per-point kernel).
+  // dissipation at one thread per face point in 64-thread blocks (a
+  // decomposition's matrices, 11 x 11 or 8 x 8, live in local memory, as in the
+  // N = 2 per-point kernel).
   template <int ND>
   static void faces(double *fb, const double *qh, const Grid &g, int dir, double dt,
                     const double *dt_dev, const double *dX, int flux, const DevPar &P,

@@ -846,9 +846,10 @@ __global__ void __launch_bounds__(32) k_predictor_stiff_n(
 // Interface terms of one face point (D_RUS / D_ROE / D_OSH and Bint,
 // fluxes.cpp:9-75, with NO path nodes): f = D + F(qL) + F(qR), D =
 // max(lambda_L, lambda_R) (qL - qR) for Rusanov (EIG false) or the eigen
-// part of D_ROE / D_OSH (EIG true, flux GPR_FLUX_ROE or GPR_FLUX_OSHER, one
-// 17 x 17 eigen-decomposition per path node for Osher, one of the
-// path-averaged matrix for Roe); b = sum_n W_n B(qL + x_n dq) dq.
+// part of D_ROE / D_OSH (EIG true, flux GPR_FLUX_ROE or GPR_FLUX_OSHER: for
+// Osher the closed form at each path node where it applies, for Roe a
+// decomposition of the path-averaged matrix's active block, 11 x 11, or 8 x 8
+// without heat conduction); b = sum_n W_n B(qL + x_n dq) dq.
 template <class L, int NO, bool EIG = false>
 GPR_D void interface_point_n(const double *ql, const double *qr, int d, const DevPar &P,
                              const ConstsN<NO> &C, double *f, double *b, int flux = 0) {
