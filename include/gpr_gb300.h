@@ -139,9 +139,10 @@ int gpr_predictor(double *qh, const double *wh, double dt, const double *dX,
  * the reference's interfs1/2 update u inside their face loops: in 2D by
  * four passes (x / y faces of even / odd index, which never share a cell),
  * in 1D in one launch with the volume term.  With the Osher and Roe fluxes
- * the face sums go through caller scratch of
- * gpr_fv_scratch_doubles(nX, ndim, nvar) doubles, which a Rusanov call
- * does not touch (it may be NULL there). */
+ * the caller passes scratch of gpr_fv_scratch_doubles(nX, ndim, nvar) doubles
+ * for the face sums (written in 1D, and in 2D by Roe and by Osher for
+ * materials without its closed form); a Rusanov call does not touch it (it may
+ * be NULL there). */
 long gpr_fv_scratch_doubles(const int32_t *nX, int ndim, int nvar);
 int gpr_fv_launcher(double *u, const double *qh, const int32_t *nX, double dt,
                     const double *dX, int ndim, int sources, int time_dg,
