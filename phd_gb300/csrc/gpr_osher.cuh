@@ -687,19 +687,35 @@ template <class L> GPR_HD constexpr bool passive_entry(int k) {
   return (k >= 5 && k < 14 && (k - 5) % 3 != 0) || k >= L::V - L::LSET;
 }
 
+// The largest passive entry of dq.
+template <class L> GPR_D double max_passive(const double *dq) {
+  double a = 0.0;
+#pragma unroll
+  for (int k = 5; k < L::V; k++)
+    if (passive_entry<L>(k))
+      a = fmax(a, fabs(dq[k]));
+  return a;
+}
+
 // |l| and g(l) of one eigenvalue l = lr + i li.  For a real l of vb's sign g is
-// that sign whatever l - vb (a semisimple l = vb included).
-GPR_D void abs_factors(double lr, double li, double vb, double &fa, double &gr, double &gi) {
+// that sign whatever l - vb (a semisimple l = vb included); where both vanish to
+// rounding (tol) it would be the sign of a rounding error, and is 0, the mean
+// of both.
+GPR_D void abs_factors(double lr, double li, double vb, double tol, double &fa, double &gr,
+                       double &gi) {
   gi = 0.0;
+  fa = li == 0.0 ? fabs(lr) : hypot(lr, li);
+  if (fa <= tol && fabs(vb) <= tol) {
+    gr = 0.0;
+    return;
+  }
   if (li == 0.0) {
-    fa = fabs(lr);
     if ((lr >= 0.0) == (vb >= 0.0))
       gr = vb >= 0.0 ? 1.0 : -1.0;
     else
       gr = (fa - fabs(vb)) / (lr - vb);
     return;
   }
-  fa = hypot(lr, li);
   const double dr = lr - vb, den = dr * dr + li * li, num = fa - fabs(vb);
   gr = num * dr / den;
   gi = -num * li / den;
@@ -760,13 +776,22 @@ GPR_D double system_active(const double *q, const double *a, double wt, const De
   return wt * s.v[0];
 }
 
+// How |M| dq by the active part ended.  Where an eigenvalue of C and vb both
+// vanish and B a has a part along its eigenvector, |M| has two limits there
+// (g = 1 and -1) that differ by that part.  No state's matrix has one (a state's
+// v is semisimple), but Roe's average at a symmetric wall does: the path's
+// velocities are v and -v, and the part is of the order of the jump.
+enum AbsStatus { ABS_FAILED = 0, ABS_OK = 1, ABS_TWO_LIMITS = 2 };
+
 // acc += w |M| dq for M given by C (n x n row-major, destroyed), Ba = B a (a the
 // passive part of dq) and vb.  With a real spectrum the eigenvectors are Z Y, Y
 // unit upper triangular (back-substitution on the Schur form), so R^-1 is Z^T
 // and a triangular solve; complex eigenvalues take the complex elimination.
+// strict: two limits are reported, with acc as it was, instead of their mean
+// taken.
 template <class L>
-GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, double w,
-                     double *acc) {
+GPR_D AbsStatus abs_apply(double *C, const double *Ba, double vb, const double *dq, double w,
+                          double *acc, bool strict = false) {
   constexpr int V = L::V, n = ACTIVE_N<L>;
   double Z[n * n], wr[n], wi[n], y[n];
 #pragma unroll 1
@@ -774,7 +799,7 @@ GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, d
     Z[i] = (i % (n + 1) == 0) ? 1.0 : 0.0;
   hess_reduce<n>(C, Z);
   if (!hqr_schur<n>(C, Z, wr, wi))
-    return false;
+    return ABS_FAILED;
   bool real = true;
 #pragma unroll 1
   for (int k = 0; k < n; k++)
@@ -783,14 +808,17 @@ GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, d
 #pragma unroll
   for (int r = 0; r < n; r++)
     dw[r] = dq[active_entry(r)];
+  double norm = 0.0;
+#pragma unroll 1
+  for (int i = 0; i < n; i++)
+#pragma unroll 1
+    for (int j = i; j < n; j++)
+      norm += fabs(C[i * n + j]);
+  const double tol = OSH_MULT_TOL * norm;
+  double part = tol * max_passive<L>(dq);  // of B a, above which two limits count
+  if (!strict || fabs(vb) > tol)
+    part = INFINITY;
   if (real) {
-    double norm = 0.0;
-#pragma unroll 1
-    for (int i = 0; i < n; i++)
-#pragma unroll 1
-      for (int j = i; j < n; j++)
-        norm += fabs(C[i * n + j]);
-    const double tol = OSH_MULT_TOL * norm;
     double Y[n * n], c2[n];  // Y by columns
 #pragma unroll 1
     for (int k = 0; k < n; k++) {
@@ -821,8 +849,10 @@ GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, d
         y[i] -= Y[k * n + i] * y[k];
         c2[i] -= Y[k * n + i] * c2[k];
       }
+      if (fabs(wr[k]) <= tol && fabs(c2[k]) > part)
+        return ABS_TWO_LIMITS;
       double fa, gr, gi;
-      abs_factors(wr[k], 0.0, vb, fa, gr, gi);
+      abs_factors(wr[k], 0.0, vb, tol, fa, gr, gi);
       y[k] = fa * y[k] + gr * c2[k];
     }
     // Y y (column by column, downwards in place), then Z
@@ -861,11 +891,13 @@ GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, d
       bi[k] = bi[n + k] = 0.0;
     }
     if (!csolve_n<n>(C, Z, br, bi))
-      return false;
+      return ABS_FAILED;
 #pragma unroll 1
     for (int k = 0; k < n; k++) {
+      if (hypot(wr[k], wi[k]) <= tol && hypot(br[n + k], bi[n + k]) > part)
+        return ABS_TWO_LIMITS;
       double fa, gr, gi;
-      abs_factors(wr[k], wi[k], vb, fa, gr, gi);
+      abs_factors(wr[k], wi[k], vb, tol, fa, gr, gi);
       const double xr = fa * br[k] + (gr * br[n + k] - gi * bi[n + k]);
       bi[k] = fa * bi[k] + (gr * bi[n + k] + gi * br[n + k]);
       br[k] = xr;
@@ -887,7 +919,7 @@ GPR_D bool abs_apply(double *C, const double *Ba, double vb, const double *dq, d
   for (int k = 5; k < V; k++)
     if (passive_entry<L>(k))
       acc[k] = fma(av, dq[k], acc[k]);
-  return true;
+  return ABS_OK;
 }
 
 // ---------------------------------------------------------------------------
@@ -1117,7 +1149,7 @@ __device__ __noinline__ bool abs_apply_general(const double *q, const double *dq
   for (int i = 0; i < n; i++)
     Ba[i] = 0.0;
   const double vb = system_active<L>(q, dq, 1.0, P, C, Ba);
-  return abs_apply<L>(C, Ba, vb, dq, w, f);
+  return abs_apply<L>(C, Ba, vb, dq, w, f) == ABS_OK;
 }
 
 // Eigen part of D_OSH along x into f (overwritten): sum_i w_i |M(q_i)| dq
@@ -1159,6 +1191,82 @@ GPR_D void osher_dissipation(const double *ql, const double *qr, const DevPar &P
   }
 }
 
+// f = |M| dq for Roe's path average M by the decomposition of the whole V x V
+// matrix, for the faces where the active part finds two limits: eigenvalues
+// that agree to rounding take independent vectors (schur_vectors), which gives
+// the value of the form before the active part was split off, and no mass flux
+// through the wall but where the solver's own roundings tell such eigenvalues
+// apart.  With heat conduction C has no zero eigenvalue there.
+template <class L, int NQ>
+__device__ __noinline__ bool roe_whole(const double *qr, const double *dq, const DevPar &P,
+                                       const double *nodes, const double *wts, double *f) {
+  constexpr int V = L::V;
+  double M[V * V], Z[V * V], Rr[V * V], Ri[V * V], wr[V], wi[V], br[2 * V], bi[2 * V], q[V];
+#pragma unroll 1
+  for (int i = 0; i < V * V; i++)
+    M[i] = 0.0;
+#pragma unroll 1
+  for (int n = 0; n < NQ; n++) {
+#pragma unroll 1
+    for (int k = 0; k < V; k++)
+      q[k] = qr[k] + nodes[n] * dq[k];
+#pragma unroll 1
+    for (int i = 0; i < V * V; i++)
+      Rr[i] = Ri[i] = 0.0;
+    Prim<L::THERMAL> s;
+    prim<L::THERMAL>(q, P, s);
+    system_fd<L::THERMAL, V>(q, s, P, Rr, Ri);
+#pragma unroll 1
+    for (int i = 0; i < V; i++)
+#pragma unroll 1
+      for (int j = 0; j < V; j++) {
+        double x = 0.0;
+#pragma unroll 1
+        for (int k = 0; k < V; k++)
+          x += Rr[i * V + k] * Ri[k * V + j];
+        Z[i * V + j] = x;
+      }
+    system_block<V, L::LSET>(s.v, Z);
+#pragma unroll 1
+    for (int i = 0; i < V * V; i++)
+      M[i] += wts[n] * Z[i];
+  }
+#pragma unroll 1
+  for (int i = 0; i < V * V; i++)
+    Z[i] = (i % (V + 1) == 0) ? 1.0 : 0.0;
+  hess_reduce<V>(M, Z);
+  if (!hqr_schur<V>(M, Z, wr, wi))
+    return false;
+  schur_vectors<V>(M, Z, wr, wi, Rr, Ri);
+#pragma unroll 1
+  for (int i = 0; i < V * V; i++) {
+    M[i] = Rr[i];
+    Z[i] = Ri[i];
+  }
+#pragma unroll 1
+  for (int k = 0; k < V; k++) {
+    br[k] = dq[k];
+    br[V + k] = bi[k] = bi[V + k] = 0.0;
+  }
+  if (!csolve_n<V>(M, Z, br, bi))
+    return false;
+#pragma unroll 1
+  for (int k = 0; k < V; k++) {
+    const double a = hypot(wr[k], wi[k]);
+    br[k] *= a;
+    bi[k] *= a;
+  }
+#pragma unroll 1
+  for (int i = 0; i < V; i++) {
+    double x = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < V; k++)
+      x += Rr[i * V + k] * br[k] - Ri[i * V + k] * bi[k];
+    f[i] = x;
+  }
+  return true;
+}
+
 // Eigen part of D_OSH (flux 2) / D_ROE (flux 1) at one interface into f
 // (overwritten); NaN if the eigen-decomposition fails (fluxes.cpp:22-64).
 // The path qR -> qL takes the scheme's NQ Gauss nodes (nodes, wts on [0, 1]).
@@ -1197,7 +1305,23 @@ GPR_D void eig_dissipation_q(const double *ql, const double *qr, int flux, const
       q[k] = qr[k] + nodes[i] * dq[k];
     vb += system_active<L>(q, dq, wts[i], P, C, Ba);
   }
-  if (!abs_apply<L>(C, Ba, vb, dq, 1.0, f)) {
+  const AbsStatus rc = abs_apply<L>(C, Ba, vb, dq, 1.0, f, !L::THERMAL);
+  bool ok = rc == ABS_OK;
+  if constexpr (!L::THERMAL) {
+    if (rc == ABS_TWO_LIMITS) {
+      double rm[V], dm[V], fm[V];
+#pragma unroll
+      for (int k = 0; k < V; k++) {
+        rm[k] = qr[k];
+        dm[k] = dq[k];
+      }
+      ok = roe_whole<L, NQ>(rm, dm, P, nodes, wts, fm);
+#pragma unroll
+      for (int k = 0; k < V; k++)
+        f[k] = fm[k];
+    }
+  }
+  if (!ok) {
 #pragma unroll
     for (int k = 0; k < V; k++)
       f[k] = __longlong_as_double(0x7ff8000000000000ll);
@@ -1286,10 +1410,11 @@ GPR_D void interface_point_eig(const double *ql, const double *qr, int flux, con
 // Rr and Ri hold dF/dP and dP/dQ before the eigen-decomposition, then the
 // eigenvectors (Y in Rr for a real spectrum; for a complex one H and Z
 // afterwards hold the copy that the complex solve factorises).
+// Sized for the whole matrix where w_roe_whole may need it (m = V).
 template <class L> struct EigWS {
-  static constexpr int V = L::V, n = ACTIVE_N<L>;
-  double H[n * n], Z[n * n], Rr[V * V], Ri[V * V];
-  double wr[n], wi[n], v[n > 3 ? n : 3], br[2 * n], bi[2 * n], Ba[n], vb;
+  static constexpr int V = L::V, n = ACTIVE_N<L>, m = L::THERMAL ? n : V;
+  double H[m * m], Z[m * m], Rr[V * V], Ri[V * V];
+  double wr[m], wi[m], v[m], br[2 * m], bi[2 * m], Ba[n], vb;
   double q[V], ql[V], qr[V], dq[V], f[V];
 };
 
@@ -1775,23 +1900,27 @@ GPR_D bool w_csolve(double *Cr, double *Ci, double *br, double *bi, int lane) {
 
 // ws.f += w |M| ws.dq for M given by ws.H (C, destroyed), ws.Ba and ws.vb, as
 // abs_apply.
-template <class L> GPR_D bool w_abs_apply(EigWS<L> &ws, double w, int lane) {
+template <class L>
+GPR_D AbsStatus w_abs_apply(EigWS<L> &ws, double w, int lane, bool strict = false) {
   constexpr int V = L::V, n = ACTIVE_N<L>;
   for (int e = lane; e < n * n; e += 32)
     ws.Z[e] = (e % (n + 1) == 0) ? 1.0 : 0.0;
   __syncwarp();
   w_hess<n>(ws.H, ws.Z, ws.v, lane);
   if (!w_hqr<n>(ws.H, ws.Z, ws.wr, ws.wi, lane))
-    return false;
+    return ABS_FAILED;
   __syncwarp();
   const bool real = __all_sync(0xffffffffu, lane >= n || ws.wi[lane < n ? lane : 0] == 0.0);
   double out = 0.0;  // entry `lane` of the active result
+  double nrm = 0.0;
+  for (int e = lane; e < n * n; e += 32)
+    if (e % n >= e / n)
+      nrm += fabs(ws.H[e]);
+  const double tol = OSH_MULT_TOL * warp_sum(nrm);
+  double part = tol * max_passive<L>(ws.dq);
+  if (!strict || fabs(ws.vb) > tol)
+    part = INFINITY;
   if (real) {
-    double nrm = 0.0;
-    for (int e = lane; e < n * n; e += 32)
-      if (e % n >= e / n)
-        nrm += fabs(ws.H[e]);
-    const double tol = OSH_MULT_TOL * warp_sum(nrm);
     double *Y = ws.Rr, *y = ws.br, *c2 = ws.br + n;  // Y by columns
     if (lane < n) {
       const int k = lane;
@@ -1820,9 +1949,12 @@ template <class L> GPR_D bool w_abs_apply(EigWS<L> &ws, double w, int lane) {
       }
       __syncwarp();
     }
+    if (__any_sync(0xffffffffu,
+                   lane < n && fabs(ws.wr[lane < n ? lane : 0]) <= tol && fabs(c2[lane < n ? lane : 0]) > part))
+      return ABS_TWO_LIMITS;
     if (lane < n) {
       double fa, gr, gi;
-      abs_factors(ws.wr[lane], 0.0, ws.vb, fa, gr, gi);
+      abs_factors(ws.wr[lane], 0.0, ws.vb, tol, fa, gr, gi);
       y[lane] = fa * y[lane] + gr * c2[lane];
     }
     __syncwarp();
@@ -1850,10 +1982,14 @@ template <class L> GPR_D bool w_abs_apply(EigWS<L> &ws, double w, int lane) {
     }
     __syncwarp();
     if (!w_csolve<n>(Cr, Ci, ws.br, ws.bi, lane))
-      return false;
+      return ABS_FAILED;
+    const int kl = lane < n ? lane : 0;
+    if (__any_sync(0xffffffffu, lane < n && hypot(ws.wr[kl], ws.wi[kl]) <= tol &&
+                                    hypot(ws.br[n + kl], ws.bi[n + kl]) > part))
+      return ABS_TWO_LIMITS;
     if (lane < n) {
       double fa, gr, gi;
-      abs_factors(ws.wr[lane], ws.wi[lane], ws.vb, fa, gr, gi);
+      abs_factors(ws.wr[lane], ws.wi[lane], ws.vb, tol, fa, gr, gi);
       const double b2r = ws.br[n + lane], b2i = ws.bi[n + lane];
       ws.br[lane] = fa * ws.br[lane] + (gr * b2r - gi * b2i);
       ws.bi[lane] = fa * ws.bi[lane] + (gr * b2i + gi * b2r);
@@ -1869,7 +2005,7 @@ template <class L> GPR_D bool w_abs_apply(EigWS<L> &ws, double w, int lane) {
     if (passive_entry<L>(k))
       ws.f[k] += w * fabs(ws.vb) * ws.dq[k];
   __syncwarp();
-  return true;
+  return ABS_OK;
 }
 
 // wt times the system matrix of ws.q added to ws.H, ws.Ba and ws.vb (as
@@ -1927,6 +2063,83 @@ template <class L> GPR_D void w_system_active(EigWS<L> &ws, double wt, const Dev
   if (lane == 0)
     ws.vb += wt * ws.v[0];
   __syncwarp();
+}
+
+// ws.f = |M| ws.dq by the whole matrix of Roe's path average, as roe_whole.
+template <class L> GPR_D bool w_roe_whole(EigWS<L> &ws, const DevPar &P, const Consts &C, int lane) {
+  constexpr int V = L::V;
+  for (int e = lane; e < V * V; e += 32)
+    ws.Z[e] = 0.0;
+#pragma unroll 1
+  for (int n = 0; n < NN; n++) {
+    for (int k = lane; k < V; k += 32)
+      ws.q[k] = ws.qr[k] + C.nodes[n] * ws.dq[k];
+    for (int e = lane; e < V * V; e += 32)
+      ws.Rr[e] = ws.Ri[e] = 0.0;
+    __syncwarp();
+    if (lane == 0) {
+      double q[V];
+#pragma unroll
+      for (int k = 0; k < V; k++)
+        q[k] = ws.q[k];
+      Prim<L::THERMAL> s;
+      prim<L::THERMAL>(q, P, s);
+      system_fd<L::THERMAL, V>(q, s, P, ws.Rr, ws.Ri);
+      ws.v[0] = s.v[0];
+      ws.v[1] = s.v[1];
+      ws.v[2] = s.v[2];
+    }
+    __syncwarp();
+    for (int e = lane; e < V * V; e += 32) {
+      const int i = e / V, j = e % V;
+      double x = 0.0;
+      for (int k = 0; k < V; k++)
+        x += ws.Rr[i * V + k] * ws.Ri[k * V + j];
+      ws.H[e] = x;
+    }
+    __syncwarp();
+    if (lane == 0)
+      system_block<V, L::LSET>(ws.v, ws.H);
+    __syncwarp();
+    for (int e = lane; e < V * V; e += 32)
+      ws.Z[e] += C.w[n] * ws.H[e];
+    __syncwarp();
+  }
+  for (int e = lane; e < V * V; e += 32) {
+    ws.H[e] = ws.Z[e];
+    ws.Z[e] = (e % (V + 1) == 0) ? 1.0 : 0.0;
+  }
+  __syncwarp();
+  w_hess<V>(ws.H, ws.Z, ws.v, lane);
+  if (!w_hqr<V>(ws.H, ws.Z, ws.wr, ws.wi, lane))
+    return false;
+  __syncwarp();
+  w_schur_vectors<V>(ws.H, ws.Z, ws.wr, ws.wi, ws.Rr, ws.Ri, lane);
+  for (int e = lane; e < V * V; e += 32) {
+    ws.H[e] = ws.Rr[e];
+    ws.Z[e] = ws.Ri[e];
+  }
+  if (lane < V) {
+    ws.br[lane] = ws.dq[lane];
+    ws.br[V + lane] = ws.bi[lane] = ws.bi[V + lane] = 0.0;
+  }
+  __syncwarp();
+  if (!w_csolve<V>(ws.H, ws.Z, ws.br, ws.bi, lane))
+    return false;
+  if (lane < V) {
+    const double a = hypot(ws.wr[lane], ws.wi[lane]);
+    ws.br[lane] *= a;
+    ws.bi[lane] *= a;
+  }
+  __syncwarp();
+  if (lane < V) {
+    double x = 0.0;
+    for (int k = 0; k < V; k++)
+      x += ws.Rr[lane * V + k] * ws.br[k] - ws.Ri[lane * V + k] * ws.bi[k];
+    ws.f[lane] = x;
+  }
+  __syncwarp();
+  return true;
 }
 
 // Osher interface terms at one point along D: f = D + F(qL) + F(qR), b = Bint.
@@ -2110,7 +2323,13 @@ __global__ void __launch_bounds__(32 * EIG_WARPS) k_faces1d_eigw(
         __syncwarp();
         w_system_active<L>(ws, osher ? 1.0 : C.w[i], P, lane);
       }
-      ok = w_abs_apply<L>(ws, osher ? C.w[ip] : 1.0, lane);
+      const AbsStatus rc =
+          w_abs_apply<L>(ws, osher ? C.w[ip] : 1.0, lane, !osher && !L::THERMAL);
+      ok = rc == ABS_OK;
+      if constexpr (!L::THERMAL) {
+        if (rc == ABS_TWO_LIMITS)
+          ok = w_roe_whole<L>(ws, P, C, lane);
+      }
     }
     if (!ok) {
       for (int k = lane; k < V; k += 32)
